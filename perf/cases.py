@@ -164,3 +164,60 @@ def run(state):
     if call == "dropout":
         return fa.attention_forward(q, k, v, dropout_p=case["dropout"], seed=state["seed"], **window)
     return fa.attention_forward(q, k, v, **window)
+
+
+def _philox_keep(seed, head, rows, n, threshold):
+    """Keep mask of the dropout call for a block of query rows: byte j % 16 of Philox-4x32-10 (key = seed,
+    counter = {j / 16, row, head, 0}; Salmon et al. 2011) below `threshold`."""
+    low = 0xFFFFFFFF
+
+    def words(block, row):
+        c = [block, row, torch.full_like(block, head), torch.zeros_like(block)]
+        k = [seed & low, (seed >> 32) & low]
+        for _ in range(10):
+            a, b = c[0] * 0xD2511F53, c[2] * 0xCD9E8D57  # 32 x 32 bits; the sign of the wrapped 64-bit product is masked off
+            c = [((b >> 32) & low) ^ c[1] ^ k[0], b & low, ((a >> 32) & low) ^ c[3] ^ k[1], a & low]
+            k = [(k[0] + 0x9E3779B9) & low, (k[1] + 0xBB67AE85) & low]
+        return c
+
+    block = torch.arange((n + 15) // 16, device=rows.device).expand(len(rows), -1)
+    out = torch.stack(words(block, rows[:, None].expand_as(block)), dim=-1)  # [row][block][word]
+    byte = torch.stack([(out >> (8 * t)) & 255 for t in range(4)], dim=-1)
+    return byte.reshape(len(rows), -1)[:, :n] < threshold
+
+
+def exact(case, seed):
+    """The attention of the same inputs in 64 bits."""
+    state = prepare(case, seed)
+    n, d, heads, call = case["seqlen"], case["head_dim"], case["heads"], case["call"]
+    q, k, v = (state[x].cuda().view(-1, n, d) for x in "qkv")
+    bh = q.shape[0]
+    out = torch.empty((bh, n, d), dtype=torch.float64)
+    lse = torch.empty((bh, n), dtype=torch.float64)
+    wl, wr = case["window_left"], 0 if case["causal"] else case["window_right"]
+    threshold = int(round(256 * (1 - case["dropout"])))
+    step = max(1, min(n, (1 << 27) // n))
+    for h in range(bh):
+        kh, vh = k[h].double(), v[h].double()
+        for r0 in range(0, n, step):
+            rows = torch.arange(r0, min(n, r0 + step), device="cuda")
+            lo = 0 if wl < 0 else max(0, r0 - wl)
+            hi = n if wr < 0 else min(n, r0 + len(rows) + wr)
+            cols = torch.arange(lo, hi, device="cuda")
+            s = q[h, rows].double() @ kh[lo:hi].T / math.sqrt(d)
+            gap = cols[None, :] - rows[:, None]
+            if call == "alibi":
+                s -= state["slopes"][h % heads].double() * gap.abs()
+            if wl >= 0:
+                s.masked_fill_(gap < -wl, -math.inf)
+            if wr >= 0:
+                s.masked_fill_(gap > wr, -math.inf)
+            top = s.amax(dim=1, keepdim=True)
+            p = s.sub_(top).exp_()
+            total = p.sum(dim=1, keepdim=True)
+            lse[h, rows.cpu()] = (top + total.log()).squeeze(1).cpu()
+            if case["dropout"] > 0:
+                p = p * _philox_keep(seed, h, rows, n, threshold)[:, lo:hi] * (256 / threshold)
+            out[h, rows.cpu()] = (p @ vh[lo:hi] / total).cpu()
+    out = out.view(case["batch"], heads, n, d)
+    return (out, lse.view(case["batch"], heads, n)) if call == "lse" else out
