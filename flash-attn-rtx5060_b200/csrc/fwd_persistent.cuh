@@ -354,9 +354,25 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
           if (kAlibi) {  // s * scale - slope * |i - j|, in log2 units (reference: src/mask.h:21-26, src/main.cu:200-207)
             const float rel = static_cast<float>(row - kv0);
+            if (kMasked) {
   #pragma unroll
-            for (int c = 0; c < kBlockN; ++c)
-              sc[c] = fmaf(sc[c], p.scale_log2, -slope_l2 * fabsf(rel - static_cast<float>(c)));
+              for (int c = 0; c < kBlockN; ++c)
+                sc[c] = fmaf(sc[c], p.scale_log2, -slope_l2 * fabsf(rel - static_cast<float>(c)));
+            } else {
+              // All keys of the tile lie on one side of all rows, so the bias is linear in the column and costs one
+              // scalar FMA and half a two-wide one per element instead of a subtraction, a product and an FMA:
+              // B2 H16 N4096 causal, d64 177.5 -> 159 us, d128 199 -> 171 (without ALiBi d64 runs in 133.5). Folding
+              // the bias into the exponent's FMA with a bound in place of the max was no faster on these (156, 173)
+              // and slower without a mask (292 -> 331).
+              const uint64_t biasscale2 = f2_pack(p.scale_log2, p.scale_log2);
+              const float step = rel > 0.f ? slope_l2 : -slope_l2;
+              const float base = -slope_l2 * fabsf(rel);
+  #pragma unroll
+              for (int c = 0; c < kBlockN; c += 2) {
+                const float b0 = fmaf(step, static_cast<float>(c), base), b1 = fmaf(step, static_cast<float>(c + 1), base);
+                f2_unpack(f2_fma(f2_pack(sc[c], sc[c + 1]), biasscale2, f2_pack(b0, b1)), sc[c], sc[c + 1]);
+              }
+            }
           }
           if (kMasked) {
             // Visible columns of this row: c_lo <= c <= c_hi, i.e. |c - mid| <= half. The predicate is applied on the
@@ -445,7 +461,10 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           __syncwarp();
           if (lane == 0) mbar_arrive(&p_full2[s]);  // P of keys 64..127
         };
-        if (kv_tile_needs_mask(kv0, q_r0, q_r1, wl, wr, N)) tile_body(std::true_type{});
+        // (ALiBi: a tile that the diagonal crosses takes the cut tiles' body, whose bias has the absolute value)
+        if (kv_tile_needs_mask(kv0, q_r0, q_r1, wl, wr, N) ||
+            (kAlibi && kv0 + kBlockN - 1 > q_r0 && kv0 < q_r1))
+          tile_body(std::true_type{});
         else tile_body(std::false_type{});
       }
       if (!ok) break;
