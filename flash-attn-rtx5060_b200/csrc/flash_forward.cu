@@ -200,6 +200,34 @@ int launch_pair_ahead(DeviceState* s, const void* q, const void* k, const void* 
   return FA_OK;
 }
 
+// Takes some of the pairs of q tiles apart into single q tiles whose kv tiles the two stages of a CTA share out
+// (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
+// the epilogue merges two outputs), but there are twice as many items of half the length.
+// - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
+//   one wave. B2 H16 N4096 d128: 3.46 waves of 32 steps, 277 -> 255 us; 8 heads of 333 rows: 14.3 -> 12.6 us.
+// - Under a causal mask items are handed out longest first and a partial wave costs little; but with few of them the
+//   longest one sets the time. All are split while a CTA has less than about 7/4 items, or, where sequences are
+//   short and the fill and drain of an item weigh more, less than a seventh of a head's pairs (d64 us, pairs against
+//   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
+//   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
+//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
+void set_work_items(fa::FwdParams* p, int num_sms) {
+  const int pairs = p->num_items;
+  int split = 0;
+  if (p->seqlen > fa::kBlockM && pairs < (1 << 30)) {
+    const int wl = p->window_left, wr = fa::eff_window_right(p->causal, p->window_right);
+    const bool even = (wl < 0 && wr < 0) || (wl >= 0 && wr >= 0 && wl < p->seqlen / 4 && wr < p->seqlen / 4);
+    if (even) {
+      const int tail = pairs % num_sms;
+      if (2 * tail <= num_sms) split = tail;
+    } else if (2 * pairs <= num_sms || 4LL * pairs <= 7LL * num_sms) {
+      if (2 * pairs <= num_sms || 7LL * pairs <= (long long)p->num_q_pairs * num_sms) split = pairs;
+    }
+  }
+  p->num_pair_items = pairs - split;
+  p->num_items = pairs + split;
+}
+
 template <int D, bool kAlibi, bool kLse, bool kDropout = false>
 int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                          const CUtensorMap& mo,
@@ -209,8 +237,9 @@ int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMa
   constexpr int slot = (kDropout ? 12 : (kLse ? 8 : 2)) + (kAlibi ? 2 : 0) + (D == 64 ? 0 : 1);
   int rc = ensure_smem_attr(s, slot, fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout>, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
-  int grid = p.num_items < s->num_sms ? p.num_items : s->num_sms;
   fa::FwdParams pp = p;
+  set_work_items(&pp, s->num_sms);
+  const int grid = pp.num_items < s->num_sms ? pp.num_items : s->num_sms;
   std::lock_guard<std::mutex> lk(s->mu);
   int sched_slot = 0;
   if ((rc = sched_acquire(s, st, &pp.sched, &sched_slot)) != FA_OK) return rc;
@@ -318,8 +347,9 @@ int noalloc_state(NoAllocState** out) {
 template <int D>
 int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                               const CUtensorMap& mo,
-                              const fa::FwdParams& p, cudaStream_t st) {
+                              fa::FwdParams p, cudaStream_t st) {
   using Cfg = fa::PersistentCfg<D>;
+  set_work_items(&p, s->num_sms);
   {
     std::lock_guard<std::mutex> lk(s->mu);
     bool& done = s->attr_set[D == 64 ? 0 : 1];
@@ -341,14 +371,18 @@ int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUte
 
 // Heads per scheduling group of the persistent kernel. Without a mask all items cost the same and head-major
 // order (1) shares K/V best. With a causal mask or a window the item costs differ, and interleaving the heads of
-// a group pair-major keeps the tail short. Three measured constraints (B200): the K and V rows that a group
-// keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
+// a group pair-major makes the order of the group longest first. Measured constraints (B200): the K and V rows that a
+// group keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
 // what both dies read: the long-context workload read K/V from DRAM 2.2 times with 96 MB in flight, 1.5 times
 // with 64 MB, 1.1 times with 48 MB, at the same speed; the 8192-row config is 0.6 % faster with 64 MB than
 // with 48); a group needs about two items per CTA to balance; and the groups must be of even size (64 heads in
-// groups of 12 leave a last group of 4 heads, too few items for 148 CTAs: -4 %).
+// groups of 12 leave a last group of 4 heads, too few items for 148 CTAs: -4 %). Within those limits a group is as
+// large as it can be: with one group for all heads the whole launch is handed out longest first and ends on its
+// cheapest items. Against groups of at most 16 heads: B4 H16 N2048 d64 causal 82.4 -> 72.8 us, 24 heads of 4001 rows
+// d128 with log-sum-exp 132 -> 116, B2 H16 N4096 d64 ALiBi 161 -> 136, B8 H16 N1024 d128 70 -> 58.
+// (flash_forward_head_group reports base groups, `most` = 16 heads; a launch takes as many heads as fit.)
 static int pick_head_group(int bh, int seqlen, int head_dim, int causal, int window_left, int window_right,
-                           int num_q_pairs, int num_sms) {
+                           int num_q_pairs, int num_sms, int most = 0x7fffffff) {
   if (!causal && window_left < 0 && window_right < 0) return 1;
   const int wr = causal ? 0 : window_right;
   long long span = seqlen;
@@ -359,9 +393,9 @@ static int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
   const double span_bytes = 4.0 * (double)span * head_dim;  // K and V rows, fp16
   int grp_l2 = (int)(64.0 * 1024 * 1024 / span_bytes);
   const int grp_bal = (2 * num_sms + num_q_pairs - 1) / num_q_pairs;
-  int grp = grp_l2 < 16 ? grp_l2 : 16;
+  int grp = grp_l2;
   if (grp < grp_bal) grp = grp_bal;
-  if (grp > 16) grp = 16;
+  if (grp > most) grp = most;
   if (grp < 1) grp = 1;
   if (grp > bh) grp = bh;
   const int groups = (bh + grp - 1) / grp;
@@ -400,7 +434,7 @@ int flash_forward_head_group(int batch_heads, int seqlen, int head_dim, int is_c
   if (batch_heads <= 0 || seqlen <= 0 || (head_dim != 64 && head_dim != 128) || num_sms <= 0) return 0;
   const int pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
   return pick_head_group(batch_heads, seqlen, head_dim, is_causal ? 1 : 0, norm_window(window_left, seqlen),
-                         norm_window(window_right, seqlen), pairs, num_sms);
+                         norm_window(window_right, seqlen), pairs, num_sms, 16);
 }
 
 int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int window_right, int row_begin,

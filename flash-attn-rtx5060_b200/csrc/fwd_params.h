@@ -27,7 +27,9 @@ struct FwdParams {
                      // persistent kernel only): CTA 0 withholds one tile so that a bounded wait runs out
   // persistent kernel only
   int num_q_pairs;   // ceil(seqlen / 256)
-  int num_items;     // bh * num_q_pairs
+  int num_items;     // bh * num_q_pairs; the one-CTA persistent kernel: work items, split ones counted singly
+  int num_pair_items;  // items below this are pairs of q tiles, later ones single q tiles whose kv tiles the two
+                       // stages share out (persistent kernel only)
   int head_group;    // heads whose items are interleaved pair-major in the work-item order
   const float* alibi_slopes;  // optional, one slope per head (device); the score of (i, j) gets
                               // -slope * |i - j| after scaling, as the reference does (src/mask.h:21-26)

@@ -79,6 +79,10 @@ struct ItemGeom {
   int r0[2], r1[2];  // first / last q row of each stage's tile (r1 < r0: stage has no rows)
   int lo[2], hi[2];  // walk steps of each stage, [lo, hi); empty when no rows. Step t works on kv tile `top - t`
   int top, steps;    // last visible kv tile of the item, number of steps
+  // 0: the stages own the two q tiles of a pair and share every kv tile (both work on tile `top - t` in step t).
+  // 1: both stages own the SAME q tile and take its kv tiles in turn: stage s works on tile top - 2t - s; the
+  //    epilogue merges their two outputs.
+  int split;
 };
 
 // Work-item order. Heads are taken in groups of `head_group` (sized on the host so that the K/V of
@@ -89,6 +93,9 @@ struct ItemGeom {
 template <int BN = kBlockN>
 __device__ __forceinline__ ItemGeom decode_item(int item, const FwdParams& p) {
   ItemGeom g;
+  const int sub = (item - p.num_pair_items) & 1;  // of a split pair: 0 the second q tile (the longer one), 1 the first
+  g.split = item >= p.num_pair_items;
+  if (g.split) item = p.num_pair_items + ((item - p.num_pair_items) >> 1);
   const int per_group = p.head_group * p.num_q_pairs;
   const int grp = item / per_group;
   const int r = item - grp * per_group;
@@ -111,6 +118,19 @@ __device__ __forceinline__ ItemGeom decode_item(int item, const FwdParams& p) {
       lo_all = min(lo_all, g.lo[s]);
       hi_all = max(hi_all, g.hi[s]);
     }
+  }
+  if (g.split) {
+    const int s = 1 - sub;
+    const int n = s ? g.hi[1] - g.lo[1] : g.hi[0] - g.lo[0];  // kv tiles of the one q tile (0: it has no rows)
+    g.top = (s ? g.hi[1] : g.hi[0]) - 1;
+    g.r0[0] = g.r0[1] = s ? g.r0[1] : g.r0[0];
+    g.r1[0] = s ? g.r1[1] : g.r1[0];
+    g.r1[1] = n > 1 ? g.r1[0] : g.r0[0] - 1;
+    g.lo[0] = g.lo[1] = 0;
+    g.hi[0] = g.steps = (n + 1) >> 1;
+    g.hi[1] = n >> 1;
+    g.split = n > 1;
+    return g;
   }
   g.top = hi_all - 1;
   g.steps = hi_all - lo_all;
@@ -231,7 +251,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   uint64_t* kv_empty = bars + 20 + Cfg::kStages;  // [kStages] MMA -> TMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // [2][16]: ItemGeom of the published item in words 0..11, its id (-1: no more items) in word 12
+  // [2][16]: ItemGeom of the published item in words 0..11, its id (-1: no more items) in word 12, `split` in word 13
   volatile int* s_geom = reinterpret_cast<volatile int*>(smem + Cfg::kOffGeom);
   constexpr uint32_t kItemReaders = 13;  // 8 softmax warps + 4 correction warps + the MMA warp
 
@@ -285,7 +305,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     g.bh = w[0]; g.pair = w[1];
     g.r0[0] = w[2]; g.r0[1] = w[3]; g.r1[0] = w[4]; g.r1[1] = w[5];
     g.lo[0] = w[6]; g.lo[1] = w[7]; g.hi[0] = w[8]; g.hi[1] = w[9];
-    g.top = w[10]; g.steps = w[11];
+    g.top = w[10]; g.steps = w[11]; g.split = w[13];
     __syncwarp();
     if (lane == 0) mbar_arrive(&item_empty[slot]);
     ++n_items;
@@ -327,7 +347,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (!mbar_wait_warp(&s_full[s], n_s & 1, abort_flag)) { ok = false; break; }
         ++n_s;
         tc_fence_after();
-        const int kv0 = (g.top - j) * kBlockN;
+        const int kv0 = (g.split ? g.top - 2 * j - s : g.top - j) * kBlockN;
         // One body, instantiated twice: tiles cut by a mask boundary (or by the end of the sequence) take the
         // per-element predicate, all others carry none of that code. (Blanking a cut tile in tensor memory first
         // and sharing one body saved 10 KB of instructions but made every tile 4 % slower: the body then
@@ -438,7 +458,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
           // (no hand-over on the first tile of an item: there is nothing to rescale yet, and the correction warps
           // may still be in the previous item's epilogue)
-          sAlpha[s * kBlockM + row_l] = alpha;
+          if (j != j_lo) sAlpha[s * kBlockM + row_l] = alpha;
           __syncwarp();
           if (lane == 0 && j != j_lo) mbar_arrive(&alpha_ready[s]);
           const float neg_ms = -m_used * sl2;
@@ -473,11 +493,14 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       // they do that after their epilogue of the previous item, which reads the sums first.
       if (!mbar_wait_warp(&p_full[s], (n_s - 1) & 1, abort_flag)) break;
       sRowSum[s * kBlockM + row_l] = l_run;
+      // a split item's epilogue also needs the reference the sums are taken against; the rescale factors of this item
+      // have all been read, and the next item's first factor is written after its first P.V, i.e. after that epilogue
+      if (g.split) sAlpha[s * kBlockM + row_l] = m_used * sl2;
       __syncwarp();
       if (lane == 0) mbar_arrive(&l_ready[s]);
       // l_run = sum over visible keys of 2^((score - m_used) * sl2), so the natural-log sum of exponentials is
       // ln2 * (m_used * sl2 + log2(l_run)).
-      if (kLse && row < N)
+      if (kLse && !g.split && row < N)
         p.lse[static_cast<size_t>(g.bh) * N + row] =
             (l_run > 0.f) ? 0.6931471805599453f * fmaf(m_used, sl2, __log2f(l_run)) : -INFINITY;
     }
@@ -501,7 +524,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       ItemGeom g;
       const int item = take_item(n_items, g);
       if (item < 0) break;
-      bool epi_pending[2] = {g.r1[0] >= g.r0[0], g.r1[1] >= g.r0[1]};
+      bool epi_pending[2] = {!g.split && g.r1[0] >= g.r0[0], !g.split && g.r1[1] >= g.r0[1]};
       // O / l -> fp16 -> global for stage s, then the early arrival for the next item's first tile
       auto epilogue = [&](auto stage_tag) {
         constexpr int s = decltype(stage_tag)::value;
@@ -558,6 +581,69 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         }
         arrived_early[s] = true;
       };
+      // Split item: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)), m the larger of the
+      // two stages' references; then as above.
+      auto epilogue_split = [&]() {
+        float l[2], m[2];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (!mbar_wait_warp(&l_ready[s], n_l[s] & 1, abort_flag)) { ok = false; return; }
+          ++n_l[s];
+          l[s] = sRowSum[s * kBlockM + row_l];
+          m[s] = l[s] > 0.f ? sAlpha[s * kBlockM + row_l] : -INFINITY;
+          if (!mbar_wait_warp(&o_full[s], n_o[s] & 1, abort_flag)) { ok = false; return; }
+          ++n_o[s];
+        }
+        tc_fence_after();
+        const float m_all = fmaxf(fmaxf(m[0], m[1]), -3.0e38f);  // (a row without visible keys: both factors are 0)
+        float f0 = ex2_approx(m[0] - m_all), f1 = ex2_approx(m[1] - m_all);
+        const float l_all = l[0] * f0 + l[1] * f1;
+        const float inv_l = ((l_all > 0.f) ? 1.f / l_all : 0.f) * (kDropout ? p.drop_scale : 1.f);
+        f0 *= inv_l;
+        f1 *= inv_l;
+        const int row0 = g.r0[0] + static_cast<int>(lane_base);
+        if (kLse && row0 + lane < N)
+          p.lse[static_cast<size_t>(g.bh) * N + row0 + lane] =
+              (l_all > 0.f) ? 0.6931471805599453f * (m_all + __log2f(l_all)) : -INFINITY;
+        const uint32_t tO0 = tmem_addr(tmem_base, lane_base, Cfg::kColO0);
+        const uint32_t tO1 = tmem_addr(tmem_base, lane_base, Cfg::kColO1);
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
+#pragma unroll 1
+        for (int c = 0; c < D / 16; ++c) {
+          uint32_t ra[16], rb[16];
+          tmem_ld16(tO0 + c * 16, ra);
+          tmem_ld16(tO1 + c * 16, rb);
+          tmem_wait_ld();
+          tmem_ld_fence16(ra);
+          tmem_ld_fence16(rb);
+          uint8_t* prow = out_stage + (c >> 2) * (32 * 128) + lane * 128;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            uint32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int e = i * 8 + 2 * k;
+              v[k] = pack_f16x2(fmaf(__uint_as_float(ra[e]), f0, __uint_as_float(rb[e]) * f1),
+                                fmaf(__uint_as_float(ra[e + 1]), f0, __uint_as_float(rb[e + 1]) * f1));
+            }
+            const int unit = ((c & 3) * 2 + i) ^ (lane & 7);
+            *reinterpret_cast<uint4*>(prow + unit * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+          }
+        }
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (row0 < N) {
+            tma_store_4d(&mapO, out_stage, 0, row0, 0, g.bh);
+            tma_store_commit();
+          }
+          mbar_arrive(&p_full[0]);
+          mbar_arrive(&p_full[1]);
+        }
+        arrived_early[0] = arrived_early[1] = true;
+      };
       for (int j = 0; j < g.steps && ok; ++j) {
         // a stage that has run out of tiles is finished first, while the other stage is still in its softmax
         if (epi_pending[0] && j >= g.hi[0]) epilogue(std::integral_constant<int, 0>{});
@@ -596,6 +682,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         }
       }
       if (!ok) break;
+      if (g.split) epilogue_split();
       if (epi_pending[0]) epilogue(std::integral_constant<int, 0>{});
       if (ok && epi_pending[1]) epilogue(std::integral_constant<int, 1>{});
     }
@@ -637,20 +724,28 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         // nor among the last two (no Q release, no final commit), and tile j+1 exists
         const int in_lo = max(g.lo[0], g.lo[1]) + 1;
         const int in_hi = min(g.hi[0], g.hi[1]) - 2;
-        auto round_body = [&](auto interior_tag, int j) {
+        // In a split item every product has a kv tile of its own: the tiles lie in the ring in the order of their use,
+        // and slot_k is the next one.
+        auto round_body = [&](auto interior_tag, auto split_tag, int j) {
           constexpr bool kInterior = decltype(interior_tag)::value;
+          constexpr bool kSplit = decltype(split_tag)::value;
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
             const bool act_j = kInterior || (j >= g.lo[s] && j < g.hi[s]);
             const bool act_n = kInterior || (j + 1 >= g.lo[s] && j + 1 < g.hi[s]);
-            const bool other_j = (s == 0) && (kInterior || (j >= g.lo[1] && j < g.hi[1]));          // stage 1 still needs V_j
-            const bool other_n = (s == 0) && (kInterior || (j + 1 >= g.lo[1] && j + 1 < g.hi[1]));  // stage 1 still needs K_j+1
+            const bool other_j = !kSplit && (s == 0) && (kInterior || (j >= g.lo[1] && j < g.hi[1]));          // stage 1 still needs V_j
+            const bool other_n = !kSplit && (s == 0) && (kInterior || (j + 1 >= g.lo[1] && j + 1 < g.hi[1]));  // stage 1 still needs K_j+1
             // stage 0 already waited for this tile in the same round
-            const bool v_seen = (s == 1) && (kInterior || (j >= g.lo[0] && j < g.hi[0]));
-            const bool k_seen = (s == 1) && (kInterior || (j + 1 >= g.lo[0] && j + 1 < g.hi[0]));
+            const bool v_seen = !kSplit && (s == 1) && (kInterior || (j >= g.lo[0] && j < g.hi[0]));
+            const bool k_seen = !kSplit && (s == 1) && (kInterior || (j + 1 >= g.lo[0] && j + 1 < g.hi[0]));
             const uint32_t colS = (s == 0) ? Cfg::kColS0 : Cfg::kColS1;
             const uint32_t colO = (s == 0) ? Cfg::kColO0 : Cfg::kColO1;
             if (act_j) {  // O_s += P_s(j) V_j, in two halves of 64 keys as P arrives
+              if (kSplit) {
+                slot_v = slot_k;
+                par_v = par_k;
+                advance(slot_k, par_k, 1);
+              }
               const uint64_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
               if (!v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
               if (!mbar_wait_warp(&p_full[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
@@ -693,12 +788,19 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 if (!kInterior && j + 2 == g.hi[s]) umma_commit(&q_empty[s]);
               }
               __syncwarp();
+              if (kSplit) advance(slot_k, par_k, 1);
             }
           }
         };
+        if (g.split) {
+          for (int j = -1; j < g.steps && ok; ++j) round_body(std::false_type{}, std::true_type{}, j);
+          ring_slot = slot_k;
+          ring_par = par_k;
+          continue;
+        }
         for (int j = -1; j < g.steps && ok; ++j) {
-          if (j >= in_lo && j < in_hi) round_body(std::true_type{}, j);
-          else round_body(std::false_type{}, j);
+          if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
+          else round_body(std::false_type{}, std::false_type{}, j);
           // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
           slot_v = slot_k;
           par_v = par_k;
@@ -732,7 +834,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             w[0] = g.bh; w[1] = g.pair;
             w[2] = g.r0[0]; w[3] = g.r0[1]; w[4] = g.r1[0]; w[5] = g.r1[1];
             w[6] = g.lo[0]; w[7] = g.lo[1]; w[8] = g.hi[0]; w[9] = g.hi[1];
-            w[10] = g.top; w[11] = g.steps;
+            w[10] = g.top; w[11] = g.steps; w[13] = g.split;
           }
           w[12] = item;
           mbar_arrive(&item_full[slot]);
@@ -750,22 +852,34 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           mbar_arrive_expect_tx(&q_full[s], Cfg::kTileBytes);
           tma_load_4d(sQ + s * Cfg::kTileBytes, &mapQ, &q_full[s], 0, g.r0[s], 0, g.bh);
         }
-        for (int j = 0; j < g.steps && ok; ++j) {
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const uint32_t slot = it % Cfg::kStages;
-            if (!mbar_wait(&kv_empty[slot], ((it / Cfg::kStages) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        auto load_tile = [&](const CUtensorMap* map, int tile) {
+          const uint32_t slot = it % Cfg::kStages;
+          if (!ok || !mbar_wait(&kv_empty[slot], ((it / Cfg::kStages) & 1) ^ 1, abort_flag)) { ok = false; return; }
 #ifdef FA_TEST_WITHHOLD_LOAD  // test build only: CTA 0 never loads its fourth tile, so that a bounded wait runs out
-            if (blockIdx.x == 0 && (p.variant & 2) != 0 && it == 3) {
-              ++it;
-              continue;
-            }
-#endif
-            {
-              mbar_arrive_expect_tx(&kv_full[slot], Cfg::kTileBytes);
-              tma_load_4d(sKV + slot * Cfg::kTileBytes, t == 0 ? &mapK : &mapV, &kv_full[slot], 0, (g.top - j) * kBlockN, 0, g.bh);
-            }
+          if (blockIdx.x == 0 && (p.variant & 2) != 0 && it == 3) {
             ++it;
+            return;
+          }
+#endif
+          mbar_arrive_expect_tx(&kv_full[slot], Cfg::kTileBytes);
+          tma_load_4d(sKV + slot * Cfg::kTileBytes, map, &kv_full[slot], 0, tile * kBlockN, 0, g.bh);
+          ++it;
+        };
+        if (g.split) {  // in the order of use
+          load_tile(&mapK, g.top);
+          load_tile(&mapK, g.top - 1);
+          for (int j = 0; j < g.steps && ok; ++j) {
+#pragma unroll 1
+            for (int s = 0; s < 2; ++s) {
+              const int hi = s ? g.hi[1] : g.hi[0], tile = g.top - 2 * j - s;
+              if (j < hi) load_tile(&mapV, tile);
+              if (j + 1 < hi) load_tile(&mapK, tile - 2);
+            }
+          }
+        } else {
+          for (int j = 0; j < g.steps && ok; ++j) {
+            load_tile(&mapK, g.top - j);
+            load_tile(&mapV, g.top - j);
           }
         }
       }

@@ -195,6 +195,29 @@ def test_large_configs_sampled(pkg, ob, B, H, N, d, causal, wl):
     assert (out2.float() - 2 * out.float()).abs().max().item() <= 2.0 ** -23
 
 
+# Work items whose two stages share out the kv tiles of one q tile: one to six tiles per q tile (odd and even, a
+# second q tile without rows), windows that hide a whole stage's tiles from some rows, and launches that mix them with
+# pairs (75 heads x 2 pairs = 150 items for 148 SMs; 80 heads x 2 under a window).
+@pytest.mark.parametrize("H,N,d,causal,wl,wr", [
+    (1, 129, 64, False, -1, -1), (2, 129, 128, True, -1, -1), (2, 256, 64, True, -1, -1), (1, 300, 128, False, -1, -1),
+    (3, 385, 64, True, -1, -1), (2, 513, 128, True, -1, -1), (2, 700, 64, False, 100, 5), (2, 640, 128, True, 40, -1),
+    (75, 512, 64, False, -1, -1), (75, 333, 128, False, -1, -1), (80, 450, 64, True, 60, -1),
+])
+def test_split_items(pkg, ob, H, N, d, causal, wl, wr):
+    import torch
+
+    q, k, v = make_inputs(4000 + N + H, 1, H, N, d)
+    want = ob.attention(q, k, v, causal=causal, window_left=wl, window_right=wr)
+    assert_close_or_one_ulp(run_gpu(pkg, q, k, v, causal, wl, wr), want)
+    tq, tk, tv = (torch.from_numpy(a).cuda() for a in (q, k, v))
+    out, lse = pkg.attention_forward(tq, tk, tv, causal=causal, window_left=wl, window_right=wr, return_lse=True)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    assert_close_or_one_ulp(out.cpu().numpy(), want)
+    rows = np.arange(0, N, 7)
+    exact = ob.log_sum_exp_fp64(q[:, :2], k[:, :2], causal=causal, window_left=wl, window_right=wr, rows=rows)
+    assert np.abs(lse[:, :2].cpu().numpy()[:, :, rows] - exact).max() <= 5e-4
+
+
 def test_very_long_sequence_and_very_many_heads(pkg, ob):
     """The two ends of the work-item space: one head of 131072 rows (512 q pairs, a 64 MB K/V working set, 1024 kv
     tiles for the last rows) and 6000 heads of 256 rows (one item per head, the dynamic work counter hands out
