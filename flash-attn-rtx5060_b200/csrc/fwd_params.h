@@ -22,6 +22,7 @@ struct FwdParams {
   int window_left;   // j >= i - window_left   (< 0: unbounded)
   int window_right;  // j <= i + window_right  (< 0: unbounded); forced to 0 by `causal`
   int* status;       // device word, 0 = ok; set non-zero when a bounded wait gave up
+  int status_per_launch;  // 1: the word is this launch's alone (the launch also writes the 0)
   float* dbg;        // optional bring-up dump (serial kernel only), else nullptr
   int variant;       // bit0 (serial kernel): P through shared memory instead of TMEM; bit1 (test build of the
                      // persistent kernel only): CTA 0 withholds one tile so that a bounded wait runs out
@@ -44,7 +45,8 @@ struct FwdParams {
   unsigned seed_lo, seed_hi;
   float drop_scale;         // 256 / drop_keep_thr: the kept elements' 1 / (1 - p), folded into the epilogue
   int* sched;        // device scratch, two words that are 0 between launches: [0] next work item to
-                     // hand out (beyond the first gridDim.x), [1] CTAs that have finished
+                     // hand out (beyond the first gridDim.x), [1] CTAs that have finished (bits 0-15) and CTAs that
+                     // gave up (bits 16-31)
 };
 
 // Visible key range of query row i is [i - wl, i + wr] ∩ [0, N-1] with "unbounded" for

@@ -290,6 +290,9 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Everything above overlaps the end of the kernel in front in the stream; nothing below this line has touched
+  // global memory (inputs, outputs, scheduler words, status) before that kernel is complete.
+  griddep_wait();
 
   const int N = p.seqlen;
   const int wl = p.window_left;
@@ -843,7 +846,10 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (item < 0) break;
         // claim the following item now; the value is not needed before this item's loads are issued
         next = static_cast<int>(gridDim.x) + atomicAdd(p.sched, 1);
-        if (next >= p.num_items) next = -1;
+        if (next >= p.num_items) {
+          next = -1;
+          griddep_launch();  // the last item of this CTA: the next kernel of the stream may take up free SMs
+        }
 #pragma unroll
         for (int s = 1; s >= 0; --s) {  // stage 1 reaches further to the right and starts first
           if (g.r1[s] < g.r0[s]) continue;
@@ -893,9 +899,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   tc_fence_before();
   __syncthreads();
   if (tid == 0) {
-    if (*abort_flag != 0) atomicExch(p.status, 1);
+    const int gave_up = *abort_flag != 0 ? 1 : 0;
+    if (gave_up) atomicExch(p.status, 1);
     // the last CTA to finish puts the scheduler words back to zero for the next launch
-    if (atomicAdd(p.sched + 1, 1) == static_cast<int>(gridDim.x) - 1) {
+    const int ended = atomicAdd(p.sched + 1, 1 + (gave_up << 16)) + 1 + (gave_up << 16);
+    if ((ended & 0xffff) == static_cast<int>(gridDim.x)) {
+      if (p.status_per_launch) *p.status = (ended >> 16) != 0 ? 1 : 0;
       p.sched[0] = 0;
       p.sched[1] = 0;
       __threadfence();

@@ -78,6 +78,13 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   return r;
 }
 
+// Programmatic dependent launch: a grid launched with that attribute may start before the grid in front of it in the
+// stream has ended. griddep_wait() holds a thread until that grid has completed and its memory is visible;
+// griddep_launch() (once per CTA) lets the grid behind this one start where SMs are free. Both do nothing in a grid
+// that was launched without the attribute or has no such successor.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------

@@ -338,6 +338,40 @@ def test_many_launches_on_two_streams(pkg):
         assert torch.equal(o, want)
 
 
+def test_chained_launches_and_more_streams_than_owned_scheduler_words(pkg):
+    """A launch may start before the one in front of it in the stream has ended: a chain in which every call reads the
+    previous call's output must give the bits of the same chain with a wait after each call. And 60 streams, more than
+    own scheduler words of their own, with three launches in flight on each."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn((1, 6, 700, 64), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    chains = []
+    for wait in (True, False):
+        x = q
+        for i in range(40):
+            x = pkg.attention_forward(x, k, v, causal=bool(i & 1))
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        chains.append(x)
+    assert torch.equal(chains[0], chains[1])
+    want = pkg.attention_forward(q, k, v, causal=True)
+    streams = [torch.cuda.Stream(priority=-(i & 1)) for i in range(60)]
+    outs = [[torch.empty_like(q) for _ in range(3)] for _ in streams]
+    torch.cuda.synchronize()
+    for r in range(3):
+        for st, o in zip(streams, outs):
+            with torch.cuda.stream(st):
+                pkg.attention_forward(q, k, v, causal=True, out=o[r])
+    torch.cuda.synchronize()
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    assert len({st.cuda_stream for st in streams}) > 40
+    for o in outs:
+        for x in o:
+            assert torch.equal(x, want)
+
+
 def exact_attention(q, k, v, scale, causal):
     """fp64 attention of fp16 inputs (numpy), rounded once to fp16: the error-free answer."""
     q64, k64, v64 = (a.astype(np.float64) for a in (q, k, v))
