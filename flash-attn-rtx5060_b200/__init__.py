@@ -196,39 +196,44 @@ def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, so
 
     assert q.is_cuda and q.dtype == torch.float16 and q.is_contiguous() and q.dim() == 4
     assert k.shape == q.shape and v.shape == q.shape and k.is_contiguous() and v.is_contiguous()
-    B, H, N, d = q.shape
     if out is None:
         out = torch.empty_like(q)
-    stream = torch.cuda.current_stream(q.device).cuda_stream
-    with torch.cuda.device(q.device):
-        if alibi_slopes is not None:
-            assert alibi_slopes.is_cuda and alibi_slopes.dtype == torch.float32 and alibi_slopes.numel() == H
-        if dropout_p > 0.0:
-            assert kernel == 0 and variant == 0 and not return_lse
-            rc = lib().flash_forward_dropout(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d,
-                                             softmax_scale, int(bool(causal)), window_left, window_right,
-                                             None if alibi_slopes is None else alibi_slopes.data_ptr(), dropout_p,
-                                             seed, stream)
-            if rc != FA_OK:
-                _raise(rc)
-            return out
-        if return_lse:
-            assert kernel == 0 and variant == 0
-            lse = torch.empty((B, H, N), device=q.device, dtype=torch.float32)
-            rc = lib().flash_forward_lse(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, H,
-                                         N, d, softmax_scale, int(bool(causal)), window_left, window_right,
-                                         None if alibi_slopes is None else alibi_slopes.data_ptr(), stream)
-            if rc != FA_OK:
-                _raise(rc)
-            return out, lse
-        if alibi_slopes is not None:  # float32 CUDA tensor with one slope per head
-            assert alibi_slopes.is_cuda and alibi_slopes.dtype == torch.float32 and alibi_slopes.numel() == H
-            rc = lib().flash_forward_alibi(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d,
-                                           softmax_scale, int(bool(causal)), window_left, window_right,
-                                           alibi_slopes.data_ptr(), stream)
-            if rc != FA_OK:
-                _raise(rc)
-        else:
-            flash_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, softmax_scale, causal,
-                          window_left, window_right, stream, kernel, variant)
-    return out
+    args = (torch, q, k, v, out, causal, window_left, window_right, softmax_scale, kernel, variant, alibi_slopes,
+            return_lse, dropout_p, seed)
+    device = q.get_device()
+    if device == torch.cuda.current_device():
+        return _enqueue_forward(device, *args)
+    with torch.cuda.device(device):
+        return _enqueue_forward(device, *args)
+
+
+def _enqueue_forward(device, torch, q, k, v, out, causal, window_left, window_right, softmax_scale, kernel, variant,
+                     alibi_slopes, return_lse, dropout_p, seed):
+    # The raw handle of the current stream: building a torch.cuda.Stream object and entering a device context for every
+    # call cost 5 us of the 14 us a call took on the host, more than the kernel of a small call (B1 H4 N512 d64).
+    stream = torch._C._cuda_getCurrentRawStream(device)
+    B, H, N, d = q.shape
+    L = lib()
+    lse = None
+    if alibi_slopes is not None:  # float32 CUDA tensor with one slope per head
+        assert alibi_slopes.is_cuda and alibi_slopes.dtype == torch.float32 and alibi_slopes.numel() == H
+    if dropout_p > 0.0:
+        assert kernel == 0 and variant == 0 and not return_lse
+        rc = L.flash_forward_dropout(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, softmax_scale,
+                                     int(bool(causal)), window_left, window_right,
+                                     None if alibi_slopes is None else alibi_slopes.data_ptr(), dropout_p, seed, stream)
+    elif return_lse:
+        assert kernel == 0 and variant == 0
+        lse = torch.empty((B, H, N), device=q.device, dtype=torch.float32)
+        rc = L.flash_forward_lse(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, H, N, d,
+                                 softmax_scale, int(bool(causal)), window_left, window_right,
+                                 None if alibi_slopes is None else alibi_slopes.data_ptr(), stream)
+    elif alibi_slopes is not None:
+        rc = L.flash_forward_alibi(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, softmax_scale,
+                                   int(bool(causal)), window_left, window_right, alibi_slopes.data_ptr(), stream)
+    else:
+        rc = L.flash_forward_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, softmax_scale,
+                                int(bool(causal)), window_left, window_right, stream, kernel, variant, None)
+    if rc != FA_OK:
+        _raise(rc)
+    return (out, lse) if return_lse else out
