@@ -844,20 +844,15 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           ++n_pub;
         }
         if (item < 0) break;
-        // claim the following item now; the value is not needed before this item's loads are issued
-        next = static_cast<int>(gridDim.x) + atomicAdd(p.sched, 1);
-        if (next >= p.num_items) {
-          next = -1;
-          griddep_launch();  // the last item of this CTA: the next kernel of the stream may take up free SMs
-        }
-#pragma unroll
-        for (int s = 1; s >= 0; --s) {  // stage 1 reaches further to the right and starts first
-          if (g.r1[s] < g.r0[s]) continue;
-          if (!mbar_wait(&q_empty[s], (n_q[s] & 1) ^ 1, abort_flag)) { ok = false; break; }
+        // Claim the following item now; the answer is looked at behind this item's loads.
+        const int claimed = atomicAdd(p.sched, 1);
+        auto load_q = [&](int s) {
+          if (g.r1[s] < g.r0[s]) return;
+          if (!ok || !mbar_wait(&q_empty[s], (n_q[s] & 1) ^ 1, abort_flag)) { ok = false; return; }
           ++n_q[s];
           mbar_arrive_expect_tx(&q_full[s], Cfg::kTileBytes);
           tma_load_4d(sQ + s * Cfg::kTileBytes, &mapQ, &q_full[s], 0, g.r0[s], 0, g.bh);
-        }
+        };
         auto load_tile = [&](const CUtensorMap* map, int tile) {
           const uint32_t slot = it % Cfg::kStages;
           if (!ok || !mbar_wait(&kv_empty[slot], ((it / Cfg::kStages) & 1) ^ 1, abort_flag)) { ok = false; return; }
@@ -871,8 +866,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           tma_load_4d(sKV + slot * Cfg::kTileBytes, map, &kv_full[slot], 0, tile * kBlockN, 0, g.bh);
           ++it;
         };
+        // The Q tiles of the previous item are released one after the other, stage 0 first; the ring slots of the
+        // first kv tiles usually before either.
+        if (g.steps > 0) load_tile(&mapK, g.top);
+        load_q(0);
+        load_q(1);
         if (g.split) {  // in the order of use
-          load_tile(&mapK, g.top);
           load_tile(&mapK, g.top - 1);
           for (int j = 0; j < g.steps && ok; ++j) {
 #pragma unroll 1
@@ -884,9 +883,14 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
         } else {
           for (int j = 0; j < g.steps && ok; ++j) {
-            load_tile(&mapK, g.top - j);
             load_tile(&mapV, g.top - j);
+            if (j + 1 < g.steps) load_tile(&mapK, g.top - j - 1);
           }
+        }
+        next = static_cast<int>(gridDim.x) + claimed;
+        if (next >= p.num_items) {
+          next = -1;
+          griddep_launch();  // this CTA takes no further item: the next kernel of the stream may take up free SMs
         }
       }
       if (!ok) {

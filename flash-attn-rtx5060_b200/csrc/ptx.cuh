@@ -130,19 +130,36 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   // The first probe stands alone and the retry loop holds nothing but the probe and a counter: what sits between
   // two probes is added to every hand-off in the kernels (a loop that also read the abort flag after each probe
-  // cost 5 % of the whole attention kernel).
-  if (mbar_try_wait(bar, parity)) return true;
-  uint32_t polls = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++polls & 63u) == 0) {
-      if (*abort_flag != 0) return false;
-      if (polls >= FA_WAIT_LIMIT_POLLS) {
-        *abort_flag = 1;
-        return false;
-      }
-    }
-  }
-  return true;
+  // cost 5 % of the whole attention kernel). Written as one block of PTX, a wait is 11 instructions in each of its
+  // many places; as C++ around single probes it came to 40, 27 KB of the kernel, and the first and last rounds of an
+  // item, whose code is rarely in the instruction caches, ran slower: B4 H16 N2048 d64 causal 72.0 -> 67.8 us, B8 H12
+  // N1000 d64 54.5 -> 51.6, B8 H16 N1024 d128 61.5 -> 58.2.
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred P, Q;\n"
+      ".reg .u32 n, f;\n"
+      "mov.u32 n, 0;\n"
+      "PROBE:\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n"
+      "@P bra DONE;\n"
+      "add.u32 n, n, 1;\n"
+      "and.b32 f, n, 63;\n"
+      "setp.ne.u32 Q, f, 0;\n"
+      "@Q bra PROBE;\n"
+      "ld.volatile.shared.u32 f, [%3];\n"
+      "setp.ne.u32 Q, f, 0;\n"
+      "@Q bra DONE;\n"
+      "setp.lt.u32 Q, n, %4;\n"
+      "@Q bra PROBE;\n"
+      "st.volatile.shared.u32 [%3], 1;\n"
+      "DONE:\n"
+      "selp.u32 %0, 1, 0, P;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<int*>(abort_flag))), "n"(FA_WAIT_LIMIT_POLLS)
+      : "memory");
+  return ok != 0;
 }
 
 // Same, for a whole warp polling one barrier: the verdict is made warp-uniform so that a
