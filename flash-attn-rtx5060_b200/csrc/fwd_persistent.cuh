@@ -700,11 +700,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       constexpr uint32_t idesc_qk = umma_idesc_f16(kBlockM, kBlockN, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_f16(kBlockM, D, 0, 1);
       // Descriptors are built once; per instruction only the 16-byte-unit start address moves.
-      const uint64_t kdesc0 = umma_desc_sw128(0, 16, 1024);               // K-major tiles (Q, K)
-      const uint64_t vdesc0 = umma_desc_sw128(0, Cfg::kPanelBytes, 1024);  // MN-major tile (V)
+      const uint32_t kdesc0 = static_cast<uint32_t>(umma_desc_sw128(0, 16, 1024));  // K-major tiles (Q, K), low word
+      const uint32_t vdesc0 = static_cast<uint32_t>(umma_desc_sw128(0, Cfg::kPanelBytes, 1024));  // MN-major tile (V)
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // row stride, version, 128-byte swizzle
       const uint32_t q_addr = smem_u32(sQ);
       const uint32_t kv_addr = smem_u32(sKV);
-      const uint64_t qdesc[2] = {kdesc0 + (q_addr >> 4), kdesc0 + ((q_addr + Cfg::kTileBytes) >> 4)};
+      const uint32_t qdesc[2] = {kdesc0 + (q_addr >> 4), kdesc0 + ((q_addr + Cfg::kTileBytes) >> 4)};
       uint32_t ring_slot = 0, ring_par = 0;  // ring position (slot, phase parity) of the first K tile of the current item
       uint32_t n_p[2] = {0, 0}, n_q[2] = {0, 0};
       uint32_t n_items = 0;
@@ -749,15 +750,15 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 par_v = par_k;
                 advance(slot_k, par_k, 1);
               }
-              const uint64_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
+              const uint32_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
               if (!v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
               if (!mbar_wait_warp(&p_full[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
               tc_fence_after();
               if (elect_one()) {
-                umma_ts(tmem_base + colO, tmem_base + colS, vdesc, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
+                umma_ts_lo(tmem_base + colO, tmem_base + colS, vdesc, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
 #pragma unroll
                 for (int kk = 1; kk < 4; ++kk)
-                  umma_ts(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), idesc_pv, 1u);
+                  umma_ts_lo(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
               }
               __syncwarp();
               if (!mbar_wait_warp(&p_full2[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
@@ -766,7 +767,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               if (elect_one()) {
 #pragma unroll
                 for (int kk = 4; kk < 8; ++kk)
-                  umma_ts(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), idesc_pv, 1u);
+                  umma_ts_lo(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
                 if (!other_j) umma_commit(&kv_empty[slot_v]);
                 if (!kInterior && j + 1 == g.hi[s]) umma_commit(&o_full[s]);
               }
@@ -779,12 +780,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               }
               if (!k_seen && !mbar_wait_warp(&kv_full[slot_k], par_k, abort_flag)) { ok = false; return; }
               tc_fence_after();
-              const uint64_t kdesc = kdesc0 + ((kv_addr + slot_k * Cfg::kTileBytes) >> 4);
+              const uint32_t kdesc = kdesc0 + ((kv_addr + slot_k * Cfg::kTileBytes) >> 4);
               if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < D / 16; ++k) {
                   const uint32_t off = ((k / 4) * Cfg::kPanelBytes + (k % 4) * 32) >> 4;
-                  umma_ss(tmem_base + colS, qdesc[s] + off, kdesc + off, idesc_qk, k > 0 ? 1u : 0u);
+                  umma_ss_lo(tmem_base + colS, qdesc[s] + off, kdesc + off, kDescHi, idesc_qk, k > 0 ? 1u : 0u);
                 }
                 umma_commit(&s_full[s]);
                 if (!other_n) umma_commit(&kv_empty[slot_k]);

@@ -283,6 +283,37 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with descriptors given as their low words (start address and leading-dimension offset); the high words are
+// constants, so that only one 32-bit addition per operand and instruction remains.
+__device__ __forceinline__ void umma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b64 a, b;\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "mov.b64 a, {%1, %3};\n"
+      "mov.b64 b, {%2, %3};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b64 b;\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "mov.b64 b, {%2, %3};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // The mbarrier receives one arrival when every tcgen05 operation issued so far by this
 // thread has completed. Implies tcgen05.fence::before_thread_sync.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
