@@ -730,6 +730,11 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int in_hi = min(g.hi[0], g.hi[1]) - 2;
         // In a split item every product has a kv tile of its own: the tiles lie in the ring in the order of their use,
         // and slot_k is the next one.
+        auto wait_next_v = [&]() {  // V_{j+1} lies behind K_{j+1}
+          uint32_t slot = slot_k, par = par_k;
+          advance(slot, par, 1);
+          return mbar_wait_warp(&kv_full[slot], par, abort_flag);
+        };
         auto round_body = [&](auto interior_tag, auto split_tag, int j) {
           constexpr bool kInterior = decltype(interior_tag)::value;
           constexpr bool kSplit = decltype(split_tag)::value;
@@ -751,7 +756,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 advance(slot_k, par_k, 1);
               }
               const uint32_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
-              if (!v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
+              if (!kInterior && !v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
               if (!mbar_wait_warp(&p_full[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
               tc_fence_after();
               if (elect_one()) {
@@ -779,6 +784,9 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 ++n_q[s];
               }
               if (!k_seen && !mbar_wait_warp(&kv_full[slot_k], par_k, abort_flag)) { ok = false; return; }
+              // Inner rounds wait for V here, one round ahead: every group of instructions then has one wait in front
+              // of it, about as long as the tensor pipe has work queued (two waits in a row let it run dry).
+              if (kInterior && s == 1 && !wait_next_v()) { ok = false; return; }
               tc_fence_after();
               const uint32_t kdesc = kdesc0 + ((kv_addr + slot_k * Cfg::kTileBytes) >> 4);
               if (elect_one()) {
@@ -803,6 +811,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           continue;
         }
         for (int j = -1; j < g.steps && ok; ++j) {
+          if (j == in_lo && in_lo < in_hi) ok = mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag);
           if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
           else round_body(std::false_type{}, std::false_type{}, j);
           // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
