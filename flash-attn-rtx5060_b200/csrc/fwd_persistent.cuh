@@ -200,6 +200,7 @@ __device__ __forceinline__ void philox4x32_10(uint32_t k0, uint32_t k1, uint32_t
 // multiple of 16) of query row `row` of head `bh`. One Philox call serves 16 columns: byte t of its 16 output bytes
 // (little endian over the four words) decides column 16 * block + t.
 __device__ __forceinline__ void dropout_mask_64(uint32_t (&pk)[32], const FwdParams& p, int bh, int row, int col0) {
+  constexpr uint32_t kHigh = 0x80808080u;
   const uint32_t thr4 = p.drop_keep_thr * 0x01010101u;
 #pragma unroll
   for (int blk = 0; blk < 4; ++blk) {
@@ -208,9 +209,15 @@ __device__ __forceinline__ void dropout_mask_64(uint32_t (&pk)[32], const FwdPar
                   static_cast<uint32_t>(bh), 0u, r);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const uint32_t keep = __vcmpltu4(r[w], thr4);                // 0xff in every byte below the threshold
-      pk[blk * 8 + 2 * w] &= __byte_perm(keep, 0u, 0x1100);        // columns 4w, 4w+1
-      pk[blk * 8 + 2 * w + 1] &= __byte_perm(keep, 0u, 0x3322);    // columns 4w+2, 4w+3
+      // High bit of each byte of `ge`: the byte is not below the threshold (a subtraction that borrows within bytes).
+      // A byte permute with the sign-replicating selectors 8 + b spreads these bits over the halves of two words.
+      const uint32_t diff = (r[w] | kHigh) - (thr4 & ~kHigh);
+      const uint32_t ge = (r[w] & ~thr4) | (~(r[w] ^ thr4) & diff);
+      uint32_t lo, hi;
+      asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(lo) : "r"(ge));
+      asm("prmt.b32 %0, %1, 0, 0xBBAA;" : "=r"(hi) : "r"(ge));
+      pk[blk * 8 + 2 * w] &= ~lo;      // columns 4w, 4w+1
+      pk[blk * 8 + 2 * w + 1] &= ~hi;  // columns 4w+2, 4w+3
     }
   }
 }
