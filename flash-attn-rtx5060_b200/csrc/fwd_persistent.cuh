@@ -522,28 +522,28 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     uint8_t* out_stage = smem + Cfg::kOffOut + (warp & 3) * Cfg::kOutWarpBytes;
-    uint32_t n_alpha[2] = {0, 0}, n_l[2] = {0, 0}, n_o[2] = {0, 0};
+    // Bit s: phase parity of stage s's barriers. The stages share one copy of this code (rolled loops, state in bit
+    // masks): with copies for both and the epilogue in four places it was 38 KB, mostly run from cold instructions.
+    uint32_t par_alpha = 0, par_l = 0, par_o = 0;
     uint32_t n_items = 0;
     // The first P.V product of an item overwrites O, so it has to wait until the epilogue of the previous item
     // has read O. That hand-off is the correction warps' arrival on p_full for the item's first tile; it is made
     // right after the epilogue (there is nothing to rescale on a first tile), so the next item's first product
     // does not wait for these warps to come round to it.
-    bool arrived_early[2] = {false, false};
+    uint32_t arrived_early = 0;  // bit s
     bool ok = true;
     while (ok) {
       ItemGeom g;
       const int item = take_item(n_items, g);
       if (item < 0) break;
-      bool epi_pending[2] = {!g.split && g.r1[0] >= g.r0[0], !g.split && g.r1[1] >= g.r0[1]};
+      uint32_t epi_pending = g.split ? 0u : (g.r1[0] >= g.r0[0] ? 1u : 0u) | (g.r1[1] >= g.r0[1] ? 2u : 0u);  // bit s
       // O / l -> fp16 -> global for stage s, then the early arrival for the next item's first tile
-      auto epilogue = [&](auto stage_tag) {
-        constexpr int s = decltype(stage_tag)::value;
-        epi_pending[s] = false;
-        if (!mbar_wait_warp(&l_ready[s], n_l[s] & 1, abort_flag)) { ok = false; return; }
-        ++n_l[s];
+      auto epilogue = [&](int s) {
+        if (!mbar_wait_warp(&l_ready[s], (par_l >> s) & 1, abort_flag)) { ok = false; return; }
+        par_l ^= 1u << s;
         const float l = sRowSum[s * kBlockM + row_l];
-        if (!mbar_wait_warp(&o_full[s], n_o[s] & 1, abort_flag)) { ok = false; return; }
-        ++n_o[s];
+        if (!mbar_wait_warp(&o_full[s], (par_o >> s) & 1, abort_flag)) { ok = false; return; }
+        par_o ^= 1u << s;
         tc_fence_after();
         const float inv_l = ((l > 0.f) ? 1.f / l : 0.f) * (kDropout ? p.drop_scale : 1.f);
         const uint32_t tO = tmem_addr(tmem_base, lane_base, s == 0 ? Cfg::kColO0 : Cfg::kColO1);
@@ -582,14 +582,14 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          const int row0 = g.r0[s] + static_cast<int>(lane_base);
+          const int row0 = (s ? g.r0[1] : g.r0[0]) + static_cast<int>(lane_base);
           if (row0 < N) {  // rows of the box beyond the sequence are clipped by the store
             tma_store_4d(&mapO, out_stage, 0, row0, 0, g.bh);
             tma_store_commit();
           }
           mbar_arrive(&p_full[s]);
         }
-        arrived_early[s] = true;
+        arrived_early |= 1u << s;
       };
       // Split item: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)), m the larger of the
       // two stages' references; then as above.
@@ -597,13 +597,13 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         float l[2], m[2];
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
-          if (!mbar_wait_warp(&l_ready[s], n_l[s] & 1, abort_flag)) { ok = false; return; }
-          ++n_l[s];
+          if (!mbar_wait_warp(&l_ready[s], (par_l >> s) & 1, abort_flag)) { ok = false; return; }
           l[s] = sRowSum[s * kBlockM + row_l];
           m[s] = l[s] > 0.f ? sAlpha[s * kBlockM + row_l] : -INFINITY;
-          if (!mbar_wait_warp(&o_full[s], n_o[s] & 1, abort_flag)) { ok = false; return; }
-          ++n_o[s];
+          if (!mbar_wait_warp(&o_full[s], (par_o >> s) & 1, abort_flag)) { ok = false; return; }
         }
+        par_l ^= 3u;
+        par_o ^= 3u;
         tc_fence_after();
         const float m_all = fmaxf(fmaxf(m[0], m[1]), -3.0e38f);  // (a row without visible keys: both factors are 0)
         float f0 = ex2_approx(m[0] - m_all), f1 = ex2_approx(m[1] - m_all);
@@ -652,23 +652,26 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           mbar_arrive(&p_full[0]);
           mbar_arrive(&p_full[1]);
         }
-        arrived_early[0] = arrived_early[1] = true;
+        arrived_early = 3u;
       };
-      for (int j = 0; j < g.steps && ok; ++j) {
-        // a stage that has run out of tiles is finished first, while the other stage is still in its softmax
-        if (epi_pending[0] && j >= g.hi[0]) epilogue(std::integral_constant<int, 0>{});
-        if (epi_pending[1] && j >= g.hi[1]) epilogue(std::integral_constant<int, 1>{});
-        if (!ok) break;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          if (j < g.lo[s] || j >= g.hi[s]) continue;
-          if (j == g.lo[s]) {  // first tile of the item: nothing to rescale, and no factors are handed over
-            const bool done = arrived_early[s];
-            arrived_early[s] = false;
+      for (int j = 0; j <= g.steps && ok; ++j) {
+#pragma unroll 1
+        for (int s = 0; s < 2 && ok; ++s) {
+          const int lo = s ? g.lo[1] : g.lo[0], hi = s ? g.hi[1] : g.hi[0];
+          // a stage that has run out of tiles is finished at once, while the other stage may still be in its softmax
+          if (((epi_pending >> s) & 1) && j >= hi) {
+            epi_pending &= ~(1u << s);
+            epilogue(s);
+            continue;
+          }
+          if (j < lo || j >= hi) continue;
+          if (j == lo) {  // first tile of the item: nothing to rescale, and no factors are handed over
+            const bool done = (arrived_early >> s) & 1;
+            arrived_early &= ~(1u << s);
             if (done) continue;
           } else {
-            if (!mbar_wait_warp(&alpha_ready[s], n_alpha[s] & 1, abort_flag)) { ok = false; break; }
-            ++n_alpha[s];
+            if (!mbar_wait_warp(&alpha_ready[s], (par_alpha >> s) & 1, abort_flag)) { ok = false; break; }
+            par_alpha ^= 1u << s;
             const float alpha = sAlpha[s * kBlockM + row_l];
             if (__any_sync(0xffffffffu, alpha != 1.f)) {
               tc_fence_after();
@@ -691,10 +694,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           if (lane == 0) mbar_arrive(&p_full[s]);
         }
       }
-      if (!ok) break;
-      if (g.split) epilogue_split();
-      if (epi_pending[0]) epilogue(std::integral_constant<int, 0>{});
-      if (ok && epi_pending[1]) epilogue(std::integral_constant<int, 1>{});
+      if (ok && g.split) epilogue_split();
     }
     if (lane == 0) tma_store_wait_all();  // also on the give-up path: stores in flight read this CTA's shared memory
   } else {
