@@ -45,10 +45,11 @@ enum {
  * The call returns once the kernel is enqueued; use flash_forward_check() to learn whether a
  * device-side wait timed out.
  *
- * Launches in flight: every launch takes one of 64 pairs of scheduler words (device scratch of a
- * few hundred bytes, allocated on the first call per device) in turn. Launches on one stream are
- * ordered anyway; when a pair is reused by a launch on ANOTHER stream, that stream is first made to
- * wait (cudaStreamWaitEvent) for the earlier launch, so any number of launches may be queued on any
+ * Launches in flight: every launch uses a pair of scheduler words (device scratch of a few hundred bytes,
+ * allocated on the first call per device). The first 40 streams that are used on a device own a pair each
+ * (launches on one stream are ordered anyway); launches on further streams take 24 more in turn, and when a
+ * pair is reused by a launch on ANOTHER stream, that stream is first made to wait (cudaStreamWaitEvent)
+ * for the earlier launch. So any number of launches may be queued on any
  * number of streams. A call whose stream is being captured into a CUDA graph is refused with
  * FA_UNSUPPORTED: a captured launch would keep its pair for every replay. flash_forward_noalloc, whose
  * scratch slot the caller chooses, is the entry point to capture.
@@ -207,8 +208,8 @@ int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int windo
  *         non-zero: block until the kernel has finished and return FA_DEVICE_TIMEOUT if its status
  *         word was set.
  *
- * All other arguments as for flash_forward(). A slot keeps the contents the last call left in it;
- * every call first clears its slot on `stream`. Calls that use the same slot must not overlap on
+ * All other arguments as for flash_forward(). Every launch leaves its slot's work counter at zero and its own
+ * verdict in the status word. Calls that use the same slot must not overlap on
  * the GPU (they would share one work counter and race); calls on different slots may.
  * The first call on a device performs a one-time set-up (looks up the scratch array's device
  * address, sets the kernel's shared-memory attribute); make that first call before any stream
