@@ -45,6 +45,9 @@ enum {
  * The call returns once the kernel is enqueued; use flash_forward_check() to learn whether a
  * device-side wait timed out.
  *
+ * Two calls with the same arguments give the same bits. The split of the work among the SMs depends on
+ * batch*heads, so a head may differ in the last place between a call on all heads and a call on some of them.
+ *
  * Launches in flight: every launch uses a pair of scheduler words (device scratch of a few hundred bytes,
  * allocated on the first call per device). The first 40 streams that are used on a device own a pair each
  * (launches on one stream are ordered anyway); launches on further streams take 24 more in turn, and when a
