@@ -713,20 +713,95 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       const uint32_t q_addr = smem_u32(sQ);
       const uint32_t kv_addr = smem_u32(sKV);
       const uint32_t qdesc[2] = {kdesc0 + (q_addr >> 4), kdesc0 + ((q_addr + Cfg::kTileBytes) >> 4)};
-      uint32_t ring_slot = 0, ring_par = 0;  // ring position (slot, phase parity) of the first K tile of the current item
-      uint32_t n_p[2] = {0, 0}, n_q[2] = {0, 0};
+      uint32_t pos = 0;               // ring position (tiles since the start) of the first K tile of the current item
+      uint32_t par_p = 0, par_q = 0;  // bit s: phase parity of stage s's barriers
       uint32_t n_items = 0;
       bool ok = true;
+      auto take_nonempty = [&](ItemGeom& g) {
+        while (take_item(n_items, g) >= 0)
+          if (g.steps > 0) return true;
+        g.steps = g.split = g.lo[0] = g.lo[1] = g.hi[0] = g.hi[1] = 0;
+        return false;
+      };
+      // Head_dim 64: the round between two items issues the last P.V of item `a`, whose tiles end at ring position `end`,
+      // and behind each stage's the first score tile of item `b`, so that a stage's softmax goes on while the other
+      // stage's last tile is still under way. Either may be missing (no steps). B200, us: B8 H12 N1000 50.6 -> 49.3,
+      // 32 heads of 8192 rows 748 -> 737 without a mask, ALiBi B2 H16 N4096 133.0 -> 131.3, B4 H16 N2048 causal
+      // 65.2 -> 64.7. At head_dim 128 long sequences do not change and B8 H16 N1024 causal loses 2.6 %, so there an
+      // item's rounds end before the next item's begin.
+      constexpr bool kJoin = D == 64;
+      auto join = [&](const ItemGeom& a, const ItemGeom& b, uint32_t end) {
+        const int j = a.steps - 1;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const int alo = s ? a.lo[1] : a.lo[0], ahi = s ? a.hi[1] : a.hi[0];
+          const int blo = s ? b.lo[1] : b.lo[0], bhi = s ? b.hi[1] : b.hi[0];
+          const uint32_t tS = tmem_base + (s ? Cfg::kColS1 : Cfg::kColS0);
+          if (j >= alo && j < ahi) {  // O_s += P_s V
+            const uint32_t tO = tmem_base + (s ? Cfg::kColO1 : Cfg::kColO0);
+            const uint32_t pv = end - ((a.split && s == 0 && j < a.hi[1]) ? 2 : 1);
+            const uint32_t slot = pv % Cfg::kStages;
+            const uint32_t vdesc = vdesc0 + ((kv_addr + slot * Cfg::kTileBytes) >> 4);
+            if (!mbar_wait_warp(&kv_full[slot], (pv / Cfg::kStages) & 1, abort_flag)) { ok = false; return; }
+            if (!mbar_wait_warp(&p_full[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
+            tc_fence_after();
+            if (elect_one()) {
+              umma_ts_lo(tO, tS, vdesc, kDescHi, idesc_pv, j > alo ? 1u : 0u);
+#pragma unroll
+              for (int kk = 1; kk < 4; ++kk) umma_ts_lo(tO, tS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
+            }
+            __syncwarp();
+            if (!mbar_wait_warp(&p_full2[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
+            par_p ^= 1u << s;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+              for (int kk = 4; kk < 8; ++kk) umma_ts_lo(tO, tS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
+              if (a.split || s == 1 || j < a.lo[1] || j >= a.hi[1]) umma_commit(&kv_empty[slot]);
+              umma_commit(&o_full[s]);
+            }
+            __syncwarp();
+          }
+          if (blo == 0 && bhi > 0) {  // S_s = Q_s K^T
+            const uint32_t pk = end + (b.split ? s : 0);
+            const uint32_t slot = pk % Cfg::kStages;
+            if (!mbar_wait_warp(&q_full[s], (par_q >> s) & 1, abort_flag)) { ok = false; return; }
+            par_q ^= 1u << s;
+            if (!mbar_wait_warp(&kv_full[slot], (pk / Cfg::kStages) & 1, abort_flag)) { ok = false; return; }
+            tc_fence_after();
+            const uint32_t kdesc = kdesc0 + ((kv_addr + slot * Cfg::kTileBytes) >> 4);
+            const uint32_t qd = s ? qdesc[1] : qdesc[0];
+            if (elect_one()) {
+#pragma unroll
+              for (int k = 0; k < D / 16; ++k) {
+                const uint32_t off = ((k / 4) * Cfg::kPanelBytes + (k % 4) * 32) >> 4;
+                umma_ss_lo(tS, qd + off, kdesc + off, kDescHi, idesc_qk, k > 0 ? 1u : 0u);
+              }
+              umma_commit(&s_full[s]);
+              if (b.split || s == 1 || b.lo[1] > 0 || b.hi[1] == 0) umma_commit(&kv_empty[slot]);
+              if (bhi == 1) umma_commit(&q_empty[s]);
+            }
+            __syncwarp();
+          }
+        }
+      };
+      ItemGeom g;
+      if (kJoin) {
+        ItemGeom none;
+        none.steps = none.split = none.lo[0] = none.lo[1] = none.hi[0] = none.hi[1] = 0;
+        if (take_nonempty(g)) join(none, g, 0);
+      }
       while (ok) {
-        ItemGeom g;
-        const int item = take_item(n_items, g);
-        if (item < 0) break;
+        if (kJoin ? g.steps == 0 : take_item(n_items, g) < 0) break;
+        const int j_first = kJoin ? 0 : -1, j_end = kJoin ? g.steps - 1 : g.steps;
         // Ring positions are carried along instead of recomputed: (slot_v, par_v) is where V_j lives,
         // (slot_k, par_k) where K_{j+1} lives. Rounds in which both stages have a P.V for tile j and a
         // score tile j+1 ("interior", nearly all of a long sequence) take a branch-free body; the first
         // and last rounds of an item take the general one.
-        uint32_t slot_k = ring_slot, par_k = ring_par;  // K of step 0
-        uint32_t slot_v = 0, par_v = 0;                 // set when j reaches 0
+        // (split items: slot_k is the next tile in the ring)
+        const uint32_t pos0 = pos + 1, pos1 = kJoin ? pos + 2 : pos;
+        uint32_t slot_v = pos0 % Cfg::kStages, par_v = (pos0 / Cfg::kStages) & 1;
+        uint32_t slot_k = pos1 % Cfg::kStages, par_k = (pos1 / Cfg::kStages) & 1;
         auto advance = [](uint32_t& slot, uint32_t& par, uint32_t n) {
           slot += n;
           if (slot >= static_cast<uint32_t>(Cfg::kStages)) { slot -= Cfg::kStages; par ^= 1u; }
@@ -764,7 +839,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               }
               const uint32_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
               if (!kInterior && !v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
-              if (!mbar_wait_warp(&p_full[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
+              if (!mbar_wait_warp(&p_full[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
               tc_fence_after();
               if (elect_one()) {
                 umma_ts_lo(tmem_base + colO, tmem_base + colS, vdesc, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
@@ -773,8 +848,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                   umma_ts_lo(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
               }
               __syncwarp();
-              if (!mbar_wait_warp(&p_full2[s], n_p[s] & 1, abort_flag)) { ok = false; return; }
-              ++n_p[s];
+              if (!mbar_wait_warp(&p_full2[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
+              par_p ^= 1u << s;
               tc_fence_after();
               if (elect_one()) {
 #pragma unroll
@@ -787,8 +862,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             }
             if (act_n) {  // S_s = Q_s K_{j+1}^T
               if (!kInterior && j + 1 == g.lo[s]) {
-                if (!mbar_wait_warp(&q_full[s], n_q[s] & 1, abort_flag)) { ok = false; return; }
-                ++n_q[s];
+                if (!mbar_wait_warp(&q_full[s], (par_q >> s) & 1, abort_flag)) { ok = false; return; }
+                par_q ^= 1u << s;
               }
               if (!k_seen && !mbar_wait_warp(&kv_full[slot_k], par_k, abort_flag)) { ok = false; return; }
               // Inner rounds wait for V here, one round ahead: every group of instructions then has one wait in front
@@ -812,25 +887,27 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
         };
         if (g.split) {
-          for (int j = -1; j < g.steps && ok; ++j) round_body(std::false_type{}, std::true_type{}, j);
-          ring_slot = slot_k;
-          ring_par = par_k;
-          continue;
+          for (int j = j_first; j < j_end && ok; ++j) round_body(std::false_type{}, std::true_type{}, j);
+          pos += 2u * static_cast<uint32_t>(g.hi[0] + g.hi[1]);
+        } else {
+          for (int j = j_first; j < j_end && ok; ++j) {
+            if (j == in_lo && in_lo < in_hi) ok = mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag);
+            if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
+            else round_body(std::false_type{}, std::false_type{}, j);
+            // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
+            slot_v = slot_k;
+            par_v = par_k;
+            advance(slot_v, par_v, 1);
+            advance(slot_k, par_k, 2);
+          }
+          pos += 2u * static_cast<uint32_t>(g.steps);
         }
-        for (int j = -1; j < g.steps && ok; ++j) {
-          if (j == in_lo && in_lo < in_hi) ok = mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag);
-          if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
-          else round_body(std::false_type{}, std::false_type{}, j);
-          // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
-          slot_v = slot_k;
-          par_v = par_k;
-          advance(slot_v, par_v, 1);
-          advance(slot_k, par_k, 2);
-        }
-        {  // the next item's first K follows this item's last V
-          uint32_t n = 2u * static_cast<uint32_t>(g.steps);
-          while (n >= static_cast<uint32_t>(Cfg::kStages)) { n -= Cfg::kStages; ring_par ^= 1u; }
-          advance(ring_slot, ring_par, n);
+        if (!ok) break;
+        if (kJoin) {
+          ItemGeom nx;
+          take_nonempty(nx);
+          join(g, nx, pos);
+          g = nx;
         }
       }
     } else if (warp == 13 && lane == 0) {
