@@ -21,6 +21,7 @@
 #include "fwd_pair_ahead.cuh"
 #include "fwd_persistent.cuh"
 #include "fwd_serial.cuh"
+#include "work_items.h"
 
 namespace {
 
@@ -217,34 +218,6 @@ int launch_pair_ahead(DeviceState* s, const void* q, const void* k, const void* 
   return FA_OK;
 }
 
-// Takes some of the pairs of q tiles apart into single q tiles whose kv tiles the two stages of a CTA share out
-// (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
-// the epilogue merges two outputs), but there are twice as many items of half the length.
-// - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
-//   one wave. B2 H16 N4096 d128: 3.46 waves of 32 steps, 277 -> 255 us; 8 heads of 333 rows: 14.3 -> 12.6 us.
-// - Under a causal mask items are handed out longest first and a partial wave costs little; but with few of them the
-//   longest one sets the time. All are split while a CTA has less than about 7/4 items, or, where sequences are
-//   short and the fill and drain of an item weigh more, less than a seventh of a head's pairs (d64 us, pairs against
-//   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
-//   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
-//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
-void set_work_items(fa::FwdParams* p, int num_sms) {
-  const int pairs = p->num_items;
-  int split = 0;
-  if (p->seqlen > fa::kBlockM && pairs < (1 << 30)) {
-    const int wl = p->window_left, wr = fa::eff_window_right(p->causal, p->window_right);
-    const bool even = (wl < 0 && wr < 0) || (wl >= 0 && wr >= 0 && wl < p->seqlen / 4 && wr < p->seqlen / 4);
-    if (even) {
-      const int tail = pairs % num_sms;
-      if (2 * tail <= num_sms) split = tail;
-    } else if (2 * pairs <= num_sms || 4LL * pairs <= 7LL * num_sms) {
-      if (2 * pairs <= num_sms || 7LL * pairs <= (long long)p->num_q_pairs * num_sms) split = pairs;
-    }
-  }
-  p->num_pair_items = pairs - split;
-  p->num_items = pairs + split;
-}
-
 // Launches with programmatic stream serialization: the kernel's prologue (barriers, tensor memory, descriptors) may
 // run while the kernel in front of it in the stream ends; see griddep_wait() in the kernel. Calls in a row, us a call
 // (for flash_forward_noalloc with the memset in front of each launch gone): 8 heads x 333 rows 14.3 -> 9.8,
@@ -277,7 +250,7 @@ int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMa
   int rc = ensure_smem_attr(s, slot, fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout>, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
   fa::FwdParams pp = p;
-  set_work_items(&pp, s->num_sms);
+  fa::set_work_items(&pp, s->num_sms);
   const int grid = pp.num_items < s->num_sms ? pp.num_items : s->num_sms;
   std::lock_guard<std::mutex> lk(s->mu);
   int sched_slot = 0;
@@ -388,7 +361,7 @@ int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUte
                               const CUtensorMap& mo,
                               fa::FwdParams p, cudaStream_t st) {
   using Cfg = fa::PersistentCfg<D>;
-  set_work_items(&p, s->num_sms);
+  fa::set_work_items(&p, s->num_sms);
   {
     std::lock_guard<std::mutex> lk(s->mu);
     bool& done = s->attr_set[D == 64 ? 0 : 1];

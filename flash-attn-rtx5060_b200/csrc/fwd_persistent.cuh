@@ -24,6 +24,7 @@
 
 #include "fwd_params.h"
 #include "ptx.cuh"
+#include "work_items.h"
 
 // Registers per thread after setmaxnreg: 8 softmax warps, 4 correction warps, 4 others; the three
 // numbers must satisfy 256 * softmax + 128 * correction + 128 * others <= 65536.
@@ -65,84 +66,6 @@ struct PersistentCfg {
   // ran in 1117 us with 2^8 and run in 1086 us with 2^14.
   static constexpr float kLazyLog2 = 14.f;
 };
-
-// Work item -> geometry. Every role decodes the same item the same way.
-// The kv tiles of an item are walked from the last visible one to the first. Under a causal mask (and for a ragged
-// end) the tiles that carry the per-element predicate then come first, where the pipeline fills anyway, instead of
-// at the item's end where nothing hides them; the two stages start one tile apart, out of phase; and with ALiBi the
-// bias falls along the walk, so the row reference is found on the first tile and stays. Measured on B200, first to
-// last against last to first (and no speculation in cut tiles): B4 H16 N2048 d64 causal 89.2 -> 82.4 us,
-// B2 H32 N8192 d128 causal 1112 -> 1079, its 16384-row sliding window 755 -> 712, B2 H16 N4096 d64 ALiBi 217 -> 182,
-// B4 H16 N2048 d64 with dropout 138 -> 125.
-struct ItemGeom {
-  int bh, pair;
-  int r0[2], r1[2];  // first / last q row of each stage's tile (r1 < r0: stage has no rows)
-  int lo[2], hi[2];  // walk steps of each stage, [lo, hi); empty when no rows. Step t works on kv tile `top - t`
-  int top, steps;    // last visible kv tile of the item, number of steps
-  // 0: the stages own the two q tiles of a pair and share every kv tile (both work on tile `top - t` in step t).
-  // 1: both stages own the SAME q tile and take its kv tiles in turn: stage s works on tile top - 2t - s; the
-  //    epilogue merges their two outputs.
-  int split;
-};
-
-// Work-item order. Heads are taken in groups of `head_group` (sized on the host so that the K/V of
-// a group stays in L2); inside a group the items run pair-major from the last (under a causal mask
-// the longest) q pair to the first. CTAs claim items in this order from a global counter, so CTAs
-// that run together read the same few heads, and the items handed out last are the cheapest ones
-// of the last group: the tail stays short.
-template <int BN = kBlockN>
-__device__ __forceinline__ ItemGeom decode_item(int item, const FwdParams& p) {
-  ItemGeom g;
-  const int sub = (item - p.num_pair_items) & 1;  // of a split pair: 0 the second q tile (the longer one), 1 the first
-  g.split = item >= p.num_pair_items;
-  if (g.split) item = p.num_pair_items + ((item - p.num_pair_items) >> 1);
-  const int per_group = p.head_group * p.num_q_pairs;
-  const int grp = item / per_group;
-  const int r = item - grp * per_group;
-  const int heads_here = min(p.head_group, p.bh - grp * p.head_group);
-  const int pr = r / heads_here;
-  g.bh = grp * p.head_group + (r - pr * heads_here);
-  g.pair = p.num_q_pairs - 1 - pr;
-  const int wr = eff_window_right(p.causal, p.window_right);
-  int lo_all = 0x7fffffff, hi_all = 0;
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    g.r0[s] = g.pair * 2 * kBlockM + s * kBlockM;
-    if (g.r0[s] >= p.seqlen) {
-      g.r1[s] = g.r0[s] - 1;
-      g.lo[s] = g.hi[s] = 0;
-    } else {
-      g.r1[s] = min(g.r0[s] + kBlockM, p.seqlen) - 1;
-      g.lo[s] = kv_tile_begin(g.r0[s], p.window_left, BN);
-      g.hi[s] = kv_tile_end(g.r1[s], wr, p.seqlen, BN);
-      lo_all = min(lo_all, g.lo[s]);
-      hi_all = max(hi_all, g.hi[s]);
-    }
-  }
-  if (g.split) {
-    const int s = 1 - sub;
-    const int n = s ? g.hi[1] - g.lo[1] : g.hi[0] - g.lo[0];  // kv tiles of the one q tile (0: it has no rows)
-    g.top = (s ? g.hi[1] : g.hi[0]) - 1;
-    g.r0[0] = g.r0[1] = s ? g.r0[1] : g.r0[0];
-    g.r1[0] = s ? g.r1[1] : g.r1[0];
-    g.r1[1] = n > 1 ? g.r1[0] : g.r0[0] - 1;
-    g.lo[0] = g.lo[1] = 0;
-    g.hi[0] = g.steps = (n + 1) >> 1;
-    g.hi[1] = n >> 1;
-    g.split = n > 1;
-    return g;
-  }
-  g.top = hi_all - 1;
-  g.steps = hi_all - lo_all;
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {  // tile range -> step range
-    if (g.r1[s] < g.r0[s]) continue;
-    const int lo = g.lo[s];
-    g.lo[s] = hi_all - g.hi[s];
-    g.hi[s] = hi_all - lo;
-  }
-  return g;
-}
 
 // exp2 of 64 scores (32 pairs) -> 32 packed fp16x2 words; adds the exponentials into two
 // (even, odd) pairs of partial row sums.
@@ -717,6 +640,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       uint32_t par_p = 0, par_q = 0;  // bit s: phase parity of stage s's barriers
       uint32_t n_items = 0;
       bool ok = true;
+      // (Every published item has rows, so the loop ends on its first pass. Written without it the compiler's code for the
+      // rounds ran 3 % slower at head_dim 64: B8 H12 N1000 48.7 -> 50.0 us, B4 H16 N2048 causal 64.7 -> 67.1.)
       auto take_nonempty = [&](ItemGeom& g) {
         while (take_item(n_items, g) >= 0)
           if (g.steps > 0) return true;
@@ -918,11 +843,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       uint32_t n_q[2] = {0, 0};
       uint32_t n_pub = 0;
       bool ok = true;
-      int next = (static_cast<int>(blockIdx.x) < p.num_items) ? static_cast<int>(blockIdx.x) : -1;
+      int next = static_cast<int>(blockIdx.x);
       while (ok) {
-        const int item = next;
         ItemGeom g;
-        if (item >= 0) g = decode_item(item, p);
+        const int item =
+            next_item(next, p, g, [&] { return static_cast<int>(gridDim.x) + atomicAdd(p.sched, 1); });
+        if (item < 0) griddep_launch();  // no further item: the next kernel of the stream may take up free SMs
         {  // publish the item to the other roles
           const uint32_t slot = n_pub & 1u;
           if (!mbar_wait(&item_empty[slot], ((n_pub >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
@@ -962,7 +888,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         };
         // The Q tiles of the previous item are released one after the other, stage 0 first; the ring slots of the
         // first kv tiles usually before either.
-        if (g.steps > 0) load_tile(&mapK, g.top);
+        load_tile(&mapK, g.top);
         load_q(0);
         load_q(1);
         if (g.split) {  // in the order of use
@@ -982,10 +908,6 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
         }
         next = static_cast<int>(gridDim.x) + claimed;
-        if (next >= p.num_items) {
-          next = -1;
-          griddep_launch();  // this CTA takes no further item: the next kernel of the stream may take up free SMs
-        }
       }
       if (!ok) {
         // give-up path: let loads that are still in flight land before the CTA retires

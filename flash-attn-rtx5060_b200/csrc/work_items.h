@@ -1,0 +1,138 @@
+// Work items of the one-CTA persistent kernel: the host's plan (which pairs of q tiles are taken apart), the geometry of
+// an item and the walk over the items that a CTA claims. Plain C++ as well as device code, so that the walk can be
+// checked without a GPU.
+#pragma once
+#include "fwd_params.h"
+
+#ifdef __CUDA_ARCH__
+#define FA_UNROLL _Pragma("unroll")
+#else
+#define FA_UNROLL
+#endif
+
+namespace fa {
+
+__host__ __device__ inline int min_int(int a, int b) { return a < b ? a : b; }
+
+// Takes some of the pairs of q tiles apart into single q tiles whose kv tiles the two stages of a CTA share out
+// (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
+// the epilogue merges two outputs), but there are twice as many items of half the length.
+// - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
+//   one wave. B2 H16 N4096 d128: 3.46 waves of 32 steps, 277 -> 255 us; 8 heads of 333 rows: 14.3 -> 12.6 us.
+// - Under a causal mask items are handed out longest first and a partial wave costs little; but with few of them the
+//   longest one sets the time. All are split while a CTA has less than about 7/4 items, or, where sequences are
+//   short and the fill and drain of an item weigh more, less than a seventh of a head's pairs (d64 us, pairs against
+//   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
+//   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
+//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
+inline void set_work_items(FwdParams* p, int num_sms) {
+  const int pairs = p->num_items;
+  int split = 0;
+  if (p->seqlen > kBlockM && pairs < (1 << 30)) {
+    const int wl = p->window_left, wr = eff_window_right(p->causal, p->window_right);
+    const bool even = (wl < 0 && wr < 0) || (wl >= 0 && wr >= 0 && wl < p->seqlen / 4 && wr < p->seqlen / 4);
+    if (even) {
+      const int tail = pairs % num_sms;
+      if (2 * tail <= num_sms) split = tail;
+    } else if (2 * pairs <= num_sms || 4LL * pairs <= 7LL * num_sms) {
+      if (2 * pairs <= num_sms || 7LL * pairs <= (long long)p->num_q_pairs * num_sms) split = pairs;
+    }
+  }
+  p->num_pair_items = pairs - split;
+  p->num_items = pairs + split;
+}
+
+// Work item -> geometry. Every role decodes the same item the same way.
+// The kv tiles of an item are walked from the last visible one to the first. Under a causal mask (and for a ragged
+// end) the tiles that carry the per-element predicate then come first, where the pipeline fills anyway, instead of
+// at the item's end where nothing hides them; the two stages start one tile apart, out of phase; and with ALiBi the
+// bias falls along the walk, so the row reference is found on the first tile and stays. Measured on B200, first to
+// last against last to first (and no speculation in cut tiles): B4 H16 N2048 d64 causal 89.2 -> 82.4 us,
+// B2 H32 N8192 d128 causal 1112 -> 1079, its 16384-row sliding window 755 -> 712, B2 H16 N4096 d64 ALiBi 217 -> 182,
+// B4 H16 N2048 d64 with dropout 138 -> 125.
+struct ItemGeom {
+  int bh, pair;
+  int r0[2], r1[2];  // first / last q row of each stage's tile (r1 < r0: stage has no rows)
+  int lo[2], hi[2];  // walk steps of each stage, [lo, hi); empty when no rows. Step t works on kv tile `top - t`
+  int top, steps;    // last visible kv tile of the item, number of steps
+  // 0: the stages own the two q tiles of a pair and share every kv tile (both work on tile `top - t` in step t).
+  // 1: both stages own the SAME q tile and take its kv tiles in turn: stage s works on tile top - 2t - s; the
+  //    epilogue merges their two outputs.
+  int split;
+};
+
+// Work-item order. Heads are taken in groups of `head_group` (sized on the host so that the K/V of
+// a group stays in L2); inside a group the items run pair-major from the last (under a causal mask
+// the longest) q pair to the first. CTAs claim items in this order from a global counter, so CTAs
+// that run together read the same few heads, and the items handed out last are the cheapest ones
+// of the last group: the tail stays short.
+template <int BN = kBlockN>
+__host__ __device__ inline ItemGeom decode_item(int item, const FwdParams& p) {
+  ItemGeom g;
+  const int sub = (item - p.num_pair_items) & 1;  // of a split pair: 0 the second q tile (the longer one), 1 the first
+  g.split = item >= p.num_pair_items;
+  if (g.split) item = p.num_pair_items + ((item - p.num_pair_items) >> 1);
+  const int per_group = p.head_group * p.num_q_pairs;
+  const int grp = item / per_group;
+  const int r = item - grp * per_group;
+  const int heads_here = min_int(p.head_group, p.bh - grp * p.head_group);
+  const int pr = r / heads_here;
+  g.bh = grp * p.head_group + (r - pr * heads_here);
+  g.pair = p.num_q_pairs - 1 - pr;
+  const int wr = eff_window_right(p.causal, p.window_right);
+  int lo_all = 0x7fffffff, hi_all = 0;
+FA_UNROLL
+  for (int s = 0; s < 2; ++s) {
+    g.r0[s] = g.pair * 2 * kBlockM + s * kBlockM;
+    if (g.r0[s] >= p.seqlen) {
+      g.r1[s] = g.r0[s] - 1;
+      g.lo[s] = g.hi[s] = 0;
+    } else {
+      g.r1[s] = min_int(g.r0[s] + kBlockM, p.seqlen) - 1;
+      g.lo[s] = kv_tile_begin(g.r0[s], p.window_left, BN);
+      g.hi[s] = kv_tile_end(g.r1[s], wr, p.seqlen, BN);
+      lo_all = min_int(lo_all, g.lo[s]);
+      hi_all = hi_all > g.hi[s] ? hi_all : g.hi[s];
+    }
+  }
+  if (g.split) {
+    const int s = 1 - sub;
+    const int n = s ? g.hi[1] - g.lo[1] : g.hi[0] - g.lo[0];  // kv tiles of the one q tile (0: it has no rows)
+    g.top = (s ? g.hi[1] : g.hi[0]) - 1;
+    g.r0[0] = g.r0[1] = s ? g.r0[1] : g.r0[0];
+    g.r1[0] = s ? g.r1[1] : g.r1[0];
+    g.r1[1] = n > 1 ? g.r1[0] : g.r0[0] - 1;
+    g.lo[0] = g.lo[1] = 0;
+    g.hi[0] = g.steps = (n + 1) >> 1;
+    g.hi[1] = n >> 1;
+    g.split = n > 1;
+    return g;
+  }
+  g.top = hi_all - 1;
+  g.steps = hi_all - lo_all;
+FA_UNROLL
+  for (int s = 0; s < 2; ++s) {  // tile range -> step range
+    if (g.r1[s] < g.r0[s]) continue;
+    const int lo = g.lo[s];
+    g.lo[s] = hi_all - g.hi[s];
+    g.hi[s] = hi_all - lo;
+  }
+  return g;
+}
+
+// The first item with rows, starting at `item` and going on with what `claim()` returns (the next unclaimed item);
+// -1 when the items have run out. A split pair whose second q tile lies past the end of the sequence counts as two items,
+// one of them without rows. Such an item is never published to the roles of the kernel: the issuing warp looks for the
+// next item before it commits the last product of the current one, the correction warps wait for that commit before they
+// free the slot of the item after next, and with two slots two row-less items in a row would close that circle.
+template <typename Claim>
+__host__ __device__ inline int next_item(int item, const FwdParams& p, ItemGeom& g, Claim claim) {
+  while (item >= 0 && item < p.num_items) {
+    g = decode_item(item, p);
+    if (g.steps > 0) return item;
+    item = claim();
+  }
+  return -1;
+}
+
+}  // namespace fa

@@ -218,6 +218,25 @@ def test_split_items(pkg, ob, H, N, d, causal, wl, wr):
     assert np.abs(lse[:, :2].cpu().numpy()[:, :, rows] - exact).max() <= 5e-4
 
 
+# Launches whose split pairs have a second q tile without rows (it lies past the end of the sequence) and whose items are
+# claimed from the counter: such a tile must not reach the roles of the kernel, and no row may be left out.
+@pytest.mark.parametrize("H,N,d,causal", [(100, 300, 64, False), (111, 300, 64, False), (123, 600, 64, False),
+                                          (111, 300, 128, False), (14, 2100, 64, True)])
+def test_split_pairs_without_a_second_tile(pkg, ob, H, N, d, causal):
+    import torch
+
+    q, k, v = make_inputs(4500 + N + H, 1, H, N, d)
+    want = ob.attention(q, k, v, causal=causal)
+    tq, tk, tv = (torch.from_numpy(a).cuda() for a in (q, k, v))
+    outs = [torch.full_like(tq, float("nan")) for _ in range(20)]
+    for o in outs:
+        pkg.attention_forward(tq, tk, tv, causal=causal, out=o)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    assert_close_or_one_ulp(outs[0].cpu().numpy(), want)
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+
+
 def test_very_long_sequence_and_very_many_heads(pkg, ob):
     """The two ends of the work-item space: one head of 131072 rows (512 q pairs, a 64 MB K/V working set, 1024 kv
     tiles for the last rows) and 6000 heads of 256 rows (one item per head, the dynamic work counter hands out

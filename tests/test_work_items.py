@@ -1,0 +1,146 @@
+"""CPU tests of the persistent kernel's work items (csrc/work_items.h, compiled here for the host): every q tile is handed
+out exactly once with exactly its visible kv tiles, and the hand-over of items through the two-slot ring ends for every
+order in which a CTA may claim them."""
+import ctypes
+import itertools
+import os
+import random
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "flash-attn-rtx5060_b200", "csrc")
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def wi(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("work_items") / "work_items.so")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-I", cuda, "-o", so,
+                           os.path.join(ROOT, "tests", "work_items_host.cpp")])
+    return ctypes.CDLL(so)
+
+
+class Launch:
+    def __init__(self, wi, bh, n, causal=False, wl=-1, wr=-1, group=1, sms=SMS):
+        self.wi, self.args = wi, (bh, n, int(causal), wl, wr, group, sms)
+        items, pairs = ctypes.c_int(), ctypes.c_int()
+        wi.plan(*self.args, ctypes.byref(items), ctypes.byref(pairs))
+        self.items, self.pair_items = items.value, pairs.value
+
+    def walk(self, item, claims):
+        out = (ctypes.c_int * 16)()
+        claims = (ctypes.c_int * (len(claims) + 1))(*claims, self.items)
+        used = self.wi.walk(*self.args, item, claims, out)
+        keys = ("item", "head", "r0a", "r1a", "loa", "hia", "r0b", "r1b", "lob", "hib", "top", "steps", "split")
+        return dict(zip(keys, out)), used
+
+    def published(self, first, claims):
+        """What one CTA publishes to its roles when it starts with `first` and its claims are answered by `claims`."""
+        out, at, item = [], 0, first
+        while True:
+            g, used = self.walk(item, claims[at:])
+            at += used
+            if g["item"] < 0:
+                return out
+            out.append(g)
+            item = claims[at] if at < len(claims) else self.items
+            at += 1
+
+
+SHAPES = [
+    dict(bh=100, n=300), dict(bh=111, n=300), dict(bh=123, n=600), dict(bh=75, n=333), dict(bh=3, n=129),
+    dict(bh=1, n=100), dict(bh=2, n=129, causal=True), dict(bh=80, n=450, causal=True, wl=60, group=80),
+    dict(bh=5, n=1000, wl=100, wr=5, group=5), dict(bh=8, n=2304 + 77, causal=True, group=8),
+    dict(bh=40, n=4097, causal=True, group=14), dict(bh=7, n=700, wl=50, group=7), dict(bh=96, n=1000),
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+def test_every_q_tile_once_with_its_kv_tiles(wi, pkg, shape):
+    L = Launch(wi, **shape)
+    n, causal = shape["n"], shape.get("causal", False)
+    wl, wr = shape.get("wl", -1), shape.get("wr", -1)
+    seen = {}
+    for item in range(L.items):
+        g, _ = L.walk(item, [])
+        if g["item"] != item:  # an item without rows: skipped, and the stand-in claim ended the walk
+            assert g["item"] == -1 and item >= L.pair_items
+            continue
+        tiles = {}
+        for s, (r0, r1, lo, hi) in enumerate([(g["r0a"], g["r1a"], g["loa"], g["hia"]),
+                                              (g["r0b"], g["r1b"], g["lob"], g["hib"])]):
+            assert r1 >= r0 or lo == hi
+            for t in range(lo, hi):
+                tiles.setdefault(r0, []).append(g["top"] - 2 * t - s if g["split"] else g["top"] - t)
+                assert 0 <= t < g["steps"] and r1 >= r0
+        assert tiles
+        for r0, js in tiles.items():
+            assert (g["head"], r0) not in seen
+            seen[g["head"], r0] = js
+    assert set(seen) == set(itertools.product(range(shape["bh"]), range(0, n, 128)))
+    for (_, r0), js in seen.items():
+        lo, hi, _ = pkg.kv_range(n, causal, wl, wr, r0, min(r0 + 128, n) - 1)
+        assert sorted(js) == list(range(lo, hi))
+
+
+def ring_ends(rows):
+    """The hand-over of items between the roles of a CTA, as the kernel does it at head_dim 64. `rows[i]`: published item i
+    has rows. Two slots; the producer fills one again when every reader has taken it. The issuing warp takes the next item
+    with rows (or the end) before it commits the last product of the current one; the correction warps take an item and
+    wait for that commit before they take another. Returns whether everybody reaches the end."""
+    end = len(rows)  # the end marker is published like an item
+    published = issuer = corr = 0  # items published / taken
+    current, committed = None, set()
+    issuer_done = corr_done = False
+    waiting = None
+    while True:
+        before = (published, issuer, corr, len(committed), issuer_done, corr_done, current, waiting)
+        if published <= end and min(issuer, corr) >= published - 1:  # the slot of item published - 2 has been read
+            published += 1
+        if not issuer_done and issuer < published:
+            i = issuer
+            issuer += 1
+            if i == end or rows[i]:
+                if current is not None:
+                    committed.add(current)
+                current = i
+                issuer_done = i == end
+        if waiting is not None and waiting in committed:
+            waiting = None
+        if waiting is None and not corr_done and corr < published:
+            if corr == end:
+                corr_done = True
+            elif rows[corr]:
+                waiting = corr
+            corr += 1
+        if (published, issuer, corr, len(committed), issuer_done, corr_done, current, waiting) == before:
+            return issuer_done and corr_done
+
+
+def test_ring_model_sees_the_cycle_of_row_less_items():
+    assert ring_ends([True] * 5) and ring_ends([]) and ring_ends([True, False, True]) and ring_ends([False, False])
+    assert not ring_ends([True, False, False]) and not ring_ends([True, False, False, True])
+
+
+@pytest.mark.parametrize("shape", [s for s in SHAPES if (s["n"] - 1) % 256 < 128], ids=str)
+def test_item_hand_over_ends_for_every_claim_order(wi, shape):
+    """One CTA starts with any item and then gets any rising sequence of the others (the rest goes to CTAs that run beside
+    it): whatever it publishes must let all its roles reach the end."""
+    L = Launch(wi, **shape)
+    rng = random.Random(5)
+    row_less = [i for i in range(L.pair_items, L.items) if L.walk(i, [])[0]["item"] < 0]
+    orders = [[]]
+    if row_less:
+        orders += [row_less, row_less[:2], [0] + row_less[:3] + [L.items - 1]]
+    for _ in range(40):
+        orders.append(sorted(rng.sample(range(L.items), min(L.items, rng.randint(1, 8)))))
+    for order in orders:
+        for first in {0, order[0] if order else 0}:
+            pub = L.published(first, [i for i in order if i != first])
+            assert ring_ends([g["steps"] > 0 for g in pub])
+            assert all(g["steps"] > 0 for g in pub)
+            assert [g["item"] for g in pub] == [i for i in [first] + [i for i in order if i != first] if i not in row_less]
