@@ -59,12 +59,20 @@ struct PersistentCfg {
   static constexpr int kSmemBytes = kOffGeom + 2 * 64;  // two work-item slots: the item's decoded geometry and its id
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 384;
-  // Softmax threshold (in log2 units) below which a larger row max does not trigger a rescale. P then stays below
-  // 2^14, inside fp16 (65504), and l and O, held in fp32, have the room; fp16 is relatively as precise there as near
-  // 1. A walk that starts on the diagonal takes its first reference from the few keys the upper rows see there, so
-  // with 2^8 many of them moved it on the second tile: scores of twice the usual spread (B2 H32 N8192 d128 causal)
-  // ran in 1117 us with 2^8 and run in 1086 us with 2^14.
-  static constexpr float kLazyLog2 = 14.f;
+  // Lazy rescale, in log2 units: a row's reference (the score that its exponentials are taken against) stays where it is
+  // until a tile's row max passes it by more than kLazyLog2, so P stays below 2^8, well inside fp16, and l and O, held
+  // in fp32, have the room. The key that sets the reference has P = 1 exactly; a key above it has a P rounded to 11 bits,
+  // which O keeps while l takes the unrounded exponential, so a row that one such key dominates loses the exactness of
+  // its main term. Two rules keep that rare. Once a warp acts for one of its rows, all its rows whose max has grown move
+  // along: the cost, 32 exponentials taken again and a rescale of O, is the warp's anyway. And on the first keys of the
+  // sequence, which the walk visits last and which many rows of a trained causal model look at, any growth moves it.
+  // Error against 64 bits (2-norm, 1e-4; 4 heads x 4096 rows d64; one early key 8 and 12 log2 units above the others;
+  // scores of spread 4; of spread 2): 2.14 2.08 2.60 2.84. With 2^14 and neither rule: 2.94 2.93 2.88 2.88; with 2^8
+  // and a walk from the first tile to the last: 2.14 2.08 2.63 2.88.
+  // What it costs against 2^14 alone (us): B4 H16 N2048 d64 causal 64.7 -> 66.4, B8 H16 N1024 d128 causal 56.8 -> 58.7,
+  // 24 heads x 4001 rows d128 causal, log-sum-exp, spread 2 115.9 -> 116.7, B2 H32 N8192 d128 causal 1041 -> 1045 (the
+  // running max as such is no longer kept; with ALiBi the register it took matters more: B2 H16 N4096 d64 131.8 -> 128.7).
+  static constexpr float kLazyLog2 = 8.f;
 };
 
 // exp2 of 64 scores (32 pairs) -> 32 packed fp16x2 words; adds the exponentials into two
@@ -273,9 +281,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       const int row = q_r0 + row_l;
       float slope_l2 = 0.f;
       if (kAlibi) slope_l2 = p.alibi_slopes[g.bh % p.heads] * 1.4426950408889634f;
-      float m_run = -INFINITY;  // true running max of the raw scores
-      float m_used = 0.f;       // max the exponentials are currently taken against
-      float l_run = 0.f;
+      float m_used = 0.f;  // the row's reference: the score that its exponentials are taken against
+      float l_run = 0.f;   // 0 until the row has seen a finite score, at least about 1 from then on
       for (int j = j_lo; j < j_hi; ++j) {
         if (!mbar_wait_warp(&s_full[s], n_s & 1, abort_flag)) { ok = false; break; }
         ++n_s;
@@ -357,7 +364,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const float neg_ms0 = -m_used * sl2;
             exp_quarter_tile(sc, scale2, f2_pack(neg_ms0, neg_ms0), pk0, lsum_a, lsum_b);
           }
-          float mx0 = m_run, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+          float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
   #pragma unroll
           for (int c = 0; c < kBlockN; c += 8) {
             mx0 = max3(mx0, sc[c], sc[c + 1]);
@@ -366,18 +373,20 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             mx3 = max3(mx3, sc[c + 6], sc[c + 7]);
           }
           float m_new = max3(mx0, mx1, fmaxf(mx2, mx3));
-          if (kMasked && m_new < -1.0e37f) m_new = -INFINITY;  // nothing visible so far (hidden scores sit near -3e38)
-          // The reference moves when the true max has grown past it by more than kLazyLog2, and always on the first tile that shows a finite score: the reference then IS
-          // the row max, so the largest term of the row is exactly 1 in fp16 (a row with a single visible key
-          // returns that key's V bit for bit).
-          const bool fresh = (m_run == -INFINITY);
-          const bool move = fresh || (m_new - m_used) * sl2 > Cfg::kLazyLog2;
+          if (kMasked && m_new < -1.0e37f) m_new = -INFINITY;  // nothing visible (hidden scores sit near -3e38)
+          // The reference moves when the tile's max has grown past it (see kLazyLog2), and always on the first tile that
+          // shows a finite score: the reference then IS the row max, so the largest term of the row is exactly 1 in
+          // fp16 (a row with a single visible key returns that key's V bit for bit). A cut tile over the first keys is
+          // the only tile of its walk (or, with ALiBi, may be the last).
+          const bool fresh = l_run == 0.f;
+          const bool first_keys = (!kMasked || kAlibi) && kv0 == 0;
           float alpha = 1.f;
-          m_run = m_new;
-          if (__any_sync(0xffffffffu, move)) {
-            const float m_next = move ? ((m_new == -INFINITY) ? 0.f : m_new) : m_used;
-            alpha = fresh ? 1.f : ex2_approx((m_used - m_next) * sl2);
-            m_used = m_next;
+          if (__any_sync(0xffffffffu, fresh || (m_new - m_used) * sl2 > (first_keys ? 0.f : Cfg::kLazyLog2))) {
+            if (fresh || m_new > m_used) {
+              const float m_next = (m_new == -INFINITY) ? 0.f : m_new;
+              alpha = fresh ? 1.f : ex2_approx((m_used - m_next) * sl2);
+              m_used = m_next;
+            }
             if (!kMasked) {
               lsum_a = 0ull;
               lsum_b = 0ull;

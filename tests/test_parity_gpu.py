@@ -448,6 +448,49 @@ def test_growing_row_max_forces_rescale(pkg, ob):
         assert_close_or_one_ulp(got, want)
 
 
+def exact_attention_gpu(q, k, v, causal):
+    """fp64 attention of fp16 torch tensors [B, H, N, d], on their device."""
+    import torch
+
+    n = q.shape[2]
+    hidden = torch.ones((n, n), dtype=torch.bool, device=q.device).triu(1) if causal else None
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    for b in range(q.shape[0]):
+        for h in range(q.shape[1]):
+            s = q[b, h].double() @ k[b, h].double().T / q.shape[3] ** 0.5
+            if causal:
+                s.masked_fill_(hidden, float("-inf"))
+            out[b, h] = torch.softmax(s, -1) @ v[b, h].double()
+    return out
+
+
+# A key near the start of the sequence that stands out by `up` powers of two for every row, as the first keys do in trained
+# causal models: below and above the threshold at which a row's reference moves. (2, 1100): items whose stages share one
+# q tile; (40, 1100): pairs.
+@pytest.mark.parametrize("H,N", [(2, 1100), (40, 1100)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("up", [7.0, 9.0, 11.0, 13.5, 16.0])
+def test_row_dominated_by_an_early_key(pkg, H, N, d, causal, up):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(int(2 * up) + d)
+    q, k, v = (torch.randn((1, H, N, d), generator=g, device="cuda") for _ in range(3))
+    q[..., 0] = 4.0
+    k[..., 0] = 0.0
+    k[..., 5, 0] = up * np.log(2.0) * d ** 0.5 / 4.0
+    q, k, v = q.half(), k.half(), v.half()
+    out = pkg.attention_forward(q, k, v, causal=causal)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    exact = exact_attention_gpu(q, k, v, causal)
+    rel = ((out.double() - exact).norm() / exact.norm()).item()
+    # Rounding the result to fp16 alone is 2^-11 / sqrt(3) times the mean spread of a mantissa, 2.05e-4. The row's main
+    # term must add nothing (its probability is held exactly); the other terms' rounded probabilities add about 2.0e-4
+    # times their share of the result's norm, at most a half here. Held against a reference far below, the main term
+    # alone would add another 2.0e-4 (2.9e-4 in all).
+    assert rel <= 2.3e-4, rel
+
+
 def test_deterministic_and_kernels_agree(pkg, ob):
     q, k, v = make_inputs(13, 2, 4, 768, 128)
     a = run_gpu(pkg, q, k, v, True)
