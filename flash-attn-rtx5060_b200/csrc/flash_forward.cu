@@ -312,12 +312,17 @@ int host_pipe(HostPipe** out) {
 
 // ---- allocation-free entry point ---------------------------------------------------------
 // Scratch of flash_forward_noalloc: a fixed block in the library's own device image instead of
-// memory obtained from cudaMalloc. kNoAllocSlots slots of four ints each:
+// memory obtained from cudaMalloc. kNoAllocSlots slots of eight ints each:
 //   word 0 status (set non-zero when a bounded wait inside the kernel gave up),
-//   words 2-3 the persistent kernel's work counter and finished-CTA counter.
-// 256 bytes per GPU that loads the library, held until the process exits.
-constexpr int kNoAllocSlots = 16;
-static __device__ __align__(256) int g_noalloc_scratch[kNoAllocSlots * 4];
+//   words 2-7 three pairs for the persistent kernel: work counter and finished-CTA counter.
+// 512 bytes per GPU that loads the library, held until the process exits.
+// A launch finds its pair at zero and leaves it at zero. A caller that lets two launches on one slot overlap, which is
+// not allowed, may leave a pair off, and a launch that started from such a pair would skip work without knowing. So the
+// launches of a slot take its pairs in turn and each, as it ends, also clears the pair of the next: whatever two
+// overlapping launches did to theirs, the third starts from zero. (A memset in front of every launch cost 2 us a call and kept the
+// kernel from overlapping its predecessor.)
+constexpr int kNoAllocSlots = 16, kSlotWords = 8, kSlotPairs = 3;
+static __device__ __align__(256) int g_noalloc_scratch[kNoAllocSlots * kSlotWords];
 
 // Host-side record of the set-up done once per device for the allocation-free path. In host code
 // `g_noalloc_scratch` is only a handle for the runtime; the device address the kernel needs comes
@@ -327,6 +332,7 @@ struct NoAllocState {
   bool ready = false;
   int num_sms = 0;
   int* scratch = nullptr;  // device address of g_noalloc_scratch on this device
+  unsigned launches[kNoAllocSlots] = {};  // per slot: the next launch takes pair launches % kSlotPairs
   bool attr_set[2] = {};
 };
 NoAllocState g_noalloc[kMaxDevices];
@@ -745,7 +751,7 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
     return fail(FA_INVALID_ARG, "tensor pointers must be 16-byte aligned");
   if (slot < 0 || slot >= kNoAllocSlots) {
     snprintf(g_err, sizeof(g_err),
-             "scratch slot %d is outside the %d slots (256 bytes) that the library's static device scratch holds",
+             "scratch slot %d is outside the %d slots (512 bytes) that the library's static device scratch holds",
              slot, kNoAllocSlots);
     return FA_INVALID_ARG;
   }
@@ -768,7 +774,7 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   if (rc != FA_OK) return rc;
   if (softmax_scale <= 0.f) softmax_scale = 1.0f / sqrtf((float)head_dim);
   const int bh = (int)bh_ll;
-  int* words = s->scratch + slot * 4;
+  int* words = s->scratch + slot * kSlotWords;
 
   fa::FwdParams p;
   memset(&p, 0, sizeof(p));
@@ -780,7 +786,6 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   p.window_left = norm_window(window_left, seqlen);
   p.window_right = norm_window(window_right, seqlen);
   p.status = words;
-  p.sched = words + 2;
   p.num_q_pairs = pairs;
   p.num_items = bh * pairs;
   p.head_group = pick_head_group(bh, seqlen, head_dim, p.causal, p.window_left, p.window_right, pairs, s->num_sms);
@@ -792,11 +797,16 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   if ((rc = make_map(&mo, o, bh, seqlen, head_dim, 32)) != FA_OK) return rc;  // one correction warp's rows per store
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // The counters are zero: the static scratch starts at zero and every launch puts its slot back, one that gave up
-  // included. The launch writes its own verdict into the status word. (A memset of the slot in front of the
-  // launch cost 2 us a call and kept the kernel from overlapping its predecessor.)
   cudaError_t e;
-  p.status_per_launch = 1;
+  unsigned turn;
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    turn = s->launches[slot];
+    s->launches[slot] = (turn + 1) % kSlotPairs;
+  }
+  p.sched = words + 2 + 2 * turn;
+  p.clear_at = 2 * (int)((turn + 1) % kSlotPairs) - 2 * (int)turn;
+  p.status_per_launch = 1;  // the launch writes its own verdict into the status word
   rc = head_dim == 64 ? launch_persistent_noalloc<64>(s, mq, mk, mv, mo, p, st)
                       : launch_persistent_noalloc<128>(s, mq, mk, mv, mo, p, st);
   if (rc != FA_OK || !wait) return rc;
@@ -820,7 +830,7 @@ int flash_forward_noalloc_check(void* stream, int slot) {
   cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail_cuda("cudaStreamSynchronize", e);
   int host = 0;
-  if ((e = cudaMemcpy(&host, s->scratch + slot * 4, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+  if ((e = cudaMemcpy(&host, s->scratch + slot * kSlotWords, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
     return fail_cuda("cudaMemcpy(status)", e);
   if (host != 0) {
     snprintf(g_err, sizeof(g_err), "a wait inside the attention kernel ran out of time (status word %d)", host);
@@ -828,6 +838,22 @@ int flash_forward_noalloc_check(void* stream, int slot) {
   }
   return FA_OK;
 }
+
+#ifdef FA_TEST_WITHHOLD_LOAD
+// Test build only: leaves the pairs of the slot's last two launches as two overlapping launches may leave them.
+int flash_forward_test_disturb_slot(int slot) {
+  NoAllocState* s = nullptr;
+  int rc = noalloc_state(&s);
+  if (rc != FA_OK) return rc;
+  const int off[2] = {1 << 20, 1};
+  for (unsigned back = 1; back <= 2; ++back) {
+    const unsigned pair = (s->launches[slot] + kSlotPairs - back) % kSlotPairs;
+    cudaError_t e = cudaMemcpy(s->scratch + slot * kSlotWords + 2 + 2 * pair, off, sizeof(off), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail_cuda("cudaMemcpy(scratch slot)", e);
+  }
+  return FA_OK;
+}
+#endif
 
 int flash_forward_shutdown(void) {
   int prev = 0;

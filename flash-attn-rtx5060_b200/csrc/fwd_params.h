@@ -23,6 +23,8 @@ struct FwdParams {
   int window_right;  // j <= i + window_right  (< 0: unbounded); forced to 0 by `causal`
   int* status;       // device word, 0 = ok; set non-zero when a bounded wait gave up
   int status_per_launch;  // 1: the word is this launch's alone (the launch also writes the 0)
+  int clear_at;           // then also: the launch clears the pair of a later launch, at sched + clear_at (here, in what was
+                          // padding: a block of parameters eight bytes longer cost 2-4 % at head_dim 64)
   float* dbg;        // optional bring-up dump (serial kernel only), else nullptr
   int variant;       // bit0 (serial kernel): P through shared memory instead of TMEM; bit1 (test build of the
                      // persistent kernel only): CTA 0 withholds one tile so that a bounded wait runs out

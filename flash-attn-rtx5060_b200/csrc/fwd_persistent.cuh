@@ -930,6 +930,10 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   if (tid == 0) {
     const int gave_up = *abort_flag != 0 ? 1 : 0;
     if (gave_up) atomicExch(p.status, 1);
+    if (p.status_per_launch && blockIdx.x == 0) {
+      p.sched[p.clear_at] = 0;
+      p.sched[p.clear_at + 1] = 0;
+    }
     // the last CTA to finish puts the scheduler words back to zero for the next launch
     const int ended = atomicAdd(p.sched + 1, 1 + (gave_up << 16)) + 1 + (gave_up << 16);
     if ((ended & 0xffff) == static_cast<int>(gridDim.x)) {

@@ -199,11 +199,11 @@ int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int windo
  * cudaMalloc can fail or fragment the pool; a latency-critical loop, because cudaMalloc
  * synchronises the whole device; a plug-in that runs under an allocator hook which forbids
  * raw allocations. For them this entry point runs the same persistent kernel with its scratch
- * in a fixed 256-byte array that is part of the library's device image (every GPU that loads
- * the library holds those 256 bytes until the process exits). It calls no cudaMalloc, cudaFree
+ * in a fixed 512-byte array that is part of the library's device image (every GPU that loads
+ * the library holds those 512 bytes until the process exits). It calls no cudaMalloc, cudaFree
  * or other allocating routine.
  *
- *   slot  which of the 16 four-word scratch slots this call uses, 0..15. Anything else is
+ *   slot  which of the 16 eight-word scratch slots this call uses, 0..15. Anything else is
  *         rejected with FA_INVALID_ARG; so is a problem whose work-item count
  *         batch*heads*ceil(seqlen/256) does not fit the slot's 32-bit work counter.
  *   wait  0: return once the work is enqueued on `stream` (flash_forward_noalloc_check() reads the
@@ -211,9 +211,9 @@ int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int windo
  *         non-zero: block until the kernel has finished and return FA_DEVICE_TIMEOUT if its status
  *         word was set.
  *
- * All other arguments as for flash_forward(). Every launch leaves its slot's work counter at zero and its own
- * verdict in the status word. Calls that use the same slot must not overlap on
- * the GPU (they would share one work counter and race); calls on different slots may.
+ * All other arguments as for flash_forward(). Every launch leaves its own verdict in the slot's status word. Calls
+ * that use the same slot must not overlap on the GPU (their results are undefined then; the calls that
+ * follow them bring the counters back in order); calls on different slots may.
  * The first call on a device performs a one-time set-up (looks up the scratch array's device
  * address, sets the kernel's shared-memory attribute); make that first call before any stream
  * capture begins. */
@@ -223,7 +223,7 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
 
 /* Status of the last flash_forward_noalloc() call on scratch slot `slot` of the current device: waits
  * for `stream`, reads the slot's status word (a 4-byte device-to-host copy; nothing is allocated) and
- * returns FA_OK or FA_DEVICE_TIMEOUT. The word is cleared by the next call on that slot. No counterpart
+ * returns FA_OK or FA_DEVICE_TIMEOUT. The word is written by every call on that slot. No counterpart
  * in the reference. */
 int flash_forward_noalloc_check(void* stream, int slot);
 

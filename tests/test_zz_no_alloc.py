@@ -106,6 +106,39 @@ def test_noalloc_in_a_cuda_graph_and_the_allocating_entry_point_refuses_capture(
     assert nans == 0 and mx <= 2e-3 and mean <= 2e-4
 
 
+def test_noalloc_slot_recovers_from_overlapping_calls(pkg):
+    # Two calls that overlap on a slot (not allowed) may leave its counters off. The test build writes counters that look
+    # so (the claims start beyond the last item, one CTA counts as finished); the next calls must do all their work.
+    import os
+
+    import torch
+
+    from conftest import ROOT
+
+    L = ctypes.CDLL(os.path.join(ROOT, "tests", "_build", "libflashfwd_waittest.so"))
+    vp, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    L.flash_forward_noalloc.argtypes = [vp, vp, vp, vp, i, i, i, i, f, i, i, i, vp, i, i]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    H, N, d = 40, 1024, 64  # 160 items: more than one per CTA
+    q, k, v = (torch.randn((1, H, N, d), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    want = pkg.attention_forward(q, k, v)
+
+    def call(out, stream, wait):
+        assert L.flash_forward_noalloc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1, H, N, d, 0.0, 0, -1,
+                                       -1, stream, 6, wait) == pkg.FA_OK
+
+    out = torch.empty_like(q)
+    torch.cuda.synchronize()
+    call(out, None, 1)
+    for _ in range(5):
+        assert L.flash_forward_test_disturb_slot(6) == pkg.FA_OK
+        for _ in range(4):
+            out.fill_(float("nan"))
+            torch.cuda.synchronize()
+            call(out, None, 1)
+            assert torch.equal(out, want)
+
+
 def test_noalloc_rejects_what_the_scratch_cannot_hold(pkg):
     import torch
 
