@@ -221,14 +221,16 @@ int launch_pair_ahead(DeviceState* s, const void* q, const void* k, const void* 
 // Launches with programmatic stream serialization: the kernel's prologue (barriers, tensor memory, descriptors) may
 // run while the kernel in front of it in the stream ends; see griddep_wait() in the kernel. Calls in a row, us a call
 // (for flash_forward_noalloc with the memset in front of each launch gone): 8 heads x 333 rows 14.3 -> 9.8,
-// 1 head x 128 rows in a graph 10.2 -> 5.3, 96 heads x 1000 rows 57.2 -> 54.8, dropout B4 H16 N2048 110 -> 107.
+// 96 heads x 1000 rows 57.2 -> 54.8, dropout B4 H16 N2048 110 -> 107. Not in a captured graph (early = false): two calls
+// in a row would leave a programmatic edge there, and cudaGraphGetEdges and the like, which report plain edges only,
+// would answer cudaErrorLossyQuery for the caller's whole graph.
 template <typename K>
 cudaError_t launch_overlapped(K kernel, int grid, int threads, int smem, cudaStream_t st, const CUtensorMap& mq,
                               const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                              const fa::FwdParams& p) {
+                              const fa::FwdParams& p, bool early = true) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  attr.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(grid);
@@ -319,8 +321,9 @@ int host_pipe(HostPipe** out) {
 // A launch finds its pair at zero and leaves it at zero. A caller that lets two launches on one slot overlap, which is
 // not allowed, may leave a pair off, and a launch that started from such a pair would skip work without knowing. So the
 // launches of a slot take its pairs in turn and each, as it ends, also clears the pair of the next: whatever two
-// overlapping launches did to theirs, the third starts from zero. (A memset in front of every launch cost 2 us a call and kept the
-// kernel from overlapping its predecessor.)
+// overlapping launches did to theirs, the third starts from zero. A launch captured into a graph keeps its pair for every replay, so there a
+// memset node goes in front of it. (A memset in front of every launch cost 2 us a call and kept the kernel from
+// overlapping its predecessor.)
 constexpr int kNoAllocSlots = 16, kSlotWords = 8, kSlotPairs = 3;
 static __device__ __align__(256) int g_noalloc_scratch[kNoAllocSlots * kSlotWords];
 
@@ -365,7 +368,7 @@ int noalloc_state(NoAllocState** out) {
 template <int D>
 int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                               const CUtensorMap& mo,
-                              fa::FwdParams p, cudaStream_t st) {
+                              fa::FwdParams p, cudaStream_t st, bool early) {
   using Cfg = fa::PersistentCfg<D>;
   fa::set_work_items(&p, s->num_sms);
   {
@@ -380,7 +383,7 @@ int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUte
   }
   const int grid = p.num_items < s->num_sms ? p.num_items : s->num_sms;
   cudaError_t e = launch_overlapped(fa::fwd_persistent_kernel<D, false>, grid, Cfg::kThreads, Cfg::kSmemBytes, st, mq, mk,
-                                    mv, mo, p);
+                                    mv, mo, p, early);
   if (e != cudaSuccess) return fail_cuda("launch fwd_persistent_kernel", e);
   return FA_OK;
 }
@@ -797,18 +800,23 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   if ((rc = make_map(&mo, o, bh, seqlen, head_dim, 32)) != FA_OK) return rc;  // one correction warp's rows per store
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(st, &cap);
+  if (e != cudaSuccess) return fail_cuda("cudaStreamIsCapturing", e);
+  const bool captured = cap != cudaStreamCaptureStatusNone;
   unsigned turn;
   {
     std::lock_guard<std::mutex> lk(s->mu);
     turn = s->launches[slot];
-    s->launches[slot] = (turn + 1) % kSlotPairs;
+    if (!captured) s->launches[slot] = (turn + 1) % kSlotPairs;
   }
   p.sched = words + 2 + 2 * turn;
   p.clear_at = 2 * (int)((turn + 1) % kSlotPairs) - 2 * (int)turn;
   p.status_per_launch = 1;  // the launch writes its own verdict into the status word
-  rc = head_dim == 64 ? launch_persistent_noalloc<64>(s, mq, mk, mv, mo, p, st)
-                      : launch_persistent_noalloc<128>(s, mq, mk, mv, mo, p, st);
+  if (captured && (e = cudaMemsetAsync(p.sched, 0, 2 * sizeof(int), st)) != cudaSuccess)
+    return fail_cuda("cudaMemsetAsync(scratch slot)", e);
+  rc = head_dim == 64 ? launch_persistent_noalloc<64>(s, mq, mk, mv, mo, p, st, !captured)
+                      : launch_persistent_noalloc<128>(s, mq, mk, mv, mo, p, st, !captured);
   if (rc != FA_OK || !wait) return rc;
 
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda("cudaStreamSynchronize", e);

@@ -108,7 +108,8 @@ def test_noalloc_in_a_cuda_graph_and_the_allocating_entry_point_refuses_capture(
 
 def test_noalloc_slot_recovers_from_overlapping_calls(pkg):
     # Two calls that overlap on a slot (not allowed) may leave its counters off. The test build writes counters that look
-    # so (the claims start beyond the last item, one CTA counts as finished); the next calls must do all their work.
+    # so (the claims start beyond the last item, one CTA counts as finished); the next calls must do all their work, and
+    # so must a call captured before, replayed after.
     import os
 
     import torch
@@ -130,6 +131,9 @@ def test_noalloc_slot_recovers_from_overlapping_calls(pkg):
     out = torch.empty_like(q)
     torch.cuda.synchronize()
     call(out, None, 1)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        call(out, torch.cuda.current_stream().cuda_stream, 0)
     for _ in range(5):
         assert L.flash_forward_test_disturb_slot(6) == pkg.FA_OK
         for _ in range(4):
@@ -137,6 +141,49 @@ def test_noalloc_slot_recovers_from_overlapping_calls(pkg):
             torch.cuda.synchronize()
             call(out, None, 1)
             assert torch.equal(out, want)
+        assert L.flash_forward_test_disturb_slot(6) == pkg.FA_OK
+        for _ in range(2):
+            out.fill_(float("nan"))
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want)
+        call(out, None, 1)
+
+
+def test_captured_calls_leave_plain_edges(pkg):
+    # Calls in a row in one graph: the edges of the caller's graph can be listed without edge data (cuGraphGetEdges
+    # refuses that for programmatic edges), and the chain gives the bits of the same chain of eager calls.
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    B, H, N, d = 1, 6, 700, 64
+    q, k, v = (torch.randn((B, H, N, d), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    a, b, c = (torch.empty_like(q) for _ in range(3))
+    torch.cuda.synchronize()
+
+    def chain():
+        for x, y in ((q, a), (a, b), (b, c)):
+            assert call_noalloc(pkg, x, k, v, y, B, H, N, d, True, -1, -1, slot=8, wait=0) == pkg.FA_OK
+
+    chain()
+    torch.cuda.synchronize()
+    want = c.clone()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        chain()
+    cu = ctypes.CDLL("libcuda.so.1")
+    n = ctypes.c_size_t(64)
+    ends = [(ctypes.c_void_p * 64)() for _ in range(2)]
+    assert cu.cuGraphGetEdges(ctypes.c_void_p(graph.raw_cuda_graph()), ends[0], ends[1], ctypes.byref(n)) == 0
+    assert n.value >= 2
+    graph.instantiate()
+    for _ in range(3):
+        for t in (a, b, c):
+            t.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(c, want)
 
 
 def test_noalloc_rejects_what_the_scratch_cannot_hold(pkg):
