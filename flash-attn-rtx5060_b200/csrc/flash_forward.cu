@@ -59,11 +59,13 @@ constexpr int kMaxDevices = 64;
 // Launches in flight at the same time must not share a pair of scheduler words (the kernel leaves its pair at zero).
 // The first kOwnedSlots streams that are used on a device each own a pair: launches on one stream run one after the
 // other, so nothing more is needed. Streams are told apart by their id, which is never used again after a stream is
-// destroyed. Launches on any further stream take the remaining pairs in turn, and one that reuses a pair last used on
-// ANOTHER stream first makes its stream wait for that earlier launch (an event per pair). (With an event behind
-// every launch a call cost 1 us more on the host, and the kernel behind it could not start early.)
-constexpr int kSchedSlots = 64;
-constexpr int kOwnedSlots = 40;
+// destroyed (nothing tells this library that one was, so its pair stays taken until flash_forward_shutdown()). Launches
+// on any further stream take the 64 remaining pairs in turn, and one that reuses a pair last used on ANOTHER stream
+// first makes its stream wait for that earlier launch (an event per pair). (With an event behind every launch a call
+// cost 1 us more on the host, and the kernel behind it could not start early. 256 owners: eight times one of
+// PyTorch's stream pools; finding the last of them takes 0.1 us.)
+constexpr int kOwnedSlots = 256;
+constexpr int kSchedSlots = kOwnedSlots + 64;
 constexpr size_t kDeviceWords = 4 + 2 * kSchedSlots;
 struct DeviceState {
   std::mutex mu;

@@ -48,9 +48,10 @@ enum {
  * Two calls with the same arguments give the same bits. The split of the work among the SMs depends on
  * batch*heads, so a head may differ in the last place between a call on all heads and a call on some of them.
  *
- * Launches in flight: every launch uses a pair of scheduler words (device scratch of a few hundred bytes,
- * allocated on the first call per device). The first 40 streams that are used on a device own a pair each
- * (launches on one stream are ordered anyway); launches on further streams take 24 more in turn, and when a
+ * Launches in flight: every launch uses a pair of scheduler words (2.5 KB of device scratch,
+ * allocated on the first call per device). The first 256 streams that are used on a device own a pair each,
+ * until flash_forward_shutdown() (launches on one stream are ordered anyway); launches on further streams take 64
+ * more in turn, and when a
  * pair is reused by a launch on ANOTHER stream, that stream is first made to wait (cudaStreamWaitEvent)
  * for the earlier launch. So any number of launches may be queued on any
  * number of streams. A call whose stream is being captured into a CUDA graph is refused with

@@ -359,8 +359,8 @@ def test_many_launches_on_two_streams(pkg):
 
 def test_chained_launches_and_more_streams_than_owned_scheduler_words(pkg):
     """A launch may start before the one in front of it in the stream has ended: a chain in which every call reads the
-    previous call's output must give the bits of the same chain with a wait after each call. And 60 streams, more than
-    own scheduler words of their own, with three launches in flight on each."""
+    previous call's output must give the bits of the same chain with a wait after each call. And 60 streams with three
+    launches in flight on each (test_streams_beyond_those_that_own_scheduler_words has more streams than that)."""
     import torch
 
     g = torch.Generator(device="cuda").manual_seed(8)
@@ -389,6 +389,107 @@ def test_chained_launches_and_more_streams_than_owned_scheduler_words(pkg):
     for o in outs:
         for x in o:
             assert torch.equal(x, want)
+
+
+def test_streams_beyond_those_that_own_scheduler_words(pkg):
+    """After a process has used (and destroyed) more streams than can own a pair of scheduler words, further streams share
+    64 pairs. 30 launches queued on a stream that is held back must not make another such stream wait; 140 launches in
+    turn on three of them, which reuse pairs across streams, must still give the right bits."""
+    import time
+
+    import torch
+
+    rt = torch.cuda.cudart()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    B, H, N, d = 1, 24, 512, 64
+    q, k, v = (torch.randn((B, H, N, d), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    want = pkg.attention_forward(q, k, v, causal=True)
+    outs = [torch.full_like(q, float("nan")) for _ in range(300)]
+    torch.cuda.synchronize()
+
+    def create():
+        handle = np.zeros(1, np.uint64)
+        assert int(rt.cudaStreamCreate(handle.ctypes.data)) == 0
+        return int(handle[0])
+
+    def launch(stream, out):
+        pkg.flash_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, is_causal=True,
+                          stream=stream)
+
+    for o in outs:
+        st = create()
+        launch(st, o)
+        assert int(rt.cudaStreamDestroy(st)) == 0  # takes effect when the launch has ended
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
+
+    for o in outs:
+        o.fill_(float("nan"))
+    held, others = create(), [create() for _ in range(8)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(held)):
+        torch.cuda._sleep(2_000_000_000)  # about a second
+    for o in outs[:30]:
+        launch(held, o)
+    for st, o in zip(others, outs[30:]):
+        launch(st, o)
+    # (of eight streams: one that happens to share a hardware queue with the held one does wait)
+    ends = [torch.cuda.ExternalStream(st) for st in others]
+    t0, passed = time.time(), False
+    while not passed and time.time() - t0 < 0.5:
+        passed = any(e.query() for e in ends)
+    assert passed and not torch.cuda.ExternalStream(held).query()
+    for i, o in enumerate(outs[38:178]):
+        launch(others[i % 3], o)
+    torch.cuda.synchronize()
+    pkg.check(held)
+    assert all(torch.equal(o, want) for o in outs[:178])
+    for st in [held] + others:
+        assert int(rt.cudaStreamDestroy(st)) == 0
+
+
+def test_per_thread_default_stream(pkg):
+    """cudaStreamPerThread names another stream in every host thread, and streams are told apart by their id."""
+    import ctypes
+    import threading
+
+    import torch
+
+    per_thread = 2  # the handle cudaStreamPerThread
+    cu = ctypes.CDLL("libcuda.so.1")
+    g = torch.Generator(device="cuda").manual_seed(10)
+    B, H, N, d = 1, 24, 1024, 64
+    q, k, v = (torch.randn((B, H, N, d), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    want = pkg.attention_forward(q, k, v)
+    outs = [[torch.full_like(q, float("nan")) for _ in range(40)] for _ in range(2)]
+    torch.cuda.synchronize()
+    ids, errors, both = [None, None], [], threading.Barrier(2)
+
+    def work(t):
+        try:
+            torch.cuda.set_device(q.device)
+            torch.cuda.current_stream().query()
+            both.wait()
+            for o in outs[t]:
+                pkg.flash_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), B, H, N, d, stream=per_thread)
+            pkg.check(per_thread)
+            sid = ctypes.c_ulonglong()
+            assert cu.cuStreamGetId(ctypes.c_void_p(per_thread), ctypes.byref(sid)) == 0
+            ids[t] = sid.value
+            both.wait()
+        except BaseException as e:  # reported by the main thread
+            errors.append(e)
+            both.abort()
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert ids[0] != ids[1]
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for side in outs for o in side)
 
 
 def exact_attention(q, k, v, scale, causal):
