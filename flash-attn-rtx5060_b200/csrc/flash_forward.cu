@@ -254,7 +254,6 @@ int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMa
   int rc = ensure_smem_attr(s, slot, fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout>, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
   fa::FwdParams pp = p;
-  fa::set_work_items(&pp, s->num_sms);
   const int grid = pp.num_items < s->num_sms ? pp.num_items : s->num_sms;
   std::lock_guard<std::mutex> lk(s->mu);
   int sched_slot = 0;
@@ -372,7 +371,6 @@ int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUte
                               const CUtensorMap& mo,
                               fa::FwdParams p, cudaStream_t st, bool early) {
   using Cfg = fa::PersistentCfg<D>;
-  fa::set_work_items(&p, s->num_sms);
   {
     std::lock_guard<std::mutex> lk(s->mu);
     bool& done = s->attr_set[D == 64 ? 0 : 1];
@@ -391,39 +389,6 @@ int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUte
 }
 
 }  // namespace
-
-// Heads per scheduling group of the persistent kernel. Without a mask all items cost the same and head-major
-// order (1) shares K/V best. With a causal mask or a window the item costs differ, and interleaving the heads of
-// a group pair-major makes the order of the group longest first. Measured constraints (B200): the K and V rows that a
-// group keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
-// what both dies read: the long-context workload read K/V from DRAM 2.2 times with 96 MB in flight, 1.5 times
-// with 64 MB, 1.1 times with 48 MB, at the same speed; the 8192-row config is 0.6 % faster with 64 MB than
-// with 48); a group needs about two items per CTA to balance; and the groups must be of even size (64 heads in
-// groups of 12 leave a last group of 4 heads, too few items for 148 CTAs: -4 %). Within those limits a group is as
-// large as it can be: with one group for all heads the whole launch is handed out longest first and ends on its
-// cheapest items. Against groups of at most 16 heads: B4 H16 N2048 d64 causal 82.4 -> 72.8 us, 24 heads of 4001 rows
-// d128 with log-sum-exp 132 -> 116, B2 H16 N4096 d64 ALiBi 161 -> 136, B8 H16 N1024 d128 70 -> 58.
-// (flash_forward_head_group reports base groups, `most` = 16 heads; a launch takes as many heads as fit.)
-static int pick_head_group(int bh, int seqlen, int head_dim, int causal, int window_left, int window_right,
-                           int num_q_pairs, int num_sms, int most = 0x7fffffff) {
-  if (!causal && window_left < 0 && window_right < 0) return 1;
-  const int wr = causal ? 0 : window_right;
-  long long span = seqlen;
-  if (window_left >= 0 && wr >= 0) {
-    span = (long long)window_left + wr + 2 * fa::kBlockM;
-    if (span > seqlen) span = seqlen;
-  }
-  const double span_bytes = 4.0 * (double)span * head_dim;  // K and V rows, fp16
-  int grp_l2 = (int)(64.0 * 1024 * 1024 / span_bytes);
-  const int grp_bal = (2 * num_sms + num_q_pairs - 1) / num_q_pairs;
-  int grp = grp_l2;
-  if (grp < grp_bal) grp = grp_bal;
-  if (grp > most) grp = most;
-  if (grp < 1) grp = 1;
-  if (grp > bh) grp = bh;
-  const int groups = (bh + grp - 1) / grp;
-  return (bh + groups - 1) / groups;
-}
 
 // A window that reaches past either end of the sequence for every row is no window. Mapping it to
 // "unbounded" (-1) here keeps the tile arithmetic (row - window_left, row + window_right) inside int
@@ -456,7 +421,7 @@ int flash_forward_head_group(int batch_heads, int seqlen, int head_dim, int is_c
                              int window_right, int num_sms) {
   if (batch_heads <= 0 || seqlen <= 0 || (head_dim != 64 && head_dim != 128) || num_sms <= 0) return 0;
   const int pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
-  return pick_head_group(batch_heads, seqlen, head_dim, is_causal ? 1 : 0, norm_window(window_left, seqlen),
+  return fa::pick_head_group(batch_heads, seqlen, head_dim, is_causal ? 1 : 0, norm_window(window_left, seqlen),
                          norm_window(window_right, seqlen), pairs, num_sms, 16);
 }
 
@@ -479,7 +444,8 @@ int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int windo
 static int forward_impl(const void* q, const void* k, const void* v, void* o, int batch, int heads, int seqlen,
                         int head_dim, float softmax_scale, int is_causal, int window_left, int window_right,
                         const float* alibi_slopes, void* stream, int kernel, int variant, float* dbg,
-                        float* lse = nullptr, float dropout_prob = 0.f, unsigned long long seed = 0) {
+                        float* lse = nullptr, float dropout_prob = 0.f, unsigned long long seed = 0,
+                        long long first_head = 0, long long total_heads = 0) {
   if (!q || !k || !v || !o) return fail(FA_INVALID_ARG, "null tensor pointer");
   if (reinterpret_cast<uintptr_t>(lse) & 3) return fail(FA_INVALID_ARG, "lse must be 4-byte aligned");
   if (lse && kernel != 0) return fail(FA_UNSUPPORTED, "only the default kernel writes the log-sum-exp");
@@ -533,7 +499,11 @@ static int forward_impl(const void* q, const void* k, const void* v, void* o, in
   p.num_q_pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
   if ((long long)bh * p.num_q_pairs > 0x7fffffffLL) return fail(FA_INVALID_ARG, "too many work items");
   p.num_items = bh * p.num_q_pairs;
-  p.head_group = pick_head_group(bh, seqlen, head_dim, p.causal, p.window_left, p.window_right, p.num_q_pairs, s->num_sms);
+  if (kernel == 0)
+    fa::set_work_items(&p, head_dim, s->num_sms, first_head, total_heads > 0 ? total_heads : bh);
+  else
+    p.head_group = fa::pick_head_group(bh, seqlen, head_dim, p.causal, p.window_left, p.window_right, p.num_q_pairs,
+                                       s->num_sms);
 
   CUtensorMap mq, mk, mv, mo;
   if ((rc = make_map(&mq, q, bh, seqlen, head_dim, fa::kBlockM)) != FA_OK) return rc;
@@ -603,13 +573,17 @@ int flash_forward_multi_gpu(int num_slabs, const int* devices, const void* const
   cudaError_t e = cudaGetDevice(&prev);
   if (e != cudaSuccess) return fail_cuda("cudaGetDevice", e);
   int rc = FA_OK;
+  long long total_heads = 0, first_head = 0;
+  for (int i = 0; i < num_slabs; ++i) total_heads += slab_heads[i] > 0 ? slab_heads[i] : 0;
   // Enqueue on every device first (the launches are asynchronous, so the devices run side by side),
   // then, if asked, wait for each and read its status word.
   for (int i = 0; i < num_slabs && rc == FA_OK; ++i) {
     if (slab_heads[i] == 0) continue;  // a device may be left without work
     if ((e = cudaSetDevice(devices[i])) != cudaSuccess) { rc = fail_cuda("cudaSetDevice", e); break; }
     rc = forward_impl(q[i], k[i], v[i], o[i], 1, slab_heads[i], seqlen, head_dim, softmax_scale, is_causal, window_left,
-                      window_right, nullptr, streams ? streams[i] : nullptr, 0, 0, nullptr);
+                      window_right, nullptr, streams ? streams[i] : nullptr, 0, 0, nullptr, nullptr, 0.f, 0, first_head,
+                      total_heads);
+    first_head += slab_heads[i];
   }
   for (int i = 0; wait && i < num_slabs && rc == FA_OK; ++i) {
     if (slab_heads[i] == 0) continue;
@@ -717,8 +691,9 @@ int flash_forward_host(const void* q_host, const void* k_host, const void* v_hos
     FA_TRY(cudaStreamWaitEvent(hp->run, hp->in_ready[slot], 0));
     if (n >= 2) FA_TRY(cudaStreamWaitEvent(hp->run, hp->out_done[slot], 0));
     if (what) break;
-    rc = flash_forward(dev_ptr(slot, 0), dev_ptr(slot, 1), dev_ptr(slot, 2), dev_ptr(slot, 3), 1, nh, seqlen, head_dim,
-                       softmax_scale, is_causal, window_left, window_right, hp->run);
+    rc = forward_impl(dev_ptr(slot, 0), dev_ptr(slot, 1), dev_ptr(slot, 2), dev_ptr(slot, 3), 1, nh, seqlen, head_dim,
+                      softmax_scale, is_causal, window_left, window_right, nullptr, hp->run, 0, 0, nullptr, nullptr, 0.f,
+                      0, h0, bh);
     if (rc != FA_OK) break;
     FA_TRY(cudaEventRecord(hp->done[slot], hp->run));
     FA_TRY(cudaStreamWaitEvent(hp->down, hp->done[slot], 0));
@@ -792,8 +767,7 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   p.window_right = norm_window(window_right, seqlen);
   p.status = words;
   p.num_q_pairs = pairs;
-  p.num_items = bh * pairs;
-  p.head_group = pick_head_group(bh, seqlen, head_dim, p.causal, p.window_left, p.window_right, pairs, s->num_sms);
+  fa::set_work_items(&p, head_dim, s->num_sms, 0, bh);
 
   CUtensorMap mq, mk, mv, mo;
   if ((rc = make_map(&mq, q, bh, seqlen, head_dim, fa::kBlockM)) != FA_OK) return rc;

@@ -14,6 +14,39 @@ namespace fa {
 
 __host__ __device__ inline int min_int(int a, int b) { return a < b ? a : b; }
 
+// Heads per scheduling group of the persistent kernel. Without a mask all items cost the same and head-major
+// order (1) shares K/V best. With a causal mask or a window the item costs differ, and interleaving the heads of
+// a group pair-major makes the order of the group longest first. Measured constraints (B200): the K and V rows that a
+// group keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
+// what both dies read: the long-context workload read K/V from DRAM 2.2 times with 96 MB in flight, 1.5 times
+// with 64 MB, 1.1 times with 48 MB, at the same speed; the 8192-row config is 0.6 % faster with 64 MB than
+// with 48); a group needs about two items per CTA to balance; and the groups must be of even size (64 heads in
+// groups of 12 leave a last group of 4 heads, too few items for 148 CTAs: -4 %). Within those limits a group is as
+// large as it can be: with one group for all heads the whole launch is handed out longest first and ends on its
+// cheapest items. Against groups of at most 16 heads: B4 H16 N2048 d64 causal 82.4 -> 72.8 us, 24 heads of 4001 rows
+// d128 with log-sum-exp 132 -> 116, B2 H16 N4096 d64 ALiBi 161 -> 136, B8 H16 N1024 d128 70 -> 58.
+// (flash_forward_head_group reports base groups, `most` = 16 heads; a launch takes as many heads as fit.)
+inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int window_left, int window_right,
+                           int num_q_pairs, int num_sms, int most = 0x7fffffff) {
+  if (!causal && window_left < 0 && window_right < 0) return 1;
+  const int wr = causal ? 0 : window_right;
+  long long span = seqlen;
+  if (window_left >= 0 && wr >= 0) {
+    span = (long long)window_left + wr + 2 * kBlockM;
+    if (span > seqlen) span = seqlen;
+  }
+  const double span_bytes = 4.0 * (double)span * head_dim;  // K and V rows, fp16
+  int grp_l2 = (int)(64.0 * 1024 * 1024 / span_bytes);
+  const int grp_bal = (2 * num_sms + num_q_pairs - 1) / num_q_pairs;
+  int grp = grp_l2;
+  if (grp < grp_bal) grp = grp_bal;
+  if (grp > most) grp = most;
+  if (grp < 1) grp = 1;
+  if (grp > bh) grp = bh;
+  const int groups = (bh + grp - 1) / grp;
+  return (bh + groups - 1) / groups;
+}
+
 // Takes some of the pairs of q tiles apart into single q tiles whose kv tiles the two stages of a CTA share out
 // (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
 // the epilogue merges two outputs), but there are twice as many items of half the length.
@@ -25,21 +58,39 @@ __host__ __device__ inline int min_int(int a, int b) { return a < b ? a : b; }
 //   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
 //   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
 //   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
-inline void set_work_items(FwdParams* p, int num_sms) {
-  const int pairs = p->num_items;
-  int split = 0;
-  if (p->seqlen > kBlockM && pairs < (1 << 30)) {
-    const int wl = p->window_left, wr = eff_window_right(p->causal, p->window_right);
-    const bool even = (wl < 0 && wr < 0) || (wl >= 0 && wr >= 0 && wl < p->seqlen / 4 && wr < p->seqlen / 4);
-    if (even) {
-      const int tail = pairs % num_sms;
-      if (2 * tail <= num_sms) split = tail;
-    } else if (2 * pairs <= num_sms || 4LL * pairs <= 7LL * num_sms) {
-      if (2 * pairs <= num_sms || 7LL * pairs <= (long long)p->num_q_pairs * num_sms) split = pairs;
-    }
+inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, int window_left, int window_right,
+                                int num_sms) {
+  if (seqlen <= kBlockM || pairs >= (1 << 30)) return 0;
+  const bool even = (window_left < 0 && window_right < 0) || (window_left >= 0 && window_right >= 0 &&
+                                                               window_left < seqlen / 4 && window_right < seqlen / 4);
+  if (even) {
+    const long long tail = pairs % num_sms;
+    return 2 * tail <= num_sms ? tail : 0;
   }
-  p->num_pair_items = pairs - split;
-  p->num_items = pairs + split;
+  if (2 * pairs <= num_sms || 4 * pairs <= 7LL * num_sms) {
+    if (2 * pairs <= num_sms || 7 * pairs <= (long long)num_q_pairs * num_sms) return pairs;
+  }
+  return 0;
+}
+
+// The items of a launch on p->bh heads, the first of which is head `first_head` of a problem of `total_heads`: its order
+// (head_group), and how many pairs at the end of that order are taken apart. A split q tile is summed in another order
+// than a pair's, so which pairs are split is decided for the whole problem: the chunks of flash_forward_host and the slabs
+// of flash_forward_multi_gpu give the bits of the call on all heads. Where only the last pairs of the problem are
+// split, the order is head-major, in which the last pairs of a chunk or slab are the problem's if it holds any of them.
+inline void set_work_items(FwdParams* p, int head_dim, int num_sms, long long first_head, long long total_heads) {
+  const int wl = p->window_left, wr = eff_window_right(p->causal, p->window_right);
+  const long long all = total_heads * p->num_q_pairs;
+  const long long split = pairs_to_split(all, p->num_q_pairs, p->seqlen, wl, wr, num_sms);
+  const int pairs = p->bh * p->num_q_pairs;
+  p->head_group = (split > 0 && split < all)
+                      ? 1
+                      : pick_head_group(p->bh, p->seqlen, head_dim, p->causal, p->window_left, p->window_right,
+                                        p->num_q_pairs, num_sms);
+  long long mine = (first_head + p->bh) * p->num_q_pairs - (all - split);
+  mine = mine < 0 ? 0 : (mine > pairs ? pairs : mine);
+  p->num_pair_items = pairs - static_cast<int>(mine);
+  p->num_items = pairs + static_cast<int>(mine);
 }
 
 // Work item -> geometry. Every role decodes the same item the same way.

@@ -45,8 +45,9 @@ enum {
  * The call returns once the kernel is enqueued; use flash_forward_check() to learn whether a
  * device-side wait timed out.
  *
- * Two calls with the same arguments give the same bits. The split of the work among the SMs depends on
- * batch*heads, so a head may differ in the last place between a call on all heads and a call on some of them.
+ * Two calls with the same arguments give the same bits, and so do flash_forward_host and flash_forward_multi_gpu on the
+ * same heads. The split of the work among the SMs depends on batch*heads, so a head may differ in the last place
+ * between a call on all heads and a separate call on some of them.
  *
  * Launches in flight: every launch uses a pair of scheduler words (2.5 KB of device scratch,
  * allocated on the first call per device). The first 256 streams that are used on a device own a pair each,

@@ -50,6 +50,32 @@ def test_slabs_equal_single_call(pkg, N, d, causal, wl):
     assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
 
 
+# Slabs that, called separately, would take other pairs of q tiles apart than the call on all heads does: few heads of a
+# causal problem, the last heads of a launch whose last pairs are split, with and without a window.
+@pytest.mark.parametrize("H,N,d,causal,wl,cuts", [
+    (40, 2048, 64, True, -1, (5, 20)), (75, 512, 64, False, -1, (70, 72)), (152, 1000, 128, True, 100, (20, 147)),
+])
+def test_slabs_equal_single_call_where_pairs_are_split(pkg, H, N, d, causal, wl, cuts):
+    import torch
+
+    q, k, v = make_inputs(950 + N, 1, H, N, d)
+    tq, tk, tv = (torch.from_numpy(a).cuda() for a in (q, k, v))
+    want = pkg.attention_forward(tq, tk, tv, causal=causal, window_left=wl)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    want = want.cpu().numpy()
+    n_dev = torch.cuda.device_count()
+    got = run_slabs(pkg, q, k, v, [i % n_dev for i in range(3)], cuts=cuts, causal=causal, wl=wl)
+    assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+    # the same through host buffers, in chunks of 7 heads
+    hq, hk, hv = (torch.from_numpy(a).pin_memory() for a in (q, k, v))
+    ho = torch.empty((1, H, N, d), dtype=torch.float16).pin_memory()
+    nbytes = pkg.host_workspace_bytes(N, d, 7)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    pkg.flash_forward_host(hq.data_ptr(), hk.data_ptr(), hv.data_ptr(), ho.data_ptr(), 1, H, N, d, ws.data_ptr(), nbytes,
+                           7, is_causal=causal, window_left=wl)
+    assert np.array_equal(ho.numpy().view(np.uint16), want.view(np.uint16))
+
+
 def test_every_visible_device_gives_the_same_bits(pkg):
     """BASELINE config 3's per-head shape on every GPU of the machine: each device computes the same two
     heads; all results must be identical (no device-dependent state in the library)."""

@@ -620,6 +620,19 @@ def test_head_shards_equal_full_call(pkg):
             assert torch.equal(part[0], full[sl])
 
 
+def test_separate_calls_on_head_shards_agree_to_an_ulp(pkg):
+    # Separate calls do not know of one another: five heads of this problem are taken apart into single q tiles, all forty
+    # are not, so their sums run in another order.
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    q, k, v = (torch.randn((1, 40, 2048, 64), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    full = pkg.attention_forward(q, k, v, causal=True).cpu().numpy()
+    for h in range(0, 40, 5):
+        part = pkg.attention_forward(*(x[:, h:h + 5].contiguous() for x in (q, k, v)), causal=True)
+        assert_close_or_one_ulp(part.cpu().numpy(), full[:, h:h + 5])
+
+
 def test_reference_entry_point_mapping(pkg, ob, capfd):
     # run_flash_attention(B, heads, S, d, Q, K, V, O, L, M, dropout, causal, local, alibi, window, ...)
     import torch

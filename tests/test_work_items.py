@@ -25,16 +25,16 @@ def wi(tmp_path_factory):
 
 
 class Launch:
-    def __init__(self, wi, bh, n, causal=False, wl=-1, wr=-1, group=1, sms=SMS):
-        self.wi, self.args = wi, (bh, n, int(causal), wl, wr, group, sms)
-        items, pairs = ctypes.c_int(), ctypes.c_int()
-        wi.plan(*self.args, ctypes.byref(items), ctypes.byref(pairs))
-        self.items, self.pair_items = items.value, pairs.value
+    def __init__(self, wi, bh, n, d=64, causal=False, wl=-1, wr=-1, first=0, total=0):
+        self.wi, self.args = wi, (ctypes.c_int * 9)(bh, n, d, int(causal), wl, wr, SMS, first, total or bh)
+        out = (ctypes.c_int * 3)()
+        wi.plan(self.args, out)
+        self.items, self.pair_items, self.group = out
 
     def walk(self, item, claims):
         out = (ctypes.c_int * 16)()
         claims = (ctypes.c_int * (len(claims) + 1))(*claims, self.items)
-        used = self.wi.walk(*self.args, item, claims, out)
+        used = self.wi.walk(self.args, item, claims, out)
         keys = ("item", "head", "r0a", "r1a", "loa", "hia", "r0b", "r1b", "lob", "hib", "top", "steps", "split")
         return dict(zip(keys, out)), used
 
@@ -53,9 +53,12 @@ class Launch:
 
 SHAPES = [
     dict(bh=100, n=300), dict(bh=111, n=300), dict(bh=123, n=600), dict(bh=75, n=333), dict(bh=3, n=129),
-    dict(bh=1, n=100), dict(bh=2, n=129, causal=True), dict(bh=80, n=450, causal=True, wl=60, group=80),
-    dict(bh=5, n=1000, wl=100, wr=5, group=5), dict(bh=8, n=2304 + 77, causal=True, group=8),
-    dict(bh=40, n=4097, causal=True, group=14), dict(bh=7, n=700, wl=50, group=7), dict(bh=96, n=1000),
+    dict(bh=1, n=100), dict(bh=2, n=129, causal=True), dict(bh=80, n=450, causal=True, wl=60),
+    dict(bh=5, n=1000, wl=100, wr=5), dict(bh=8, n=2304 + 77, causal=True),
+    dict(bh=40, n=4097, causal=True), dict(bh=7, n=700, wl=50), dict(bh=96, n=1000),
+    # window, last pairs split; causal with several head groups; causal, all pairs split; slabs of such problems
+    dict(bh=152, n=1000, d=128, wl=100, wr=0), dict(bh=64, n=32768 // 8 + 5, d=128, causal=True), dict(bh=8, n=4096, causal=True),
+    dict(bh=5, n=512, first=70, total=75), dict(bh=5, n=2048, causal=True, first=0, total=40),
 ]
 
 
@@ -85,6 +88,26 @@ def test_every_q_tile_once_with_its_kv_tiles(wi, pkg, shape):
     for (_, r0), js in seen.items():
         lo, hi, _ = pkg.kv_range(n, causal, wl, wr, r0, min(r0 + 128, n) - 1)
         assert sorted(js) == list(range(lo, hi))
+
+
+@pytest.mark.parametrize("shape", [
+    dict(n=512, total=75), dict(n=333, total=75), dict(n=2048, total=40, causal=True), dict(n=4096, total=9, causal=True),
+    dict(n=8192, total=32, d=128, causal=True), dict(n=1000, total=152, wl=100, wr=0), dict(n=4096, total=10, causal=True, wl=500),
+    dict(n=900, total=41, wl=60), dict(n=4096, total=30),
+], ids=str)
+def test_slabs_take_the_same_pairs_apart(wi, shape):
+    """Whether a q tile is summed by one stage or by two does not depend on how the heads are cut into calls that know the
+    whole problem (the bits of flash_forward_host and flash_forward_multi_gpu)."""
+    def split_tiles(**kw):
+        L = Launch(wi, **{**shape, **kw})
+        geoms = (L.walk(i, [])[0] for i in range(L.items))
+        return {(kw["first"] + g["head"], g["r0a"]) for g in geoms if g["item"] >= 0 and g["split"]}
+
+    total = shape["total"]
+    whole = split_tiles(bh=total, first=0)
+    for step in (1, 3, 8, total - 1):
+        parts = [split_tiles(bh=min(step, total - h), first=h) for h in range(0, total, step)]
+        assert set().union(*parts) == whole
 
 
 def ring_ends(rows):

@@ -4,37 +4,34 @@
 #include "work_items.h"
 
 namespace {
-fa::FwdParams params(int bh, int seqlen, int causal, int window_left, int window_right, int head_group, int num_sms) {
+fa::FwdParams params(const int* a) {  // bh, seqlen, head_dim, causal, window_left, window_right, num_sms, first, total heads
   fa::FwdParams p;
   std::memset(&p, 0, sizeof(p));
-  p.bh = bh;
-  p.seqlen = seqlen;
-  p.causal = causal;
-  p.window_left = window_left;
-  p.window_right = window_right;
-  p.head_group = head_group;
-  p.num_q_pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
-  p.num_items = bh * p.num_q_pairs;
-  fa::set_work_items(&p, num_sms);
+  p.bh = a[0];
+  p.seqlen = a[1];
+  p.causal = a[3];
+  p.window_left = a[4];
+  p.window_right = a[5];
+  p.num_q_pairs = (p.seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
+  fa::set_work_items(&p, a[2], a[6], a[7], a[8]);
   return p;
 }
 }  // namespace
 
 extern "C" {
 
-// Number of items, and of those the pairs, that a launch hands out.
-void plan(int bh, int seqlen, int causal, int window_left, int window_right, int head_group, int num_sms, int* items,
-          int* pair_items) {
-  const fa::FwdParams p = params(bh, seqlen, causal, window_left, window_right, head_group, num_sms);
-  *items = p.num_items;
-  *pair_items = p.num_pair_items;
+// out[0..2] = number of items that a launch hands out, of those the pairs, heads per scheduling group
+void plan(const int* args, int* out) {
+  const fa::FwdParams p = params(args);
+  out[0] = p.num_items;
+  out[1] = p.num_pair_items;
+  out[2] = p.head_group;
 }
 
-// next_item() from `item` on, claims taken from the list; out[0..13] = item, head, rows and steps of both stages, top,
+// next_item() from `item` on, claims taken from the list; out[0..12] = item, head, rows and steps of both stages, top,
 // steps, split. Returns the number of claims used.
-int walk(int bh, int seqlen, int causal, int window_left, int window_right, int head_group, int num_sms, int item,
-         const int* claims, int* out) {
-  const fa::FwdParams p = params(bh, seqlen, causal, window_left, window_right, head_group, num_sms);
+int walk(const int* args, int item, const int* claims, int* out) {
+  const fa::FwdParams p = params(args);
   fa::ItemGeom g;
   std::memset(&g, 0, sizeof(g));
   int used = 0;
