@@ -420,9 +420,17 @@ double flash_forward_flops(int batch, int heads, int seqlen, int head_dim, int i
 int flash_forward_head_group(int batch_heads, int seqlen, int head_dim, int is_causal, int window_left,
                              int window_right, int num_sms) {
   if (batch_heads <= 0 || seqlen <= 0 || (head_dim != 64 && head_dim != 128) || num_sms <= 0) return 0;
-  const int pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
-  return fa::pick_head_group(batch_heads, seqlen, head_dim, is_causal ? 1 : 0, norm_window(window_left, seqlen),
-                         norm_window(window_right, seqlen), pairs, num_sms, 16);
+  fa::FwdParams p;
+  memset(&p, 0, sizeof(p));
+  p.bh = batch_heads;
+  p.seqlen = seqlen;
+  p.causal = is_causal ? 1 : 0;
+  p.window_left = norm_window(window_left, seqlen);
+  p.window_right = norm_window(window_right, seqlen);
+  p.num_q_pairs = (seqlen + 2 * fa::kBlockM - 1) / (2 * fa::kBlockM);
+  if ((long long)batch_heads * p.num_q_pairs > 0x7fffffffLL) return 0;
+  fa::set_work_items(&p, head_dim, num_sms, 0, batch_heads);
+  return p.head_group;
 }
 
 int flash_forward_kv_range(int seqlen, int is_causal, int window_left, int window_right, int row_begin,

@@ -25,7 +25,6 @@ __host__ __device__ inline int min_int(int a, int b) { return a < b ? a : b; }
 // large as it can be: with one group for all heads the whole launch is handed out longest first and ends on its
 // cheapest items. Against groups of at most 16 heads: B4 H16 N2048 d64 causal 82.4 -> 72.8 us, 24 heads of 4001 rows
 // d128 with log-sum-exp 132 -> 116, B2 H16 N4096 d64 ALiBi 161 -> 136, B8 H16 N1024 d128 70 -> 58.
-// (flash_forward_head_group reports base groups, `most` = 16 heads; a launch takes as many heads as fit.)
 inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int window_left, int window_right,
                            int num_q_pairs, int num_sms, int most = 0x7fffffff) {
   if (!causal && window_left < 0 && window_right < 0) return 1;

@@ -170,9 +170,8 @@ int run_flash_attention_c(int B, int N, int S, int d, void* Q, void* K, void* V,
                           int Is_dropout, int Is_causal, int Is_local, int Has_alibi, int window_size,
                           float* alibi_slopes, float dropout_prob, void* states);
 
-/* Heads per base scheduling group of the default kernel for batch_heads = batch*heads problems of this shape on a
- * GPU with num_sms SMs (1 = head-major order, at most 16). Where the K and V of several base groups fit L2 together the
- * kernel hands their work out as one group. Host logic only, for tests and tuning; the reference
+/* Heads per scheduling group of a launch of the default kernel on batch_heads = batch*heads problems of this shape on a
+ * GPU with num_sms SMs (1 = head-major order). Host logic only, for tests and tuning; the reference
  * schedules q tiles in natural order (src/flash_forward.h:43-64) and has no such notion. 0 on bad arguments. */
 int flash_forward_head_group(int batch_heads, int seqlen, int head_dim, int is_causal, int window_left,
                              int window_right, int num_sms);

@@ -62,6 +62,12 @@ SHAPES = [
 ]
 
 
+@pytest.mark.parametrize("shape", [s for s in SHAPES if "total" not in s], ids=str)
+def test_head_group_is_the_launch_s(wi, pkg, shape):
+    s = {"d": 64, "causal": False, "wl": -1, "wr": -1, **shape}
+    assert pkg.head_group(s["bh"], s["n"], s["d"], s["causal"], s["wl"], s["wr"], SMS) == Launch(wi, **shape).group
+
+
 @pytest.mark.parametrize("shape", SHAPES, ids=str)
 def test_every_q_tile_once_with_its_kv_tiles(wi, pkg, shape):
     L = Launch(wi, **shape)
