@@ -509,9 +509,9 @@ static int forward_impl(const void* q, const void* k, const void* v, void* o, in
   p.num_items = bh * p.num_q_pairs;
   if (kernel == 0)
     fa::set_work_items(&p, head_dim, s->num_sms, first_head, total_heads > 0 ? total_heads : bh);
-  else
+  else  // the CTA-pair kernel was measured with groups of at most 16 heads (its items are assigned statically)
     p.head_group = fa::pick_head_group(bh, seqlen, head_dim, p.causal, p.window_left, p.window_right, p.num_q_pairs,
-                                       s->num_sms);
+                                       s->num_sms, 16);
 
   CUtensorMap mq, mk, mv, mo;
   if ((rc = make_map(&mq, q, bh, seqlen, head_dim, fa::kBlockM)) != FA_OK) return rc;
