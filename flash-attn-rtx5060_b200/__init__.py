@@ -207,11 +207,17 @@ def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, so
         return _enqueue_forward(device, *args)
 
 
+def _current_raw_stream(torch, device):
+    """Handle of the current stream. Building a torch.cuda.Stream object and entering a device context for every call
+    cost 5 us of the 14 us a call took on the host, more than the kernel of a small call (B1 H4 N512 d64), so the handle
+    comes from the accessor that torch's own generated code uses; it is not public API, hence the second way."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream
+
+
 def _enqueue_forward(device, torch, q, k, v, out, causal, window_left, window_right, softmax_scale, kernel, variant,
                      alibi_slopes, return_lse, dropout_p, seed):
-    # The raw handle of the current stream: building a torch.cuda.Stream object and entering a device context for every
-    # call cost 5 us of the 14 us a call took on the host, more than the kernel of a small call (B1 H4 N512 d64).
-    stream = torch._C._cuda_getCurrentRawStream(device)
+    stream = _current_raw_stream(torch, device)
     B, H, N, d = q.shape
     L = lib()
     lse = None

@@ -79,6 +79,15 @@ def test_no_gpu_is_an_error_not_a_fallback(pkg):
     assert rc in (pkg.FA_CUDA_ERROR, pkg.FA_UNSUPPORTED)
 
 
+def test_current_stream_without_the_private_accessor(pkg):
+    from types import SimpleNamespace as NS
+
+    public = NS(current_stream=lambda device: NS(cuda_stream=("public", device)))
+    assert pkg._current_raw_stream(NS(_C=NS(), cuda=public), 3) == ("public", 3)
+    private = NS(_cuda_getCurrentRawStream=lambda device: ("raw", device))
+    assert pkg._current_raw_stream(NS(_C=private, cuda=public), 3) == ("raw", 3)
+
+
 def brute_pairs(N, causal, wl, wr):
     i = np.arange(N)[:, None]
     j = np.arange(N)[None, :]
