@@ -58,13 +58,17 @@ def test_lse_with_alibi_and_scale(pkg, ob):
     assert np.abs(lse2.cpu().numpy() - want2).max() <= 2e-3  # logits of +-40
 
 
-def test_lse_growing_row_max(pkg, ob):
-    """Keys grow along the sequence, so the running max moves in every tile and the lazy threshold is
-    crossed repeatedly; the final (max, sum) pair must still describe the whole row."""
+@pytest.mark.parametrize("falling", [False, True])
+def test_lse_growing_row_max(pkg, ob, falling):
+    """Keys grow along the sequence or against it (the kernel walks from the last kv tile to the first), so the running
+    max moves in every tile and the lazy threshold is crossed repeatedly; the final (max, sum) pair must still describe
+    the whole row."""
     N, d = 1536, 64
     rng = np.random.default_rng(9)
     q = np.abs(rng.standard_normal((1, 2, N, d), dtype=np.float32)).astype(np.float16)
     ramp = np.linspace(0.05, 3.0, N, dtype=np.float32)[None, None, :, None]
+    if falling:
+        ramp = ramp[:, :, ::-1]
     k = (np.abs(rng.standard_normal((1, 2, N, d), dtype=np.float32)) * ramp).astype(np.float16)
     v = rng.standard_normal((1, 2, N, d), dtype=np.float32).astype(np.float16)
     _, lse, _ = run(pkg, q, k, v, causal=False)

@@ -1,4 +1,5 @@
-"""flash_forward_multi_gpu: slabs of heads on one or several devices equal the single call bit for bit.
+"""flash_forward_multi_gpu: slabs of heads on one or several devices equal the single call bit for bit, also where a slab
+alone would be split among the SMs in another way.
 On a one-GPU machine both slabs run on device 0; with two or more GPUs every slab has its own device."""
 import numpy as np
 import pytest

@@ -535,34 +535,47 @@ def test_tiny_scale_keeps_hidden_keys_hidden(pkg, ob, scale):
         assert np.abs(got[:, :, i] - want).max() <= 2e-3, i
 
 
-def test_growing_row_max_forces_rescale(pkg, ob):
-    # keys ordered so that every later kv tile raises the row max by far more than the lazy threshold
+@pytest.mark.parametrize("falling", [False, True])
+def test_growing_row_max_forces_rescale(pkg, ob, falling):
+    # keys ordered so that every later kv tile raises the row max by far more than the lazy threshold: in the order of the
+    # columns for the serial kernel, against it for the default kernel, which walks from the last kv tile to the first
     N, d = 1024, 64
     rng = np.random.default_rng(12)
     q = np.ones((1, 1, N, d), np.float16)
     k = (np.arange(N, dtype=np.float32)[:, None] / 8.0 * np.ones((1, d), np.float32) / d * 8).astype(np.float16)
     k = k.reshape(1, 1, N, d)
+    if falling:
+        k = np.ascontiguousarray(k[:, :, ::-1])
     v = rng.standard_normal((1, 1, N, d), dtype=np.float32).astype(np.float16)
     for kernel in (0, 1):
         got = run_gpu(pkg, q, k, v, False, -1, -1, kernel, scale=1.0)
-        want = ob.attention(q, k, v, scale=1.0)
+        # All rows are one and the same here, 64 numbers in all. With falling keys the oracle, which rounds probabilities
+        # to fp16, has a mean error of 2.33e-4 in them against fp64 (1.87e-4 with rising ones), above the bar of 2e-4 for
+        # means; the rounded fp64 result (1.06e-4 from the unrounded) is the reference there.
+        want = exact_attention(q, k, v, 1.0, False) if falling else ob.attention(q, k, v, scale=1.0)
         assert_close_or_one_ulp(got, want)
 
 
-def exact_attention_gpu(q, k, v, causal):
-    """fp64 attention of fp16 torch tensors [B, H, N, d], on their device."""
+def exact_attention_gpu(q, k, v, causal, slopes=None):
+    """fp64 attention of fp16 torch tensors [B, H, N, d], on their device, and its log-sum-exp."""
     import torch
 
     n = q.shape[2]
+    gap = torch.arange(n, device=q.device, dtype=torch.float64)
+    gap = (gap[:, None] - gap[None, :]).abs()
+    lse = torch.empty(q.shape[:3], dtype=torch.float64, device=q.device)
     hidden = torch.ones((n, n), dtype=torch.bool, device=q.device).triu(1) if causal else None
     out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
     for b in range(q.shape[0]):
         for h in range(q.shape[1]):
             s = q[b, h].double() @ k[b, h].double().T / q.shape[3] ** 0.5
+            if slopes is not None:
+                s -= slopes[h].double() * gap
             if causal:
                 s.masked_fill_(hidden, float("-inf"))
             out[b, h] = torch.softmax(s, -1) @ v[b, h].double()
-    return out
+            lse[b, h] = torch.logsumexp(s, -1)
+    return out, lse
 
 
 # A key near the start of the sequence that stands out by `up` powers of two for every row, as the first keys do in trained
@@ -583,13 +596,64 @@ def test_row_dominated_by_an_early_key(pkg, H, N, d, causal, up):
     q, k, v = q.half(), k.half(), v.half()
     out = pkg.attention_forward(q, k, v, causal=causal)
     pkg.check(torch.cuda.current_stream().cuda_stream)
-    exact = exact_attention_gpu(q, k, v, causal)
+    exact, _ = exact_attention_gpu(q, k, v, causal)
     rel = ((out.double() - exact).norm() / exact.norm()).item()
     # Rounding the result to fp16 alone is 2^-11 / sqrt(3) times the mean spread of a mantissa, 2.05e-4. The row's main
     # term must add nothing (its probability is held exactly); the other terms' rounded probabilities add about 2.0e-4
     # times their share of the result's norm, at most a half here. Held against a reference far below, the main term
     # alone would add another 2.0e-4 (2.9e-4 in all).
     assert rel <= 2.3e-4, rel
+
+
+# Rounding the result to fp16 is 2.05e-4 (2-norm, relative; see above), and a row's probabilities rounded to fp16 add at
+# most as much again, independently of it: 2.9e-4; a tenth on top for the spread between inputs.
+ROUNDING = 3.2e-4
+
+
+# Scores that rise or fall by `step` powers of two from one kv tile to the next: falling ones give the walk, which starts
+# at the last tile, a new row max on every tile, by less than the threshold of a move (2^8), by just more and by far
+# more. (2, 1100): items whose stages take the kv tiles of one q tile in turn; (40, 1100): pairs.
+@pytest.mark.parametrize("H,N", [(2, 1100), (40, 1100)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("step", [-40.0, -8.5, -7.5, -3.0, 8.5])
+def test_row_max_moving_along_the_walk(pkg, H, N, d, causal, step):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(int(10 * step) + 1000 + d)
+    q, k, v = (torch.randn((1, H, N, d), generator=g, device="cuda") for _ in range(3))
+    tile = (torch.arange(N, device="cuda") // 128).float()
+    q[..., 0] = 4.0
+    k[..., 0] = step * np.log(2.0) * d ** 0.5 / 4.0 * tile
+    q, k, v = q.half(), k.half(), v.half()
+    out, lse = pkg.attention_forward(q, k, v, causal=causal, return_lse=True)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    exact, exact_lse = exact_attention_gpu(q, k, v, causal)
+    assert ((out.double() - exact).norm() / exact.norm()).item() <= ROUNDING
+    assert (lse.double() - exact_lse).abs().max().item() <= 5e-4
+
+
+# Slopes of either sign (and none): tiles left and right of the diagonal take the bias as a linear function of the column
+# whose direction depends on both, tiles on the diagonal take the absolute distance.
+@pytest.mark.parametrize("H,N", [(5, 1000), (45, 700)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_alibi_slopes_of_either_sign(pkg, H, N, d, causal):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(N + d)
+    q, k, v = (torch.randn((1, H, N, d), generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+    some = [0.5, 2.0 ** -4, 0.0, -(2.0 ** -4), -0.5]
+    slopes = torch.tensor([some[h % 5] for h in range(H)], device="cuda")
+    out, lse = pkg.attention_forward(q, k, v, causal=causal, alibi_slopes=slopes, return_lse=True)
+    plain = pkg.attention_forward(q, k, v, causal=causal, alibi_slopes=slopes)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    exact, exact_lse = exact_attention_gpu(q, k, v, causal, slopes)
+    for h in range(5):
+        assert ((out - exact)[:, h::5].norm() / exact[:, h::5].norm()).item() <= ROUNDING, some[h]
+    # a bias of up to 720 (in powers of two) is rounded to fp32 twice and added once: 3 * 2^-15 powers of two
+    assert (lse.double() - exact_lse).abs().max().item() <= 5e-4
+    assert torch.equal(out, plain)
 
 
 def test_deterministic_and_kernels_agree(pkg, ob):

@@ -57,7 +57,7 @@ SHAPES = [
     dict(bh=5, n=1000, wl=100, wr=5), dict(bh=8, n=2304 + 77, causal=True),
     dict(bh=40, n=4097, causal=True), dict(bh=7, n=700, wl=50), dict(bh=96, n=1000),
     # window, last pairs split; causal with several head groups; causal, all pairs split; slabs of such problems
-    dict(bh=152, n=1000, d=128, wl=100, wr=0), dict(bh=64, n=32768 // 8 + 5, d=128, causal=True), dict(bh=8, n=4096, causal=True),
+    dict(bh=152, n=1000, d=128, wl=100, wr=0), dict(bh=64, n=4101, d=128, causal=True), dict(bh=8, n=4096, causal=True),
     dict(bh=5, n=512, first=70, total=75), dict(bh=5, n=2048, causal=True, first=0, total=40),
 ]
 
@@ -98,7 +98,8 @@ def test_every_q_tile_once_with_its_kv_tiles(wi, pkg, shape):
 
 @pytest.mark.parametrize("shape", [
     dict(n=512, total=75), dict(n=333, total=75), dict(n=2048, total=40, causal=True), dict(n=4096, total=9, causal=True),
-    dict(n=8192, total=32, d=128, causal=True), dict(n=1000, total=152, wl=100, wr=0), dict(n=4096, total=10, causal=True, wl=500),
+    dict(n=8192, total=32, d=128, causal=True), dict(n=1000, total=152, wl=100, wr=0),
+    dict(n=4096, total=10, causal=True, wl=500),
     dict(n=900, total=41, wl=60), dict(n=4096, total=30),
 ], ids=str)
 def test_slabs_take_the_same_pairs_apart(wi, shape):
