@@ -322,9 +322,9 @@ int host_pipe(HostPipe** out) {
 // A launch finds its pair at zero and leaves it at zero. A caller that lets two launches on one slot overlap, which is
 // not allowed, may leave a pair off, and a launch that started from such a pair would skip work without knowing. So the
 // launches of a slot take its pairs in turn and each, as it ends, also clears the pair of the next: whatever two
-// overlapping launches did to theirs, the third starts from zero. A launch captured into a graph keeps its pair for every replay, so there a
-// memset node goes in front of it. (A memset in front of every launch cost 2 us a call and kept the kernel from
-// overlapping its predecessor.)
+// overlapping launches did to theirs, the third starts from zero. A launch captured into a graph keeps its pair for
+// every replay, so there a memset node goes in front of it. (A memset in front of every launch cost 2 us a call and kept
+// the kernel from overlapping its predecessor.)
 constexpr int kNoAllocSlots = 16, kSlotWords = 8, kSlotPairs = 3;
 static __device__ __align__(256) int g_noalloc_scratch[kNoAllocSlots * kSlotWords];
 

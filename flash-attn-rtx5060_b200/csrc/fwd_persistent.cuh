@@ -1,11 +1,13 @@
 // Warp-specialised persistent attention-forward kernel for sm_100a.
 //
-// One CTA per SM walks a list of work items; a work item is a pair of adjacent 128-row q tiles
-// of one (batch, head). Roles (16 warps):
-//   warps 0-3   softmax of q tile 0: one thread per score row (TMEM lane), exp2 online softmax
-//   warps 4-7   softmax of q tile 1
+// One CTA per SM walks a list of work items (work_items.h); a work item is a pair of adjacent 128-row q tiles of one
+// (batch, head), one for each of the two stages, or a single q tile whose kv tiles the stages take in turn. The kv
+// tiles are walked from the last visible one to the first. Roles (16 warps):
+//   warps 0-3   softmax of stage 0: one thread per score row (TMEM lane), exp2 online softmax
+//   warps 4-7   softmax of stage 1
 //   warps 8-11  correction: rescales the running output in TMEM when a row max moved, and the
-//               epilogue (O / l -> fp16 -> the warp's staging area in shared memory -> one TMA store)
+//               epilogue (O / l, or for a single q tile the sum of both stages' O over the sum of their l, -> fp16 ->
+//               the warp's staging area in shared memory -> one TMA store)
 //   warp 12     tensor-core issuer: the warp walks the schedule, one elected lane issues tcgen05.mma
 //   warp 13     TMA producer: Q tiles and the K/V tile ring
 //   warps 14-15 idle (they only donate registers)
@@ -15,7 +17,7 @@
 //
 // Replaces the reference's forward_kernel, Schedule and SMem (src/flash_forward.h:22-366),
 // apply_mask (src/mask.h:10-84) and apply_softmax (src/softmax.h:9-86): same function, but
-// the contractions run on tcgen05 with TMEM accumulators, the two q tiles ping-pong so that
+// the contractions run on tcgen05 with TMEM accumulators, the two stages ping-pong so that
 // the tensor pipe works on one while the other is in softmax, masks touch only boundary
 // tiles, kv tiles outside a q tile's visible range are never loaded for it, and the output
 // is rescaled lazily.
@@ -377,7 +379,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           // The reference moves when the tile's max has grown past it (see kLazyLog2), and always on the first tile that
           // shows a finite score: the reference then IS the row max, so the largest term of the row is exactly 1 in
           // fp16 (a row with a single visible key returns that key's V bit for bit). A cut tile over the first keys is
-          // the only tile of its walk (or, with ALiBi, may be the last).
+          // the only tile of its walk (with ALiBi it may be the last), or the far edge of a left window lies in it.
           const bool fresh = l_run == 0.f;
           const bool first_keys = (!kMasked || kAlibi) && kv0 == 0;
           float alpha = 1.f;

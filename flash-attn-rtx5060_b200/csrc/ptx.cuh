@@ -128,9 +128,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 #endif
 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  // The first probe stands alone and the retry loop holds nothing but the probe and a counter: what sits between
-  // two probes is added to every hand-off in the kernels (a loop that also read the abort flag after each probe
-  // cost 5 % of the whole attention kernel). Written as one block of PTX, a wait is 11 instructions in each of its
+  // Between two probes stand a counter and its test; the abort flag is read after every 64th only: what sits there is
+  // added to every hand-off in the kernels (a loop that read the flag after each probe cost 5 % of the whole attention
+  // kernel). Written as one block of PTX, a wait is 11 instructions in each of its
   // many places; as C++ around single probes it came to 40, 27 KB of the kernel, and the first and last rounds of an
   // item, whose code is rarely in the instruction caches, ran slower: B4 H16 N2048 d64 causal 72.0 -> 67.8 us, B8 H12
   // N1000 d64 54.5 -> 51.6, B8 H16 N1024 d128 61.5 -> 58.2.

@@ -16,8 +16,8 @@ __host__ __device__ inline int min_int(int a, int b) { return a < b ? a : b; }
 
 // Heads per scheduling group of the persistent kernel. Without a mask all items cost the same and head-major
 // order (1) shares K/V best. With a causal mask or a window the item costs differ, and interleaving the heads of
-// a group pair-major makes the order of the group longest first. Measured constraints (B200): the K and V rows that a
-// group keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
+// a group pair-major makes the order of the group longest first (causal masks). Measured constraints (B200): the K and V
+// rows that a group keeps live (the whole head, or the window span) should stay within ~64 MB (the 126 MB L2 holds two copies of
 // what both dies read: the long-context workload read K/V from DRAM 2.2 times with 96 MB in flight, 1.5 times
 // with 64 MB, 1.1 times with 48 MB, at the same speed; the 8192-row config is 0.6 % faster with 64 MB than
 // with 48); a group needs about two items per CTA to balance; and the groups must be of even size (64 heads in
@@ -52,8 +52,9 @@ inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
 // - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
 //   one wave. B2 H16 N4096 d128: 3.46 waves of 32 steps, 277 -> 255 us; 8 heads of 333 rows: 14.3 -> 12.6 us.
 // - Under a causal mask items are handed out longest first and a partial wave costs little; but with few of them the
-//   longest one sets the time. All are split while a CTA has less than about 7/4 items, or, where sequences are
-//   short and the fill and drain of an item weigh more, less than a seventh of a head's pairs (d64 us, pairs against
+//   longest one sets the time. All are split while a CTA has at most half an item, or at most 7/4 items that are also
+//   at most a seventh of a head's pairs (where sequences are short, the fill and drain of an item weigh more). The same
+//   rule serves a window bounded on one side without a causal mask, whose items differ likewise. (d64 us, pairs against
 //   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
 //   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
 //   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
@@ -66,10 +67,8 @@ inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, in
     const long long tail = pairs % num_sms;
     return 2 * tail <= num_sms ? tail : 0;
   }
-  if (2 * pairs <= num_sms || 4 * pairs <= 7LL * num_sms) {
-    if (2 * pairs <= num_sms || 7 * pairs <= (long long)num_q_pairs * num_sms) return pairs;
-  }
-  return 0;
+  const bool few = 4 * pairs <= 7LL * num_sms && 7 * pairs <= (long long)num_q_pairs * num_sms;
+  return few || 2 * pairs <= num_sms ? pairs : 0;
 }
 
 // The items of a launch on p->bh heads, the first of which is head `first_head` of a problem of `total_heads`: its order
@@ -114,8 +113,9 @@ struct ItemGeom {
 // Work-item order. Heads are taken in groups of `head_group` (sized on the host so that the K/V of
 // a group stays in L2); inside a group the items run pair-major from the last (under a causal mask
 // the longest) q pair to the first. CTAs claim items in this order from a global counter, so CTAs
-// that run together read the same few heads, and the items handed out last are the cheapest ones
-// of the last group: the tail stays short.
+// that run together read the same few heads, and under a causal mask the items handed out last are the
+// cheapest ones of the last group: the tail stays short. (With a window bounded on the left only and no causal mask
+// the first pairs are the longest, and come last.)
 template <int BN = kBlockN>
 __host__ __device__ inline ItemGeom decode_item(int item, const FwdParams& p) {
   ItemGeom g;
