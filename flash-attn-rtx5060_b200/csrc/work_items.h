@@ -57,7 +57,9 @@ inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
 //   rule serves a window bounded on one side without a causal mask, whose items differ likewise. (d64 us, pairs against
 //   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
 //   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
-//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %).
+//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %). Singles over
+//   pairs with ALiBi, log-sum-exp and dropout, where the rule splits: 0.75-0.95, 0.79-1.01, 0.76-1.03 (20x1024 to
+//   4x16384, both head dims; the largest at d128 16x4096), and at d64 30x1024, where it does not, 1.11, 1.05, 1.10.
 inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, int window_left, int window_right,
                                 int num_sms) {
   if (seqlen <= kBlockM || pairs >= (1 << 30)) return 0;
@@ -75,20 +77,34 @@ inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, in
 // (head_group), and how many pairs at the end of that order are taken apart. A split q tile is summed in another order
 // than a pair's, so which pairs are split is decided for the whole problem: the chunks of flash_forward_host and the slabs
 // of flash_forward_multi_gpu give the bits of the call on all heads. Where only the last pairs of the problem are
-// split, the order is head-major, in which the last pairs of a chunk or slab are the problem's if it holds any of them.
+// split, they must be the last ones of the slab's order as well, if it holds any of them. That is so in head-major order
+// and where all heads form one group; with several groups (windows over so many heads that K and V pass L2, hence with
+// many waves of items) nothing is split. (Head-major order for windows whose last pairs are split would serve too, but
+// runs up to 17 % slower: 40 heads x 4096 rows d128, window 512 75 -> 84 us, 256 x 1500 d64, window 128 71 -> 83.)
 inline void set_work_items(FwdParams* p, int head_dim, int num_sms, long long first_head, long long total_heads) {
-  const int wl = p->window_left, wr = eff_window_right(p->causal, p->window_right);
-  const long long all = total_heads * p->num_q_pairs;
-  const long long split = pairs_to_split(all, p->num_q_pairs, p->seqlen, wl, wr, num_sms);
-  const int pairs = p->bh * p->num_q_pairs;
-  p->head_group = (split > 0 && split < all)
-                      ? 1
-                      : pick_head_group(p->bh, p->seqlen, head_dim, p->causal, p->window_left, p->window_right,
-                                        p->num_q_pairs, num_sms);
-  long long mine = (first_head + p->bh) * p->num_q_pairs - (all - split);
-  mine = mine < 0 ? 0 : (mine > pairs ? pairs : mine);
-  p->num_pair_items = pairs - static_cast<int>(mine);
-  p->num_items = pairs + static_cast<int>(mine);
+  const int wl = p->window_left, wr = eff_window_right(p->causal, p->window_right), nq = p->num_q_pairs;
+  auto group = [&](long long heads) {
+    const int bh = heads > 0x7fffffff ? 0x7fffffff : static_cast<int>(heads);
+    return pick_head_group(bh, p->seqlen, head_dim, p->causal, p->window_left, p->window_right, nq, num_sms);
+  };
+  const long long all = total_heads * nq, last = first_head + p->bh;
+  const int pairs = p->bh * nq, group_all = group(total_heads);
+  p->head_group = group(p->bh);
+  long long split = pairs_to_split(all, nq, p->seqlen, wl, wr, num_sms);
+  if (split > 0 && split < all && group_all > 1) {
+    if (group_all < total_heads) {
+      split = 0;
+    } else {  // one group: pairs in the order (pair, head), the first split one is `head` of pair `pr`
+      const long long pr = (all - split) / total_heads, head = (all - split) % total_heads;
+      split = (nq - 1 - pr) * p->bh;
+      if (last > head) split += last - (first_head > head ? first_head : head);
+    }
+  } else {  // head-major, or all or none of the pairs
+    split = last * nq - (all - split);
+    split = split < 0 ? 0 : (split > pairs ? pairs : split);
+  }
+  p->num_pair_items = pairs - static_cast<int>(split);
+  p->num_items = pairs + static_cast<int>(split);
 }
 
 // Work item -> geometry. Every role decodes the same item the same way.

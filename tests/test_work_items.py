@@ -100,7 +100,8 @@ def test_every_q_tile_once_with_its_kv_tiles(wi, pkg, shape):
     dict(n=512, total=75), dict(n=333, total=75), dict(n=2048, total=40, causal=True), dict(n=4096, total=9, causal=True),
     dict(n=8192, total=32, d=128, causal=True), dict(n=1000, total=152, wl=100, wr=0),
     dict(n=4096, total=10, causal=True, wl=500),
-    dict(n=900, total=41, wl=60), dict(n=4096, total=30),
+    dict(n=900, total=41, wl=60), dict(n=4096, total=30), dict(n=4096, total=40, d=128, causal=True, wl=512),
+    dict(n=2048, total=223, d=128, causal=True, wl=500), dict(n=1500, total=7, wl=128, wr=128),
 ], ids=str)
 def test_slabs_take_the_same_pairs_apart(wi, shape):
     """Whether a q tile is summed by one stage or by two does not depend on how the heads are cut into calls that know the
