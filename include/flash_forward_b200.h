@@ -49,6 +49,10 @@ enum {
  * same heads. The split of the work among the SMs depends on batch*heads, so a head may differ in the last place
  * between a call on all heads and a separate call on some of them.
  *
+ * Early start: a launch may take up SMs a few microseconds before the kernel in front of it in the stream has ended
+ * (programmatic stream serialization); it touches no global memory before that kernel is complete. Launches captured
+ * into a graph (flash_forward_noalloc) do not, so the graph's edges are plain ones.
+ *
  * Launches in flight: every launch uses a pair of scheduler words (2.5 KB of device scratch,
  * allocated on the first call per device). The first 256 streams that are used on a device own a pair each,
  * until flash_forward_shutdown() (launches on one stream are ordered anyway); launches on further streams take 64
