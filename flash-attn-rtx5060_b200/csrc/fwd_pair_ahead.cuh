@@ -360,9 +360,9 @@ fwd_pair_ahead_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           uint64_t lsum_a = 0ull, lsum_b = 0ull;
           uint32_t pk0[32], pk1[32];
           // masked tiles hold -inf scores, which only the MUFU path maps to 0
-          exp_half_tile(sc, scale2, negms2, pk0, lsum_a, lsum_b);
+          exp_tile<32, 0>(sc, scale2, negms2, pk0, lsum_a, lsum_b);
           tmem_st32(tP + 0, pk0);
-          exp_half_tile(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
+          exp_tile<32, 0>(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
           __syncwarp();
           if (lane == 0) mbar_arrive(e_mine);
           float l0, l1;

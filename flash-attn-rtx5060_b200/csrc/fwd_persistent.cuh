@@ -5,15 +5,26 @@
 // tiles are walked from the last visible one to the first. Roles (16 warps):
 //   warps 0-3   softmax of stage 0: one thread per score row (TMEM lane), exp2 online softmax
 //   warps 4-7   softmax of stage 1
-//   warps 8-11  correction: rescales the running output in TMEM when a row max moved, and the
-//               epilogue (O / l, or for a single q tile the sum of both stages' O over the sum of their l, -> fp16 ->
+//   warps 8-11  epilogue (O / l, or for a single q tile the sum of both stages' O over the sum of their l, -> fp16 ->
 //               the warp's staging area in shared memory -> one TMA store)
 //   warp 12     tensor-core issuer: the warp walks the schedule, one elected lane issues tcgen05.mma
 //   warp 13     TMA producer: Q tiles and the K/V tile ring
 //   warps 14-15 idle (they only donate registers)
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D); the fp16 P tile of a
 // stage overwrites the first 64 columns of its own S and is handed to the tensor pipe in two
-// halves of 64 keys, so that P.V starts while the second half is still being exponentiated.
+// parts of 96 and 32 keys, so that most of P.V runs while the last keys are still being exponentiated and little of it
+// stands between the last of P and the stage's next score tile.
+//
+// What sets the pace of a long sequence is the loop of one stage, softmax tile -> rest of P.V -> next score tile ->
+// softmax, together with the issue slots of the four SM sub-partitions, each of which runs one softmax warp of either
+// stage. Shortening the issuer alone or the softmax alone gained nothing or lost: a faster issuer only made the two
+// stages' tiles overlap more. Done together (B200, us): the issuer's products in branch-free groups (umma_pv64 and the
+// like) without a vote behind each wait; O rescaled by the softmax warps themselves, which took a hand-over per tile to
+// the warps 8-11 off the path; a fifth of the exponentials on the FMA pipe (exp2_poly); what is fixed for an item
+// computed once per item. B2 H32 N8192 d128 causal 1085 -> 971, B2 H16 N4096 d128 268 -> 237, B4 H16 N16384 d128 window
+// 1024 690 -> 613, 24 heads x 4001 rows d128 with log-sum-exp 120 -> 109, 32 heads x 8192 rows d64 761 -> 675, B8 H12
+// N1000 d64 50.0 -> 47.4, B4 H16 N2048 d64 causal 66.5 -> 62.8, with dropout 97.2 -> 94.5, ALiBi B2 H16 N4096 d64 128.9
+// -> 121.0. Of a round of two tiles at head_dim 128, 2725 clocks of 3050 before, 2370 remain without any products.
 //
 // Replaces the reference's forward_kernel, Schedule and SMem (src/flash_forward.h:22-366),
 // apply_mask (src/mask.h:10-84) and apply_softmax (src/softmax.h:9-86): same function, but
@@ -28,15 +39,6 @@
 #include "ptx.cuh"
 #include "work_items.h"
 
-// Registers per thread after setmaxnreg: 8 softmax warps, 4 correction warps, 4 others; the three
-// numbers must satisfy 256 * softmax + 128 * correction + 128 * others <= 65536.
-#ifndef FA_REG_SOFTMAX
-#define FA_REG_SOFTMAX 184
-#define FA_REG_CORR 72
-#define FA_REG_MISC 72
-#endif
-
-
 
 namespace fa {
 
@@ -48,11 +50,11 @@ struct PersistentCfg {
   static constexpr int kStages = (D == 128) ? 4 : 8;  // ring slots, each one K or one V tile
   static constexpr int kOffQ = 0;
   static constexpr int kOffKV = 2 * kTileBytes;
-  // Output staging: each correction warp owns 32 rows, laid out [panel][row][64] with the 128-byte swizzle, the
+  // Output staging: each epilogue warp owns 32 rows, laid out [panel][row][64] with the 128-byte swizzle, the
   // source of its TMA store.
   static constexpr int kOffOut = kOffKV + kStages * kTileBytes;
   static constexpr int kOutWarpBytes = 32 * D * 2;
-  static constexpr int kOffAlpha = kOffOut + 4 * kOutWarpBytes;  // float[2][128]
+  static constexpr int kOffAlpha = kOffOut + 4 * kOutWarpBytes;  // float[2][128]: references of a split item; drop_blocks
   static constexpr int kOffRowSum = kOffAlpha + 2 * kBlockM * 4;   // float[2][128]
   static constexpr int kOffBars = kOffRowSum + 2 * kBlockM * 4;
   static constexpr int kNumBars = 20 + 2 * kStages;
@@ -75,33 +77,57 @@ struct PersistentCfg {
   // 24 heads x 4001 rows d128 causal, log-sum-exp, spread 2 115.9 -> 116.7, B2 H32 N8192 d128 causal 1041 -> 1045 (the
   // running max as such is no longer kept; with ALiBi the register it took matters more: B2 H16 N4096 d64 131.8 -> 128.7).
   static constexpr float kLazyLog2 = 8.f;
+  // One pair of exponentials in kPolyOf is taken on the FMA pipe (keys 32-63, 64-95, 96-127 of a tile that is not cut; the
+  // first 32 keys share their time with the row max). A softmax tile alone takes 1336 clocks, two at once on a
+  // sub-partition 2275; with one pair in four 1243 and 2063. Nearly all at once the special-function unit is no longer the
+  // limit, so more does not help: against these fractions (us; B2 H32 N8192 d128 causal, 32 heads x 8192 rows d64, B8 H12
+  // N1000 d64: 969, 672, 47.2), half as many 972, 692, 48.4; twice as many in the second part of d128 1061; in the last
+  // part 1059, 705, 48.4; one pair in four of the first 32 keys too 991, 745, 51.0. None with dropout, whose mask fills
+  // the same pipes (103 -> 101).
+  static constexpr int kPolyOf1 = D == 64 ? 2 : 4, kPolyOf2 = 4, kPolyOf3 = 4;
+  // Registers per thread after setmaxnreg: 8 softmax warps, 4 epilogue warps, 4 others; 256 * softmax + 128 * epilogue +
+  // 128 * others <= 65536. At head_dim 64, where the exponentials are the limit, 200 let more of them be in flight (32
+  // heads x 8192 rows 719 -> 680 us); at head_dim 128 it costs 2-4 %.
+  static constexpr int kRegSoftmax = D == 64 ? 200 : 184, kRegEpilogue = D == 64 ? 40 : 72, kRegOthers = 72;
 };
 
-// exp2 of 64 scores (32 pairs) -> 32 packed fp16x2 words; adds the exponentials into two
-// (even, odd) pairs of partial row sums.
-__device__ __forceinline__ void exp_half_tile(const float* sc, uint64_t scale2, uint64_t negms2, uint32_t (&pk)[32],
-                                              uint64_t& lsum_a, uint64_t& lsum_b) {
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    float x0, x1, e0, e1;
-    f2_unpack(f2_fma(f2_pack(sc[2 * c], sc[2 * c + 1]), scale2, negms2), x0, x1);
-    e0 = ex2_approx(x0);
-    e1 = ex2_approx(x1);
-    if (c & 1) lsum_b = f2_add(lsum_b, f2_pack(e0, e1));
-    else lsum_a = f2_add(lsum_a, f2_pack(e0, e1));
-    pk[c] = pack_f16x2(e0, e1);
-  }
+// 2^x of two values on the FMA pipe: x = n + f with n the nearest integer (the usual addition of 1.5 * 2^23 rounds x to
+// one), 2^f a polynomial, 2^n by way of the exponent field. The polynomial is the minimax approximation of 2^f in
+// relative error on [-1/2, 1/2] among those of degree 5 with constant term 1 (Remez exchange): 1.6e-7 in fp32
+// arithmetic, where ex2.approx states 2.4e-7. 2^0 is exactly 1; below 2^-126.5, down to -infinity, the result is 0; NaN
+// stays NaN (a product, not an addition to the exponent field, and a maximum that keeps it).
+__device__ __forceinline__ void exp2_poly(float x0, float x1, float& e0, float& e1) {
+  const uint64_t x = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
+  const uint64_t magic = f2_pack(12582912.f, 12582912.f);
+  const uint64_t t = f2_add(x, magic);
+  const uint64_t f = f2_add(x, f2_fma(t, f2_pack(-1.f, -1.f), magic));
+  uint64_t p = f2_fma(f2_pack(0x1.5bba14p-10f, 0x1.5bba14p-10f), f, f2_pack(0x1.3cea88p-7f, 0x1.3cea88p-7f));
+  p = f2_fma(p, f, f2_pack(0x1.c6b752p-5f, 0x1.c6b752p-5f));
+  p = f2_fma(p, f, f2_pack(0x1.ebf9bcp-3f, 0x1.ebf9bcp-3f));
+  p = f2_fma(p, f, f2_pack(0x1.62e42ap-1f, 0x1.62e42ap-1f));
+  p = f2_fma(p, f, f2_pack(1.f, 1.f));
+  float t0, t1;
+  f2_unpack(t, t0, t1);
+  const float s0 = __uint_as_float((__float_as_uint(t0) << 23) + 0x3f800000u);
+  const float s1 = __uint_as_float((__float_as_uint(t1) << 23) + 0x3f800000u);
+  f2_unpack(f2_mul(p, f2_pack(s0, s1)), e0, e1);
 }
 
-// Same for 32 scores (16 pairs) -> the first 16 words of pk.
-__device__ __forceinline__ void exp_quarter_tile(const float* sc, uint64_t scale2, uint64_t negms2, uint32_t* pk,
-                                                 uint64_t& lsum_a, uint64_t& lsum_b) {
+// exp2 of 2 * kPairs scores -> packed fp16x2 words; adds the exponentials into two (even, odd) pairs of partial row sums.
+// Of every kPolyOf pairs one takes exp2_poly instead of the special-function unit (0: none).
+template <int kPairs, int kPolyOf>
+__device__ __forceinline__ void exp_tile(const float* sc, uint64_t scale2, uint64_t negms2, uint32_t* pk, uint64_t& lsum_a,
+                                         uint64_t& lsum_b) {
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
+  for (int c = 0; c < kPairs; ++c) {
     float x0, x1, e0, e1;
     f2_unpack(f2_fma(f2_pack(sc[2 * c], sc[2 * c + 1]), scale2, negms2), x0, x1);
-    e0 = ex2_approx(x0);
-    e1 = ex2_approx(x1);
+    if (kPolyOf > 0 && c % (kPolyOf > 0 ? kPolyOf : 1) == 1) {
+      exp2_poly(x0, x1, e0, e1);
+    } else {
+      e0 = ex2_approx(x0);
+      e1 = ex2_approx(x1);
+    }
     if (c & 1) lsum_b = f2_add(lsum_b, f2_pack(e0, e1));
     else lsum_a = f2_add(lsum_a, f2_pack(e0, e1));
     pk[c] = pack_f16x2(e0, e1);
@@ -113,44 +139,52 @@ __device__ __forceinline__ void exp_quarter_tile(const float* sc, uint64_t scale
 // whatever tile shape or schedule computes it. (The reference keeps ONE generator state per q tile, copies it into
 // every thread of the CTA, so all threads draw the same numbers, and stores it back: src/flash_forward.h:185-186,
 // :248-265, :361-363. That flaw is not reproduced.)
-__device__ __forceinline__ void philox4x32_10(uint32_t k0, uint32_t k1, uint32_t c0, uint32_t c1, uint32_t c2,
-                                              uint32_t c3, uint32_t (&out)[4]) {
+// The counter is {column block, row, head, 0}, so what the first rounds multiply depends on the row alone or on the block
+// alone: DropRow holds the row's part, DropBlock the block's, which 8 lanes of a warp compute for the 8 blocks of a tile
+// (they are the same for all rows) and leave in shared memory. Of a block's 20 wide products 15 remain per row.
+constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u, kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
+struct DropRow { uint32_t hi, lo; };  // second round: product of the row's word
+__device__ __forceinline__ DropRow drop_row(const FwdParams& p, int bh, int row) {
+  const uint32_t c0 = __umulhi(kPhiloxM1, bh) ^ static_cast<uint32_t>(row) ^ p.seed_lo;
+  return {__umulhi(kPhiloxM0, c0), kPhiloxM0 * c0};
+}
+// Words of the third round that the block alone decides, keys included: {c2, c0, c2 of the next round, c3}
+__device__ __forceinline__ uint4 drop_block(const FwdParams& p, int bh, uint32_t block) {
+  const uint32_t c2 = __umulhi(kPhiloxM0, block) ^ p.seed_hi;
+  const uint32_t c0 = __umulhi(kPhiloxM1, c2) ^ (kPhiloxM1 * static_cast<uint32_t>(bh)) ^ (p.seed_lo + kPhiloxW0);
+  return make_uint4((kPhiloxM0 * block) ^ (p.seed_hi + kPhiloxW1), (kPhiloxM1 * c2) ^ (p.seed_lo + 2u * kPhiloxW0),
+                    __umulhi(kPhiloxM0, c0) ^ (p.seed_hi + 2u * kPhiloxW1), kPhiloxM0 * c0);
+}
+__device__ __forceinline__ void drop_words(const FwdParams& p, const DropRow& row, const uint4& blk, uint32_t (&out)[4]) {
+  uint32_t c2 = row.hi ^ blk.x;
+  uint32_t c0 = __umulhi(kPhiloxM1, c2) ^ blk.y, c1 = kPhiloxM1 * c2, c3 = blk.w;
+  c2 = row.lo ^ blk.z;
 #pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-    c0 = hi1 ^ c1 ^ k0;
+  for (uint32_t r = 3; r < 10; ++r) {
+    const uint32_t hi0 = __umulhi(kPhiloxM0, c0), lo0 = kPhiloxM0 * c0;
+    const uint32_t hi1 = __umulhi(kPhiloxM1, c2), lo1 = kPhiloxM1 * c2;
+    c0 = hi1 ^ c1 ^ (p.seed_lo + r * kPhiloxW0);
     c1 = lo1;
-    c2 = hi0 ^ c3 ^ k1;
+    c2 = hi0 ^ c3 ^ (p.seed_hi + r * kPhiloxW1);
     c3 = lo0;
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
   }
   out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
 }
 
-// Zeroes the dropped elements of 32 packed fp16 pairs (64 consecutive columns starting at global column `col0`, a
-// multiple of 16) of query row `row` of head `bh`. One Philox call serves 16 columns: byte t of its 16 output bytes
-// (little endian over the four words) decides column 16 * block + t.
-__device__ __forceinline__ void dropout_mask_64(uint32_t (&pk)[32], const FwdParams& p, int bh, int row, int col0) {
-  constexpr uint32_t kHigh = 0x80808080u;
-  const uint32_t thr4 = p.drop_keep_thr * 0x01010101u;
+// Zeroes the dropped elements of kBlocks * 8 packed fp16 pairs (16 columns per block). Byte t of a block's 16 random bytes
+// (little endian over the four words) decides column t: kept when below the threshold. Two bytes at a time are compared
+// as the fp16 values 1024 + byte, which are exact, and the comparison leaves a mask over the pair.
+template <int kBlocks>
+__device__ __forceinline__ void dropout_mask(uint32_t* pk, const FwdParams& p, const DropRow& row, const uint4* blocks) {
+  const uint32_t limit = 0x64006400u + p.drop_keep_thr * 0x00010001u;
 #pragma unroll
-  for (int blk = 0; blk < 4; ++blk) {
+  for (int blk = 0; blk < kBlocks; ++blk) {
     uint32_t r[4];
-    philox4x32_10(p.seed_lo, p.seed_hi, static_cast<uint32_t>(col0 / 16 + blk), static_cast<uint32_t>(row),
-                  static_cast<uint32_t>(bh), 0u, r);
+    drop_words(p, row, blocks[blk], r);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      // High bit of each byte of `ge`: the byte is not below the threshold (a subtraction that borrows within bytes).
-      // A byte permute with the sign-replicating selectors 8 + b spreads these bits over the halves of two words.
-      const uint32_t diff = (r[w] | kHigh) - (thr4 & ~kHigh);
-      const uint32_t ge = (r[w] & ~thr4) | (~(r[w] ^ thr4) & diff);
-      uint32_t lo, hi;
-      asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(lo) : "r"(ge));
-      asm("prmt.b32 %0, %1, 0, 0xBBAA;" : "=r"(hi) : "r"(ge));
-      pk[blk * 8 + 2 * w] &= ~lo;      // columns 4w, 4w+1
-      pk[blk * 8 + 2 * w + 1] &= ~hi;  // columns 4w+2, 4w+3
+      pk[blk * 8 + 2 * w] &= f16x2_less_mask(__byte_perm(r[w], 0x64646464u, 0x4140), limit);      // columns 4w, 4w+1
+      pk[blk * 8 + 2 * w + 1] &= f16x2_less_mask(__byte_perm(r[w], 0x64646464u, 0x4342), limit);  // columns 4w+2, 4w+3
     }
   }
 }
@@ -164,7 +198,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   extern __shared__ __align__(1024) uint8_t smem[];
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
 
   if ((smem_u32(smem) & 1023u) != 0) {  // swizzled tiles need a 1024-byte aligned base
@@ -180,11 +214,11 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   uint64_t* q_full = bars;            // [2] TMA -> MMA
   uint64_t* q_empty = bars + 2;       // [2] MMA -> TMA
   uint64_t* s_full = bars + 4;        // [2] MMA -> softmax: S tile in TMEM
-  uint64_t* p_full = bars + 6;        // [2] softmax (first half of P) + correction (O rescaled) -> MMA
-  uint64_t* alpha_ready = bars + 8;   // [2] softmax -> correction: rescale factors in smem
-  uint64_t* l_ready = bars + 10;      // [2] softmax -> correction: final row sums in smem
-  uint64_t* o_full = bars + 12;       // [2] MMA -> correction: last P.V of the item landed
-  uint64_t* p_full2 = bars + 14;      // [2] softmax -> MMA: second half of P written
+  uint64_t* p_full = bars + 6;        // [2] softmax -> MMA: P of the first 96 keys written, O rescaled
+  uint64_t* o_empty = bars + 8;       // [2] epilogue -> MMA, softmax: O and the row sums of the item have been read
+  uint64_t* l_ready = bars + 10;      // [2] softmax -> epilogue: final row sums in smem
+  uint64_t* o_full = bars + 12;       // [2] MMA -> epilogue: last P.V of the item landed
+  uint64_t* p_full2 = bars + 14;      // [2] softmax -> MMA: rest of P written
   uint64_t* item_full = bars + 16;    // [2] producer -> all roles: next work item id published
   uint64_t* item_empty = bars + 18;   // [2] all roles -> producer: id slot read
   uint64_t* kv_full = bars + 20;      // [kStages] TMA -> MMA
@@ -193,7 +227,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   // [2][16]: ItemGeom of the published item in words 0..11, its id (-1: no more items) in word 12, `split` in word 13
   volatile int* s_geom = reinterpret_cast<volatile int*>(smem + Cfg::kOffGeom);
-  constexpr uint32_t kItemReaders = 13;  // 8 softmax warps + 4 correction warps + the MMA warp
+  constexpr uint32_t kItemReaders = 13;  // 8 softmax warps + 4 epilogue warps + the MMA warp
 
   if (warp == 12) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -205,9 +239,9 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       mbar_init(&q_full[s], 1);
       mbar_init(&q_empty[s], 1);
       mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 8);  // one arrival per softmax warp and per correction warp
+      mbar_init(&p_full[s], 4);
       mbar_init(&p_full2[s], 4);
-      mbar_init(&alpha_ready[s], 4);
+      mbar_init(&o_empty[s], 4);
       mbar_init(&l_ready[s], 4);
       mbar_init(&o_full[s], 1);
       mbar_init(&item_full[s], 1);
@@ -259,7 +293,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // =====================================================================================
     // softmax: stage s = warp / 4, row = tid % 128
     // =====================================================================================
-    reg_inc<FA_REG_SOFTMAX>();
+    reg_inc<Cfg::kRegSoftmax>();
     const int s = warp >> 2;
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
@@ -268,8 +302,13 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // everything downstream works with a unit scale.
     const float sl2 = kAlibi ? 1.f : p.scale_log2;
     const uint64_t scale2 = f2_pack(sl2, sl2);
-    uint32_t n_s = 0;  // completed s_full phases
+    const uint32_t tO = tmem_addr(tmem_base, lane_base, s == 0 ? Cfg::kColO0 : Cfg::kColO1);
+    uint32_t par_s = 0;  // parity of the next s_full phase
+    const float lazy = Cfg::kLazyLog2 / sl2;
     uint32_t n_items = 0;
+    uint32_t par_e = 1;  // parity of the o_empty phase of this stage's previous item
+    uint4* drop_blocks = reinterpret_cast<uint4*>(sAlpha + warp * 32);
+    bool after_split = false;
     bool ok = true;
     while (ok) {
       ItemGeom g;
@@ -281,21 +320,39 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       const int j_hi = s ? g.hi[1] : g.hi[0];
       if (q_r1 < q_r0) continue;
       const int row = q_r0 + row_l;
+      DropRow drow = {0u, 0u};
+      if (kDropout) {
+        drow = drop_row(p, g.bh, row);
+        // (the references of a split item lie where this warp's drop_blocks do)
+        if (after_split && !mbar_wait_warp(&o_empty[s], par_e, abort_flag)) break;
+        after_split = g.split;
+      }
       float slope_l2 = 0.f;
       if (kAlibi) slope_l2 = p.alibi_slopes[g.bh % p.heads] * 1.4426950408889634f;
       float m_used = 0.f;  // the row's reference: the score that its exponentials are taken against
+      float m_limit = -INFINITY;  // a tile max above this moves the reference
       float l_run = 0.f;   // 0 until the row has seen a finite score, at least about 1 from then on
-      for (int j = j_lo; j < j_hi; ++j) {
-        if (!mbar_wait_warp(&s_full[s], n_s & 1, abort_flag)) { ok = false; break; }
-        ++n_s;
+      const int kv_step = g.split ? 2 * kBlockN : kBlockN;
+      int kv0 = (g.split ? g.top - 2 * j_lo - s : g.top - j_lo) * kBlockN;
+      const int kv_end = kv0 - (j_hi - j_lo) * kv_step, kv_first = kv0;
+      // Tiles with kv_a <= kv0 <= kv_b are not cut (see kv_tile_needs_mask).
+      const int kv_a = wl >= 0 ? q_r1 - wl : 0;
+      const int kv_b = wr >= 0 ? min(N, q_r0 + wr + 1) - kBlockN : N - kBlockN;
+      for (; kv0 != kv_end && ok; kv0 -= kv_step) {
+        ok = mbar_wait(&s_full[s], par_s, abort_flag);
+        par_s ^= 1u;
         tc_fence_after();
-        const int kv0 = (g.split ? g.top - 2 * j - s : g.top - j) * kBlockN;
         // One body, instantiated twice: tiles cut by a mask boundary (or by the end of the sequence) take the
         // per-element predicate, all others carry none of that code. (Blanking a cut tile in tensor memory first
         // and sharing one body saved 10 KB of instructions but made every tile 4 % slower: the body then
         // starts behind a merge point instead of directly behind the wait.)
         auto tile_body = [&](auto masked_tag) {
           constexpr bool kMasked = decltype(masked_tag)::value;
+          constexpr bool kPoly = !kMasked && !kDropout;
+          if (kDropout) {
+            if (lane < 8) drop_blocks[lane] = drop_block(p, g.bh, static_cast<uint32_t>(kv0 / 16 + lane));
+            __syncwarp();
+          }
           uint32_t r0[32], r1[32], r2[32], r3[32];
           tmem_ld32(tS + 0, r0);
           tmem_ld32(tS + 32, r1);
@@ -361,10 +418,10 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           // (always on the first tile of an item), the 32 exponentials are taken again. Cut tiles do not
           // speculate: most of them are the first tile of their walk.
           uint64_t lsum_a = 0ull, lsum_b = 0ull;
-          uint32_t pk0[32], pk1[32];
+          uint32_t pk0[32];
           if (!kMasked) {
             const float neg_ms0 = -m_used * sl2;
-            exp_quarter_tile(sc, scale2, f2_pack(neg_ms0, neg_ms0), pk0, lsum_a, lsum_b);
+            exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms0, neg_ms0), pk0, lsum_a, lsum_b);
           }
           float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
   #pragma unroll
@@ -380,65 +437,77 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           // shows a finite score: the reference then IS the row max, so the largest term of the row is exactly 1 in
           // fp16 (a row with a single visible key returns that key's V bit for bit). A cut tile over the first keys is
           // the only tile of its walk (with ALiBi it may be the last), or the far edge of a left window lies in it.
-          const bool fresh = l_run == 0.f;
           const bool first_keys = (!kMasked || kAlibi) && kv0 == 0;
-          float alpha = 1.f;
-          if (__any_sync(0xffffffffu, fresh || (m_new - m_used) * sl2 > (first_keys ? 0.f : Cfg::kLazyLog2))) {
+          if (__any_sync(0xffffffffu, m_new > (first_keys ? fminf(m_used, m_limit) : m_limit))) {
+            const bool fresh = l_run == 0.f;
+            float alpha = 1.f;
             if (fresh || m_new > m_used) {
               const float m_next = (m_new == -INFINITY) ? 0.f : m_new;
               alpha = fresh ? 1.f : ex2_approx((m_used - m_next) * sl2);
               m_used = m_next;
             }
+            m_limit = l_run == 0.f && m_new == -INFINITY ? -INFINITY : m_used + lazy;
+            l_run *= alpha;
+            // s_full for this tile was committed behind the previous tile's P.V, so O is at rest here.
+            if (kv0 != kv_first && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+              for (int c = 0; c < D / 16; ++c) {
+                uint32_t r[16];
+                tmem_ld16(tO + c * 16, r);
+                tmem_wait_ld();
+                tmem_ld_fence16(r);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+                tmem_st16(tO + c * 16, r);
+              }
+            }
             if (!kMasked) {
               lsum_a = 0ull;
               lsum_b = 0ull;
               const float neg_ms1 = -m_used * sl2;
-              exp_quarter_tile(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
+              exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
             }
           }
           if (kMasked) {
             const float neg_ms1 = -m_used * sl2;
-            exp_quarter_tile(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
+            exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
           }
-          // (no hand-over on the first tile of an item: there is nothing to rescale yet, and the correction warps
-          // may still be in the previous item's epilogue)
-          if (j != j_lo) sAlpha[s * kBlockM + row_l] = alpha;
-          __syncwarp();
-          if (lane == 0 && j != j_lo) mbar_arrive(&alpha_ready[s]);
           const float neg_ms = -m_used * sl2;
           const uint64_t negms2 = f2_pack(neg_ms, neg_ms);
-          exp_quarter_tile(sc + 32, scale2, negms2, pk0 + 16, lsum_a, lsum_b);
-          if (kDropout) dropout_mask_64(pk0, p, g.bh, row, kv0);  // the row sum keeps every exponential
+          exp_tile<16, kPoly ? Cfg::kPolyOf1 : 0>(sc + 32, scale2, negms2, pk0 + 16, lsum_a, lsum_b);
+          if (kDropout) dropout_mask<4>(pk0, p, drow, drop_blocks);  // the row sum keeps every exponential
           tmem_st32(tS + 0, pk0);
+          uint32_t pk1[16], pk2[16];
+          exp_tile<16, kPoly ? Cfg::kPolyOf2 : 0>(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
+          if (kDropout) dropout_mask<2>(pk1, p, drow, drop_blocks + 4);
+          tmem_st16(tS + 32, pk1);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&p_full[s]);  // P of keys 0..63 is in TMEM
-          exp_half_tile(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
-          if (kDropout) dropout_mask_64(pk1, p, g.bh, row, kv0 + 64);
-          tmem_st32(tS + 32, pk1);
+          mbar_arrive_lane0(&p_full[s], lane);  // P of keys 0..95 is in TMEM
+          exp_tile<16, kPoly ? Cfg::kPolyOf3 : 0>(sc + 96, scale2, negms2, pk2, lsum_a, lsum_b);
+          if (kDropout) dropout_mask<2>(pk2, p, drow, drop_blocks + 6);
+          tmem_st16(tS + 48, pk2);
           float l0, l1;
           f2_unpack(f2_add(lsum_a, lsum_b), l0, l1);
-          l_run = l_run * alpha + (l0 + l1);
+          l_run += l0 + l1;
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&p_full2[s]);  // P of keys 64..127
+          mbar_arrive_lane0(&p_full2[s], lane);  // P of keys 96..127
         };
         // (ALiBi: a tile that the diagonal crosses takes the cut tiles' body, whose bias has the absolute value)
-        if (kv_tile_needs_mask(kv0, q_r0, q_r1, wl, wr, N) ||
-            (kAlibi && kv0 + kBlockN - 1 > q_r0 && kv0 < q_r1))
+        if (kv0 < kv_a || kv0 > kv_b || (kAlibi && kv0 + kBlockN - 1 > q_r0 && kv0 < q_r1))
           tile_body(std::true_type{});
         else tile_body(std::false_type{});
+        ok = __all_sync(0xffffffffu, ok);
       }
       if (!ok) break;
-      // The row sums of the previous item may still be unread when this item is a single tile. The last tile's
-      // p_full phase completes only after the correction warps have arrived on it, and on an item's first tile
-      // they do that after their epilogue of the previous item, which reads the sums first.
-      if (!mbar_wait_warp(&p_full[s], (n_s - 1) & 1, abort_flag)) break;
+      // the epilogue warps have read the row sums of the previous item
+      if (!mbar_wait_warp(&o_empty[s], par_e, abort_flag)) break;
+      par_e ^= 1u;
       sRowSum[s * kBlockM + row_l] = l_run;
-      // a split item's epilogue also needs the reference the sums are taken against; the rescale factors of this item
-      // have all been read, and the next item's first factor is written after its first P.V, i.e. after that epilogue
+      // a split item's epilogue also needs the reference the sums are taken against
       if (g.split) sAlpha[s * kBlockM + row_l] = m_used * sl2;
       __syncwarp();
       if (lane == 0) mbar_arrive(&l_ready[s]);
@@ -450,28 +519,22 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     }
   } else if (warp < 12) {
     // =====================================================================================
-    // correction + epilogue: row = tid % 128 of both stages
+    // epilogue: row = tid % 128 of both stages
     // =====================================================================================
-    reg_dec<FA_REG_CORR>();
+    reg_dec<Cfg::kRegEpilogue>();
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     uint8_t* out_stage = smem + Cfg::kOffOut + (warp & 3) * Cfg::kOutWarpBytes;
     // Bit s: phase parity of stage s's barriers. The stages share one copy of this code (rolled loops, state in bit
     // masks): with copies for both and the epilogue in four places it was 38 KB, mostly run from cold instructions.
-    uint32_t par_alpha = 0, par_l = 0, par_o = 0;
+    uint32_t par_l = 0, par_o = 0;
     uint32_t n_items = 0;
-    // The first P.V product of an item overwrites O, so it has to wait until the epilogue of the previous item
-    // has read O. That hand-off is the correction warps' arrival on p_full for the item's first tile; it is made
-    // right after the epilogue (there is nothing to rescale on a first tile), so the next item's first product
-    // does not wait for these warps to come round to it.
-    uint32_t arrived_early = 0;  // bit s
     bool ok = true;
     while (ok) {
       ItemGeom g;
       const int item = take_item(n_items, g);
       if (item < 0) break;
-      uint32_t epi_pending = g.split ? 0u : (g.r1[0] >= g.r0[0] ? 1u : 0u) | (g.r1[1] >= g.r0[1] ? 2u : 0u);  // bit s
-      // O / l -> fp16 -> global for stage s, then the early arrival for the next item's first tile
+      // O / l -> fp16 -> global for stage s, then the next item's first product may overwrite O
       auto epilogue = [&](int s) {
         if (!mbar_wait_warp(&l_ready[s], (par_l >> s) & 1, abort_flag)) { ok = false; return; }
         par_l ^= 1u << s;
@@ -521,9 +584,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             tma_store_4d(&mapO, out_stage, 0, row0, 0, g.bh);
             tma_store_commit();
           }
-          mbar_arrive(&p_full[s]);
+          mbar_arrive(&o_empty[s]);
         }
-        arrived_early |= 1u << s;
       };
       // Split item: O = (O_0 2^(m_0 - m) + O_1 2^(m_1 - m)) / (l_0 2^(m_0 - m) + l_1 2^(m_1 - m)), m the larger of the
       // two stages' references; then as above.
@@ -583,60 +645,31 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             tma_store_4d(&mapO, out_stage, 0, row0, 0, g.bh);
             tma_store_commit();
           }
-          mbar_arrive(&p_full[0]);
-          mbar_arrive(&p_full[1]);
+          mbar_arrive(&o_empty[0]);
+          mbar_arrive(&o_empty[1]);
         }
-        arrived_early = 3u;
       };
-      for (int j = 0; j <= g.steps && ok; ++j) {
+      if (g.split) {
+        epilogue_split();
+      } else {
+        // the stage that runs out of tiles first is finished first
+        const int first = g.hi[1] < g.hi[0] ? 1 : 0;
 #pragma unroll 1
-        for (int s = 0; s < 2 && ok; ++s) {
-          const int lo = s ? g.lo[1] : g.lo[0], hi = s ? g.hi[1] : g.hi[0];
-          // a stage that has run out of tiles is finished at once, while the other stage may still be in its softmax
-          if (((epi_pending >> s) & 1) && j >= hi) {
-            epi_pending &= ~(1u << s);
-            epilogue(s);
-            continue;
-          }
-          if (j < lo || j >= hi) continue;
-          if (j == lo) {  // first tile of the item: nothing to rescale, and no factors are handed over
-            const bool done = (arrived_early >> s) & 1;
-            arrived_early &= ~(1u << s);
-            if (done) continue;
-          } else {
-            if (!mbar_wait_warp(&alpha_ready[s], (par_alpha >> s) & 1, abort_flag)) { ok = false; break; }
-            par_alpha ^= 1u << s;
-            const float alpha = sAlpha[s * kBlockM + row_l];
-            if (__any_sync(0xffffffffu, alpha != 1.f)) {
-              tc_fence_after();
-              const uint32_t tO = tmem_addr(tmem_base, lane_base, s == 0 ? Cfg::kColO0 : Cfg::kColO1);
-#pragma unroll 1
-              for (int c = 0; c < D / 32; ++c) {
-                uint32_t r[32];
-                tmem_ld32(tO + c * 32, r);
-                tmem_wait_ld();
-                tmem_ld_fence(r);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                tmem_st32(tO + c * 32, r);
-              }
-              tmem_wait_st();
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&p_full[s]);
+        for (int k = 0; k < 2 && ok; ++k) {
+          const int s = first ^ k;
+          if ((s ? g.r1[1] : g.r1[0]) >= (s ? g.r0[1] : g.r0[0])) epilogue(s);
         }
       }
-      if (ok && g.split) epilogue_split();
     }
     if (lane == 0) tma_store_wait_all();  // also on the give-up path: stores in flight read this CTA's shared memory
   } else {
-    reg_dec<FA_REG_MISC>();
+    reg_dec<Cfg::kRegOthers>();
     if (warp == 12) {
       // ===================================================================================
       // tensor-core issuer. The whole warp walks the schedule and waits, so that addresses and
-      // descriptors are warp-uniform values; one elected lane issues the tcgen05 instructions.
+      // descriptors are warp-uniform values; one elected lane issues the tcgen05 instructions. The
+      // verdicts of the waits are gathered and looked at once per round: products issued behind a wait
+      // that gave up stay inside the CTA's own memory, and the round's results are discarded.
       // ===================================================================================
       constexpr uint32_t idesc_qk = umma_idesc_f16(kBlockM, kBlockN, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_f16(kBlockM, D, 0, 1);
@@ -648,7 +681,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       const uint32_t kv_addr = smem_u32(sKV);
       const uint32_t qdesc[2] = {kdesc0 + (q_addr >> 4), kdesc0 + ((q_addr + Cfg::kTileBytes) >> 4)};
       uint32_t pos = 0;               // ring position (tiles since the start) of the first K tile of the current item
-      uint32_t par_p = 0, par_q = 0;  // bit s: phase parity of stage s's barriers
+      uint32_t par_p = 0, par_q = 0, par_e = 3;  // bit s: phase parity of stage s's barriers
       uint32_t n_items = 0;
       bool ok = true;
       // (Every published item has rows, so the loop ends on its first pass. Written without it the compiler's code for the
@@ -678,46 +711,36 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const uint32_t pv = end - ((a.split && s == 0 && j < a.hi[1]) ? 2 : 1);
             const uint32_t slot = pv % Cfg::kStages;
             const uint32_t vdesc = vdesc0 + ((kv_addr + slot * Cfg::kTileBytes) >> 4);
-            if (!mbar_wait_warp(&kv_full[slot], (pv / Cfg::kStages) & 1, abort_flag)) { ok = false; return; }
-            if (!mbar_wait_warp(&p_full[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
-            tc_fence_after();
-            if (elect_one()) {
-              umma_ts_lo(tO, tS, vdesc, kDescHi, idesc_pv, j > alo ? 1u : 0u);
-#pragma unroll
-              for (int kk = 1; kk < 4; ++kk) umma_ts_lo(tO, tS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
+            ok &= mbar_wait(&kv_full[slot], (pv / Cfg::kStages) & 1, abort_flag);
+            if (j == alo) {  // the previous item's O has been read
+              ok &= mbar_wait(&o_empty[s], (par_e >> s) & 1, abort_flag);
+              par_e ^= 1u << s;
             }
-            __syncwarp();
-            if (!mbar_wait_warp(&p_full2[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
+            ok &= mbar_wait(&p_full[s], (par_p >> s) & 1, abort_flag);
+            tc_fence_after();
+            umma_pv96(tO, tS, vdesc, kDescHi, idesc_pv, j > alo ? 1u : 0u);
+            ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
             par_p ^= 1u << s;
             tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-              for (int kk = 4; kk < 8; ++kk) umma_ts_lo(tO, tS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
-              if (a.split || s == 1 || j < a.lo[1] || j >= a.hi[1]) umma_commit(&kv_empty[slot]);
-              umma_commit(&o_full[s]);
-            }
-            __syncwarp();
+            umma_pv32(tO, tS + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
+            umma_commit_warp(&kv_empty[slot], a.split || s == 1 || j < a.lo[1] || j >= a.hi[1]);
+            umma_commit_warp(&o_full[s]);
           }
           if (blo == 0 && bhi > 0) {  // S_s = Q_s K^T
             const uint32_t pk = end + (b.split ? s : 0);
             const uint32_t slot = pk % Cfg::kStages;
-            if (!mbar_wait_warp(&q_full[s], (par_q >> s) & 1, abort_flag)) { ok = false; return; }
+            ok &= mbar_wait(&q_full[s], (par_q >> s) & 1, abort_flag);
             par_q ^= 1u << s;
-            if (!mbar_wait_warp(&kv_full[slot], (pk / Cfg::kStages) & 1, abort_flag)) { ok = false; return; }
+            ok &= mbar_wait(&kv_full[slot], (pk / Cfg::kStages) & 1, abort_flag);
             tc_fence_after();
             const uint32_t kdesc = kdesc0 + ((kv_addr + slot * Cfg::kTileBytes) >> 4);
             const uint32_t qd = s ? qdesc[1] : qdesc[0];
-            if (elect_one()) {
 #pragma unroll
-              for (int k = 0; k < D / 16; ++k) {
-                const uint32_t off = ((k / 4) * Cfg::kPanelBytes + (k % 4) * 32) >> 4;
-                umma_ss_lo(tS, qd + off, kdesc + off, kDescHi, idesc_qk, k > 0 ? 1u : 0u);
-              }
-              umma_commit(&s_full[s]);
-              if (b.split || s == 1 || b.lo[1] > 0 || b.hi[1] == 0) umma_commit(&kv_empty[slot]);
-              if (bhi == 1) umma_commit(&q_empty[s]);
-            }
-            __syncwarp();
+            for (int h = 0; h < D / 64; ++h)
+              umma_qk64(tS, qd + h * (Cfg::kPanelBytes >> 4), kdesc + h * (Cfg::kPanelBytes >> 4), kDescHi, idesc_qk, h);
+            umma_commit_warp(&s_full[s]);
+            umma_commit_warp(&kv_empty[slot], b.split || s == 1 || b.lo[1] > 0 || b.hi[1] == 0);
+            umma_commit_warp(&q_empty[s], bhi == 1);
           }
         }
       };
@@ -726,6 +749,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         ItemGeom none;
         none.steps = none.split = none.lo[0] = none.lo[1] = none.hi[0] = none.hi[1] = 0;
         if (take_nonempty(g)) join(none, g, 0);
+        ok = __all_sync(0xffffffffu, ok);
       }
       while (ok) {
         if (kJoin ? g.steps == 0 : take_item(n_items, g) < 0) break;
@@ -751,7 +775,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         auto wait_next_v = [&]() {  // V_{j+1} lies behind K_{j+1}
           uint32_t slot = slot_k, par = par_k;
           advance(slot, par, 1);
-          return mbar_wait_warp(&kv_full[slot], par, abort_flag);
+          return mbar_wait(&kv_full[slot], par, abort_flag);
         };
         auto round_body = [&](auto interior_tag, auto split_tag, int j) {
           constexpr bool kInterior = decltype(interior_tag)::value;
@@ -767,67 +791,58 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const bool k_seen = !kSplit && (s == 1) && (kInterior || (j + 1 >= g.lo[0] && j + 1 < g.hi[0]));
             const uint32_t colS = (s == 0) ? Cfg::kColS0 : Cfg::kColS1;
             const uint32_t colO = (s == 0) ? Cfg::kColO0 : Cfg::kColO1;
-            if (act_j) {  // O_s += P_s(j) V_j, in two halves of 64 keys as P arrives
+            if (act_j) {  // O_s += P_s(j) V_j, 96 keys and 32 as P arrives
               if (kSplit) {
                 slot_v = slot_k;
                 par_v = par_k;
                 advance(slot_k, par_k, 1);
               }
               const uint32_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
-              if (!kInterior && !v_seen && !mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag)) { ok = false; return; }
-              if (!mbar_wait_warp(&p_full[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
-              tc_fence_after();
-              if (elect_one()) {
-                umma_ts_lo(tmem_base + colO, tmem_base + colS, vdesc, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
-#pragma unroll
-                for (int kk = 1; kk < 4; ++kk)
-                  umma_ts_lo(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
+              if (!kInterior && !v_seen) ok &= mbar_wait(&kv_full[slot_v], par_v, abort_flag);
+              if (!kInterior && j == g.lo[s]) {  // the previous item's O has been read
+                ok &= mbar_wait(&o_empty[s], (par_e >> s) & 1, abort_flag);
+                par_e ^= 1u << s;
               }
-              __syncwarp();
-              if (!mbar_wait_warp(&p_full2[s], (par_p >> s) & 1, abort_flag)) { ok = false; return; }
+              ok &= mbar_wait(&p_full[s], (par_p >> s) & 1, abort_flag);
+              tc_fence_after();
+              umma_pv96(tmem_base + colO, tmem_base + colS, vdesc, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
+              ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
               par_p ^= 1u << s;
               tc_fence_after();
-              if (elect_one()) {
-#pragma unroll
-                for (int kk = 4; kk < 8; ++kk)
-                  umma_ts_lo(tmem_base + colO, tmem_base + colS + kk * 8, vdesc + kk * (2048 >> 4), kDescHi, idesc_pv, 1u);
-                if (!other_j) umma_commit(&kv_empty[slot_v]);
-                if (!kInterior && j + 1 == g.hi[s]) umma_commit(&o_full[s]);
-              }
-              __syncwarp();
+              umma_pv32(tmem_base + colO, tmem_base + colS + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
+              if (!kInterior || !other_j) umma_commit_warp(&kv_empty[slot_v], !other_j);
+              if (!kInterior) umma_commit_warp(&o_full[s], j + 1 == g.hi[s]);
             }
             if (act_n) {  // S_s = Q_s K_{j+1}^T
               if (!kInterior && j + 1 == g.lo[s]) {
-                if (!mbar_wait_warp(&q_full[s], (par_q >> s) & 1, abort_flag)) { ok = false; return; }
+                ok &= mbar_wait(&q_full[s], (par_q >> s) & 1, abort_flag);
                 par_q ^= 1u << s;
               }
-              if (!k_seen && !mbar_wait_warp(&kv_full[slot_k], par_k, abort_flag)) { ok = false; return; }
+              if (!k_seen) ok &= mbar_wait(&kv_full[slot_k], par_k, abort_flag);
               // Inner rounds wait for V here, one round ahead: every group of instructions then has one wait in front
               // of it, about as long as the tensor pipe has work queued (two waits in a row let it run dry).
-              if (kInterior && s == 1 && !wait_next_v()) { ok = false; return; }
+              if (kInterior && s == 1) ok &= wait_next_v();
               tc_fence_after();
               const uint32_t kdesc = kdesc0 + ((kv_addr + slot_k * Cfg::kTileBytes) >> 4);
-              if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < D / 16; ++k) {
-                  const uint32_t off = ((k / 4) * Cfg::kPanelBytes + (k % 4) * 32) >> 4;
-                  umma_ss_lo(tmem_base + colS, qdesc[s] + off, kdesc + off, kDescHi, idesc_qk, k > 0 ? 1u : 0u);
-                }
-                umma_commit(&s_full[s]);
-                if (!other_n) umma_commit(&kv_empty[slot_k]);
-                if (!kInterior && j + 2 == g.hi[s]) umma_commit(&q_empty[s]);
-              }
-              __syncwarp();
+              for (int h = 0; h < D / 64; ++h)
+                umma_qk64(tmem_base + colS, qdesc[s] + h * (Cfg::kPanelBytes >> 4), kdesc + h * (Cfg::kPanelBytes >> 4), kDescHi, idesc_qk, h);
+              umma_commit_warp(&s_full[s]);
+              if (!kInterior || !other_n) umma_commit_warp(&kv_empty[slot_k], !other_n);
+              if (!kInterior) umma_commit_warp(&q_empty[s], j + 2 == g.hi[s]);
               if (kSplit) advance(slot_k, par_k, 1);
             }
           }
         };
         if (g.split) {
-          for (int j = j_first; j < j_end && ok; ++j) round_body(std::false_type{}, std::true_type{}, j);
+          for (int j = j_first; j < j_end && ok; ++j) {
+            round_body(std::false_type{}, std::true_type{}, j);
+            ok = __all_sync(0xffffffffu, ok);
+          }
           pos += 2u * static_cast<uint32_t>(g.hi[0] + g.hi[1]);
         } else {
           for (int j = j_first; j < j_end && ok; ++j) {
-            if (j == in_lo && in_lo < in_hi) ok = mbar_wait_warp(&kv_full[slot_v], par_v, abort_flag);
+            if (j == in_lo && in_lo < in_hi) ok &= mbar_wait(&kv_full[slot_v], par_v, abort_flag);
             if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
             else round_body(std::false_type{}, std::false_type{}, j);
             // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
@@ -835,6 +850,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             par_v = par_k;
             advance(slot_v, par_v, 1);
             advance(slot_k, par_k, 2);
+            ok = __all_sync(0xffffffffu, ok);
           }
           pos += 2u * static_cast<uint32_t>(g.steps);
         }
@@ -843,8 +859,13 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           ItemGeom nx;
           take_nonempty(nx);
           join(g, nx, pos);
+          ok = __all_sync(0xffffffffu, ok);
           g = nx;
         }
+      }
+      if (!ok) {
+        // give-up path: let products that are still in flight end before the CTA retires
+        for (int i = 0; i < 64; ++i) __nanosleep(2000);
       }
     } else if (warp == 13 && lane == 0) {
       // ===================================================================================

@@ -71,6 +71,23 @@ __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
   asm("add.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// 0xFFFF in each half where a < b as fp16
+__device__ __forceinline__ uint32_t f16x2_less_mask(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("set.lt.u32.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// the larger of two values, NaN if either is
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // two floats -> packed fp16x2, round-to-nearest-even; `lo` lands in bits [15:0]
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   uint32_t r;
@@ -103,6 +120,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// Arrival by lane 0 of a warp, without a branch.
+__device__ __forceinline__ void mbar_arrive_lane0(uint64_t* bar, int lane) {
+  asm volatile("{\n.reg .pred p;\nsetp.eq.s32 p, %1, 0;\n@p mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -283,35 +304,92 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same with descriptors given as their low words (start address and leading-dimension offset); the high words are
-// constants, so that only one 32-bit addition per operand and instruction remains.
-__device__ __forceinline__ void umma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                           uint32_t accumulate) {
+// Groups of products issued by a converged warp: one elected lane issues them under a guard predicate, in one block
+// without branches. The 32 products and six satisfied waits of a round at head_dim 128, issued in a loop of their own
+// beside eight softmax warps: 2985 clocks as `if (elect_one()) { products } __syncwarp();` with a vote behind each wait,
+// 2547 in this form, 2366 in this form without the votes; 24 products at head_dim 64 2482, 2093, 1934.
+// Descriptors are given as their low words (start address and leading-dimension offset); the high words are a constant.
+// D (+)= P V for 64 keys: P at `p_tmem`, 8 columns per product; V read MN-major, 2048 bytes per product.
+__device__ __forceinline__ void umma_pv64(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo, uint32_t hi, uint32_t idesc,
+                                          uint32_t accumulate) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
-      ".reg .b64 a, b;\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "mov.b64 a, {%1, %3};\n"
-      "mov.b64 b, {%2, %3};\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n"
+      ".reg .pred lead, acc, yes;\n"
+      ".reg .b64 v;\n"
+      ".reg .b32 lo, p;\n"
+      "elect.sync _|lead, 0xffffffff;\n"
+      "setp.ne.b32 acc, %5, 0;\n"
+      "setp.eq.b32 yes, 0, 0;\n"
+      "mov.b64 v, {%2, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], v, %4, acc;\n"
+      "add.u32 lo, %2, 128;\n add.u32 p, %1, 8;\n mov.b64 v, {lo, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [p], v, %4, yes;\n"
+      "add.u32 lo, %2, 256;\n add.u32 p, %1, 16;\n mov.b64 v, {lo, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [p], v, %4, yes;\n"
+      "add.u32 lo, %2, 384;\n add.u32 p, %1, 24;\n mov.b64 v, {lo, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [p], v, %4, yes;\n"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(p_tmem), "r"(v_lo), "r"(hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                           uint32_t accumulate) {
+// D += P V for 32 keys.
+__device__ __forceinline__ void umma_pv32(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo, uint32_t hi, uint32_t idesc) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
-      ".reg .b64 b;\n"
-      "setp.ne.b32 p, %5, 0;\n"
-      "mov.b64 b, {%2, %3};\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n"
+      ".reg .pred lead, yes;\n"
+      ".reg .b64 v;\n"
+      ".reg .b32 lo, p;\n"
+      "elect.sync _|lead, 0xffffffff;\n"
+      "setp.eq.b32 yes, 0, 0;\n"
+      "mov.b64 v, {%2, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], v, %4, yes;\n"
+      "add.u32 lo, %2, 128;\n add.u32 p, %1, 8;\n mov.b64 v, {lo, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], [p], v, %4, yes;\n"
       "}\n"
       :
-      : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "r"(d_tmem), "r"(p_tmem), "r"(v_lo), "r"(hi), "r"(idesc)
+      : "memory");
+}
+// D (+)= P V for 96 keys.
+__device__ __forceinline__ void umma_pv96(uint32_t d_tmem, uint32_t p_tmem, uint32_t v_lo, uint32_t hi, uint32_t idesc,
+                                          uint32_t accumulate) {
+  umma_pv64(d_tmem, p_tmem, v_lo, hi, idesc, accumulate);
+  umma_pv32(d_tmem, p_tmem + 32, v_lo + 512, hi, idesc);
+}
+// D (+)= Q K^T over 64 elements of head_dim (one 128-byte panel), 32 bytes per product.
+__device__ __forceinline__ void umma_qk64(uint32_t d_tmem, uint32_t q_lo, uint32_t k_lo, uint32_t hi, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred lead, acc, yes;\n"
+      ".reg .b64 q, k;\n"
+      ".reg .b32 a, b;\n"
+      "elect.sync _|lead, 0xffffffff;\n"
+      "setp.ne.b32 acc, %5, 0;\n"
+      "setp.eq.b32 yes, 0, 0;\n"
+      "mov.b64 q, {%1, %3};\n mov.b64 k, {%2, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], q, k, %4, acc;\n"
+      "add.u32 a, %1, 2;\n add.u32 b, %2, 2;\n mov.b64 q, {a, %3};\n mov.b64 k, {b, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], q, k, %4, yes;\n"
+      "add.u32 a, %1, 4;\n add.u32 b, %2, 4;\n mov.b64 q, {a, %3};\n mov.b64 k, {b, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], q, k, %4, yes;\n"
+      "add.u32 a, %1, 6;\n add.u32 b, %2, 6;\n mov.b64 q, {a, %3};\n mov.b64 k, {b, %3};\n"
+      "@lead tcgen05.mma.cta_group::1.kind::f16 [%0], q, k, %4, yes;\n"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(q_lo), "r"(k_lo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// umma_commit() by one elected lane of a converged warp, if `cond`.
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar, bool cond = true) {
+  asm volatile(
+      "{\n"
+      ".reg .pred lead, c;\n"
+      "elect.sync _|lead, 0xffffffff;\n"
+      "setp.ne.and.b32 c, %1, 0, lead;\n"
+      "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(smem_u32(bar)), "r"(static_cast<uint32_t>(cond))
       : "memory");
 }
 // The mbarrier receives one arrival when every tcgen05 operation issued so far by this
@@ -356,6 +434,15 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]),
         "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]),
         "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 // tcgen05.ld writes its destination registers asynchronously; tcgen05.wait::ld makes them valid.

@@ -189,7 +189,7 @@ FA_UNROLL
 // The first item with rows, starting at `item` and going on with what `claim()` returns (the next unclaimed item);
 // -1 when the items have run out. A split pair whose second q tile lies past the end of the sequence counts as two items,
 // one of them without rows. Such an item is never published to the roles of the kernel: the issuing warp looks for the
-// next item before it commits the last product of the current one, the correction warps wait for that commit before they
+// next item before it commits the last product of the current one, the epilogue warps wait for that commit before they
 // free the slot of the item after next, and with two slots two row-less items in a row would close that circle.
 template <typename Claim>
 __host__ __device__ inline int next_item(int item, const FwdParams& p, ItemGeom& g, Claim claim) {

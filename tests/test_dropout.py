@@ -89,6 +89,17 @@ def test_kernel_matches_oracle_with_the_same_mask(pkg, ob, N, d, causal, wl, p):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("H,N,d,causal", [(14, 2048, 64, True), (10, 2048, 128, True), (75, 500, 128, False)])
+def test_mask_of_split_items_that_follow_one_another(pkg, ob, H, N, d, causal):
+    """Several items of one q tile per CTA: what the epilogue of one reads lies where the mask words of the next go."""
+    q, k, v = make_inputs(800 + N + d, 1, H, N, d)
+    got = run_dropout(pkg, q, k, v, 0.2, 99, causal)
+    want = ob.attention_dropout(q, k, v, 0.2, 99, causal=causal)
+    mx, mean, nans = ob.abs_error(got, want)
+    assert nans == 0 and mx <= 2.5e-3 and mean <= 2.5e-4, (mx, mean, nans)  # the bars of the other shapes, times 1/(1-p)
+
+
+@pytest.mark.gpu
 def test_dropout_properties(pkg, ob):
     import torch
 
