@@ -321,7 +321,7 @@ int host_pipe(HostPipe** out) {
 // 512 bytes per GPU that loads the library, held until the process exits.
 // A launch finds its pair at zero and leaves it at zero. A caller that lets two launches on one slot overlap, which is
 // not allowed, may leave a pair off, and a launch that started from such a pair would skip work without knowing. So the
-// launches of a slot take its pairs in turn and each, as it ends, also clears the pair of the next: whatever two
+// launches of a slot take its pairs in turn and each, as it starts, also clears the pair of the next: whatever two
 // overlapping launches did to theirs, the third starts from zero. A launch captured into a graph keeps its pair for
 // every replay, so there a memset node goes in front of it. (A memset in front of every launch cost 2 us a call and kept
 // the kernel from overlapping its predecessor.)

@@ -22,7 +22,7 @@ struct FwdParams {
   int window_left;   // j >= i - window_left   (< 0: unbounded)
   int window_right;  // j <= i + window_right  (< 0: unbounded); forced to 0 by `causal`
   int* status;       // device word, 0 = ok; set non-zero when a bounded wait gave up
-  int status_per_launch;  // 1: the word is this launch's alone (the launch also writes the 0)
+  int status_per_launch;  // 1: the word is this launch's alone (the launch, as it starts, also writes the 0)
   int clear_at;           // then also: the launch clears the pair of a later launch, at sched + clear_at (here, in what was
                           // padding: a block of parameters eight bytes longer cost 2-4 % at head_dim 64)
   float* dbg;        // optional bring-up dump (serial kernel only), else nullptr
@@ -47,8 +47,7 @@ struct FwdParams {
   unsigned seed_lo, seed_hi;
   float drop_scale;         // 256 / drop_keep_thr: the kept elements' 1 / (1 - p), folded into the epilogue
   int* sched;        // device scratch, two words that are 0 between launches: [0] next work item to
-                     // hand out (beyond the first gridDim.x), [1] CTAs that have finished (bits 0-15) and CTAs that
-                     // gave up (bits 16-31)
+                     // hand out (beyond the first gridDim.x), [1] CTAs that claim no more
 };
 
 // Visible key range of query row i is [i - wl, i + wr] ∩ [0, N-1] with "unbounded" for

@@ -254,19 +254,40 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     *abort_flag = 0;
     fence_mbar_init();
   }
+  // Work item in slot `slot` of s_geom
+  auto write_item = [&](uint32_t slot, const ItemGeom& g, int item) {
+    volatile int* w = s_geom + slot * 16;
+    if (item >= 0) {
+      w[0] = g.bh; w[1] = g.pair;
+      w[2] = g.r0[0]; w[3] = g.r0[1]; w[4] = g.r1[0]; w[5] = g.r1[1];
+      w[6] = g.lo[0]; w[7] = g.lo[1]; w[8] = g.hi[0]; w[9] = g.hi[1];
+      w[10] = g.top; w[11] = g.steps; w[13] = g.split;
+    }
+    w[12] = item;
+  };
+  ItemGeom g_first;
+  g_first.steps = 0;
   if (warp == 13 && lane == 0) {
-    prefetch_tensormap(&mapQ);
     prefetch_tensormap(&mapK);
+    prefetch_tensormap(&mapQ);
     prefetch_tensormap(&mapV);
     prefetch_tensormap(&mapO);
+    g_first = decode_item(static_cast<int>(blockIdx.x), p);
+    if (g_first.steps > 0) write_item(0, g_first, static_cast<int>(blockIdx.x));
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Everything above overlaps the end of the kernel in front in the stream; nothing below this line has touched
-  // global memory (inputs, outputs, scheduler words, status) before that kernel is complete.
-  griddep_wait();
+  // Everything above overlaps the end of the kernel in front in the stream, the first item's geometry included. Nothing
+  // touches global memory (inputs, outputs, scheduler words, status) before that kernel is complete: the warps that do
+  // (producer, softmax, epilogue) wait for it at their beginning, and the issuer works on what the producer loads.
+  // A short launch is one chain of latencies: with the first item decoded here, the next launch let in at once where each
+  // CTA has one item, the first loads without waits, and the last CTA found by the producers instead of at the very end,
+  // calls in a row take (us, B200): 1 head x 64 rows d64 6.8 -> 5.0, 4 x 512 d64 9.4 -> 7.2, 8 x 333 d128 causal
+  // 10.4 -> 8.1, 16 x 256 d128 8.3 -> 6.2, 8 x 1024 d128 causal 13.8 -> 11.9. (Running a tile's code once on nothing
+  // while the first loads are under way, so that it comes from the instruction caches, gained nothing in a row of calls
+  // and cost a lone one up to 2 us.)
 
   const int N = p.seqlen;
   const int wl = p.window_left;
@@ -304,6 +325,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const uint64_t scale2 = f2_pack(sl2, sl2);
     const uint32_t tO = tmem_addr(tmem_base, lane_base, s == 0 ? Cfg::kColO0 : Cfg::kColO1);
     uint32_t par_s = 0;  // parity of the next s_full phase
+    griddep_wait();
     const float lazy = Cfg::kLazyLog2 / sl2;
     uint32_t n_items = 0;
     uint32_t par_e = 1;  // parity of the o_empty phase of this stage's previous item
@@ -522,6 +544,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // epilogue: row = tid % 128 of both stages
     // =====================================================================================
     reg_dec<Cfg::kRegEpilogue>();
+    griddep_wait();
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     uint8_t* out_stage = smem + Cfg::kOffOut + (warp & 3) * Cfg::kOutWarpBytes;
@@ -661,7 +684,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         }
       }
     }
-    if (lane == 0) tma_store_wait_all();  // also on the give-up path: stores in flight read this CTA's shared memory
+    if (lane == 0) tma_store_wait_read();  // also on the give-up path: stores in flight read this CTA's shared memory
   } else {
     reg_dec<Cfg::kRegOthers>();
     if (warp == 12) {
@@ -875,39 +898,48 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       uint32_t n_q[2] = {0, 0};
       uint32_t n_pub = 0;
       bool ok = true;
-      int next = static_cast<int>(blockIdx.x);
+      // The first item was decoded in front of the CTA's first barrier. (It may be without rows: then it is none.)
+      ItemGeom g = g_first;
+      int item = -1, claimed = -1;
+      if (g.steps > 0) {
+        mbar_arrive(&item_full[0]);
+        n_pub = 1;
+        item = static_cast<int>(blockIdx.x);
+      }
+      griddep_wait();
+      if (p.status_per_launch && blockIdx.x == 0) {  // (a wait that gives up sets the status much later than this)
+        *p.status = 0;
+        p.sched[p.clear_at] = 0;
+        p.sched[p.clear_at + 1] = 0;
+      }
+      // One item per CTA: the next kernel of the stream may take up the free SMs at once.
+      if (p.num_items <= static_cast<int>(gridDim.x)) griddep_launch();
       while (ok) {
-        ItemGeom g;
-        const int item =
-            next_item(next, p, g, [&] { return static_cast<int>(gridDim.x) + atomicAdd(p.sched, 1); });
-        if (item < 0) griddep_launch();  // no further item: the next kernel of the stream may take up free SMs
-        {  // publish the item to the other roles
+        if (item < 0) {
+          const int next = static_cast<int>(gridDim.x) + (claimed >= 0 ? claimed : atomicAdd(p.sched, 1));
+          item = next_item(next, p, g, [&] { return static_cast<int>(gridDim.x) + atomicAdd(p.sched, 1); });
+          if (item < 0) griddep_launch();  // no further item
           const uint32_t slot = n_pub & 1u;
           if (!mbar_wait(&item_empty[slot], ((n_pub >> 1) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-          volatile int* w = s_geom + slot * 16;
-          if (item >= 0) {
-            w[0] = g.bh; w[1] = g.pair;
-            w[2] = g.r0[0]; w[3] = g.r0[1]; w[4] = g.r1[0]; w[5] = g.r1[1];
-            w[6] = g.lo[0]; w[7] = g.lo[1]; w[8] = g.hi[0]; w[9] = g.hi[1];
-            w[10] = g.top; w[11] = g.steps; w[13] = g.split;
-          }
-          w[12] = item;
+          write_item(slot, g, item);
           mbar_arrive(&item_full[slot]);
           ++n_pub;
+          if (item < 0) break;
         }
-        if (item < 0) break;
-        // Claim the following item now; the answer is looked at behind this item's loads.
-        const int claimed = atomicAdd(p.sched, 1);
         auto load_q = [&](int s) {
           if (g.r1[s] < g.r0[s]) return;
-          if (!ok || !mbar_wait(&q_empty[s], (n_q[s] & 1) ^ 1, abort_flag)) { ok = false; return; }
+          if (n_q[s] > 0 && !mbar_wait(&q_empty[s], (n_q[s] & 1) ^ 1, abort_flag)) ok = false;
+          if (!ok) return;
           ++n_q[s];
           mbar_arrive_expect_tx(&q_full[s], Cfg::kTileBytes);
           tma_load_4d(sQ + s * Cfg::kTileBytes, &mapQ, &q_full[s], 0, g.r0[s], 0, g.bh);
         };
         auto load_tile = [&](const CUtensorMap* map, int tile) {
           const uint32_t slot = it % Cfg::kStages;
-          if (!ok || !mbar_wait(&kv_empty[slot], ((it / Cfg::kStages) & 1) ^ 1, abort_flag)) { ok = false; return; }
+          if (it >= static_cast<uint32_t>(Cfg::kStages) &&
+              !mbar_wait(&kv_empty[slot], ((it / Cfg::kStages) & 1) ^ 1, abort_flag))
+            ok = false;
+          if (!ok) return;
 #ifdef FA_TEST_WITHHOLD_LOAD  // test build only: CTA 0 never loads its fourth tile, so that a bounded wait runs out
           if (blockIdx.x == 0 && (p.variant & 2) != 0 && it == 3) {
             ++it;
@@ -923,6 +955,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         load_tile(&mapK, g.top);
         load_q(0);
         load_q(1);
+        // Claim the following item; the answer is looked at behind this item's loads.
+        claimed = atomicAdd(p.sched, 1);
         if (g.split) {  // in the order of use
           load_tile(&mapK, g.top - 1);
           for (int j = 0; j < g.steps && ok; ++j) {
@@ -939,7 +973,12 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (j + 1 < g.steps) load_tile(&mapK, g.top - j - 1);
           }
         }
-        next = static_cast<int>(gridDim.x) + claimed;
+        item = -1;
+      }
+      // This CTA claims no more: the last one to come here puts the scheduler words back to zero for the next launch.
+      if (atomicAdd(p.sched + 1, 1) + 1 == static_cast<int>(gridDim.x)) {
+        p.sched[0] = 0;
+        p.sched[1] = 0;
       }
       if (!ok) {
         // give-up path: let loads that are still in flight land before the CTA retires
@@ -950,22 +989,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
 
   tc_fence_before();
   __syncthreads();
-  if (tid == 0) {
-    const int gave_up = *abort_flag != 0 ? 1 : 0;
-    if (gave_up) atomicExch(p.status, 1);
-    if (p.status_per_launch && blockIdx.x == 0) {
-      p.sched[p.clear_at] = 0;
-      p.sched[p.clear_at + 1] = 0;
-    }
-    // the last CTA to finish puts the scheduler words back to zero for the next launch
-    const int ended = atomicAdd(p.sched + 1, 1 + (gave_up << 16)) + 1 + (gave_up << 16);
-    if ((ended & 0xffff) == static_cast<int>(gridDim.x)) {
-      if (p.status_per_launch) *p.status = (ended >> 16) != 0 ? 1 : 0;
-      p.sched[0] = 0;
-      p.sched[1] = 0;
-      __threadfence();
-    }
-  }
+  if (tid == 0 && *abort_flag != 0) atomicExch(p.status, 1);
   if (warp == 12) tmem_dealloc(tmem_base, Cfg::kTmemCols);
 }
 
