@@ -13,6 +13,7 @@ reference) and its call site (src/main.cu:99).
 """
 import ctypes
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflashfwd_b200.so")
@@ -43,6 +44,7 @@ EXPORTS = (
 )
 
 _lib = None
+_native = None  # forward() of _torch_binding once looked for; answers NotImplemented where there is none
 
 
 class FlashForwardError(RuntimeError):
@@ -99,7 +101,30 @@ def lib():
     L.flash_forward_shutdown.argtypes = []
     L.flash_forward_shutdown.restype = i
     _lib = L
+    if "torch" in sys.modules:
+        _load_native()
     return L
+
+
+def _load_native():
+    """The native form of attention_forward (host/torch_binding.cpp), which is built against the torch it is used with.
+    Without it everything runs through ctypes, with the same results. With it the loaded library's flash_forward_noalloc is
+    called without ctypes as well, where the arguments are plain numbers."""
+    global _native
+    L = lib()
+    if _native is not None:
+        return _native
+    try:
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+
+        from . import _torch_binding
+    except ImportError:
+        _native = lambda *args: NotImplemented  # noqa: E731
+        return _native
+    _torch_binding.set_noalloc(L.flash_forward_noalloc)
+    L.flash_forward_noalloc = _torch_binding.noalloc
+    _native = _torch_binding.forward
+    return _native
 
 
 def _raise(code):
@@ -192,6 +217,13 @@ def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, so
     With return_lse the result is (out, lse), lse a float32 [B, H, N] tensor (flash_forward_lse).
     With dropout_p > 0 the call is flash_forward_dropout(dropout_p, seed).
     """
+    if kernel == 0 and variant == 0:
+        r = (_native or _load_native())(q, k, v, causal, window_left, window_right, softmax_scale, out, alibi_slopes,
+                                        return_lse, dropout_p, seed)
+        if r is not NotImplemented:
+            if type(r) is int:
+                _raise(r)
+            return r
     import torch
 
     assert q.is_cuda and q.dtype == torch.float16 and q.is_contiguous() and q.dim() == 4

@@ -1,0 +1,104 @@
+"""The native form of the Python entry points (host/torch_binding.cpp) against the Python code that it stands in for: the
+same results bit for bit, the same errors, and whatever it does not know is left to the Python code."""
+import ctypes
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture
+def native(pkg):
+    pkg.lib()
+    fn = pkg._load_native()
+    assert type(fn).__name__ == "builtin_function_or_method", "the binding was not built"
+    return fn
+
+
+def test_arguments_that_are_not_plain_go_to_ctypes(pkg, native):
+    fn = pkg.lib().flash_forward_noalloc
+    assert fn(0, None, 0, 0, 1, 1, 1, 64, 0.0, 0, -1, -1, None, 0, 0) == pkg.FA_INVALID_ARG
+    assert b"null tensor" in pkg.lib().flash_forward_last_error()
+    assert fn(ctypes.c_void_p(16), 16, 16, 16, 1, 1, 1, 63, 0, 0, -1, -1, None, 0, False) == pkg.FA_UNSUPPORTED
+    assert fn(16, 16, 16, 16, 1, 1, 1, 64, 0.0, 0, -1, -1, None, 99, 0) == pkg.FA_INVALID_ARG
+    with pytest.raises(TypeError):
+        fn(1, 2, 3)
+    with pytest.raises(ctypes.ArgumentError):
+        fn(object(), 16, 16, 16, 1, 1, 1, 63, 0.0, 0, -1, -1, None, 0, 0)
+    with pytest.raises(ctypes.ArgumentError):
+        fn(16, 16, 16, 16, 1, 1, 1, 63.0, 0.0, 0, -1, -1, None, 0, 0)
+
+
+def test_tensors_that_are_refused_stay_refused(pkg, native):
+    q = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
+    with pytest.raises(AssertionError):
+        pkg.attention_forward(q, q, q)
+    assert native(q, q, q, False, -1, -1, 0.0, None, None, False, 0.0, 0) is NotImplemented
+    assert native(q, q, q) is NotImplemented
+    with pytest.raises(AttributeError):
+        pkg.attention_forward(None, q, q)
+
+
+FORMS = [dict(), dict(causal=True), dict(causal=1), dict(causal=True, window_left=40), dict(window_left=64, window_right=10),
+         dict(softmax_scale=0.25), dict(softmax_scale=1), dict(alibi=True, causal=True), dict(return_lse=True),
+         dict(return_lse=True, alibi=True), dict(dropout_p=0.3, seed=7), dict(dropout_p=0.3, seed=-1),
+         dict(dropout_p=0.5, alibi=True, seed=1 << 63), dict(out=True), dict(out=True, return_lse=True)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,n", [(64, 200), (128, 77)])
+@pytest.mark.parametrize("form", FORMS, ids=str)
+def test_same_bits_as_the_python_code(pkg, native, monkeypatch, d, n, form):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    q, k, v = (torch.randn(2, 3, n, d, generator=g, device="cuda", dtype=torch.float16) for _ in range(3))
+
+    def call():
+        kw = dict(form)
+        if kw.pop("alibi", False):
+            kw["alibi_slopes"] = torch.tensor([0.5, 0.25, 0.125], device="cuda")
+        given = torch.empty_like(q) if kw.pop("out", False) else None
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+            r = pkg.attention_forward(q, k, v, out=given, **kw)
+            torch.cuda.current_stream().synchronize()
+        r = r if isinstance(r, tuple) else (r,)
+        assert given is None or r[0] is given
+        return r
+    fast = call()
+    monkeypatch.setattr(pkg, "_native", lambda *a: NotImplemented)
+    slow = call()
+    assert len(fast) == len(slow)
+    for a, b in zip(fast, slow):
+        assert a.dtype == b.dtype and a.shape == b.shape and a.device == b.device and not a.requires_grad
+        assert torch.equal(a.view(torch.int16 if a.dtype == torch.float16 else torch.int32),
+                           b.view(torch.int16 if b.dtype == torch.float16 else torch.int32))
+
+
+@pytest.mark.gpu
+def test_errors_and_special_tensors(pkg, native):
+    q = torch.randn(1, 2, 96, 64, device="cuda", dtype=torch.float16)
+    for bad in (q.float(), q[0], q.transpose(1, 2), q[:, :, ::2]):
+        with pytest.raises(AssertionError):
+            pkg.attention_forward(bad, bad, bad)
+    with pytest.raises(AssertionError):
+        pkg.attention_forward(q, q[:, :1].contiguous(), q)
+    with pytest.raises(AssertionError):
+        pkg.attention_forward(q, q, q, alibi_slopes=torch.zeros(3, device="cuda"))
+    with pytest.raises(AssertionError):
+        pkg.attention_forward(q, q, q, dropout_p=0.1, return_lse=True)
+    x = torch.randn(1, 2, 96, 32, device="cuda", dtype=torch.float16)
+    with pytest.raises(pkg.FlashForwardError) as e:
+        pkg.attention_forward(x, x, x)
+    assert e.value.code == pkg.FA_UNSUPPORTED and "head_dim" in str(e.value)
+    with pytest.raises(pkg.FlashForwardError):
+        pkg.attention_forward(q, q, q, softmax_scale=float("nan"))
+    want = pkg.attention_forward(q, q, q)
+    # a parameter that requires a gradient, and a subclass
+    p = torch.nn.Parameter(q.clone())
+    assert torch.equal(pkg.attention_forward(p, p, p), want)
+
+    class Sub(torch.Tensor):
+        pass
+    s = q.clone().as_subclass(Sub)
+    assert torch.equal(pkg.attention_forward(s, s, s).as_subclass(torch.Tensor), want)
