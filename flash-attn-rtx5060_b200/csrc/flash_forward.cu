@@ -80,7 +80,7 @@ struct DeviceState {
   unsigned long long slot_stream[kSchedSlots] = {};  // the id of that launch's stream
   bool slot_used[kSchedSlots] = {};
   unsigned long long acquired_by = 0;  // the stream id of the launch between sched_acquire and sched_release
-  bool attr_set[16] = {};
+  bool attr_set[22] = {};
 };
 
 // Hands out the scheduler words for one launch on `st`. Call with s->mu held; `*slot_out` is passed to
@@ -244,22 +244,24 @@ cudaError_t launch_overlapped(K kernel, int grid, int threads, int smem, cudaStr
   return cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mo, p);
 }
 
-template <int D, bool kAlibi, bool kLse, bool kDropout = false>
+template <int D, bool kAlibi, bool kLse, bool kDropout = false, bool kShort = false>
 int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                          const CUtensorMap& mo,
                          const fa::FwdParams& p, cudaStream_t st) {
   using Cfg = fa::PersistentCfg<D>;
-  // attribute slots 2..5, 8..11 and 12..15: one per instantiation
-  constexpr int slot = (kDropout ? 12 : (kLse ? 8 : 2)) + (kAlibi ? 2 : 0) + (D == 64 ? 0 : 1);
-  int rc = ensure_smem_attr(s, slot, fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout>, Cfg::kSmemBytes);
+  // attribute slots 2..5, 8..15 and 16..21: one per instantiation
+  constexpr int slot = (kShort ? (kDropout ? 20 : kLse ? 18 : 16) : kDropout ? 12 : kLse ? 8 : 2) + (kAlibi ? 2 : 0) +
+                       (D == 64 ? 0 : 1);
+  static_assert(!(kShort && kAlibi), "the short build has no ALiBi");
+  constexpr auto kernel = fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout, kShort>;
+  int rc = ensure_smem_attr(s, slot, kernel, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
   fa::FwdParams pp = p;
   const int grid = pp.num_items < s->num_sms ? pp.num_items : s->num_sms;
   std::lock_guard<std::mutex> lk(s->mu);
   int sched_slot = 0;
   if ((rc = sched_acquire(s, st, &pp.sched, &sched_slot)) != FA_OK) return rc;
-  cudaError_t e = launch_overlapped(fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout>, grid, Cfg::kThreads,
-                                    Cfg::kSmemBytes, st, mq, mk, mv, mo, pp);
+  cudaError_t e = launch_overlapped(kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, st, mq, mk, mv, mo, pp);
   if (e != cudaSuccess) return fail_cuda("launch fwd_persistent_kernel", e);
   return sched_release(s, st, sched_slot);
 }
@@ -271,6 +273,10 @@ int launch_persistent(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& 
                       const CUtensorMap& mo,
                       const fa::FwdParams& p, cudaStream_t st, bool dropout) {
   const bool alibi = p.alibi_slopes != nullptr, lse = p.lse != nullptr;
+  if (!alibi && fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right))
+    return dropout ? launch_persistent_as<D, false, false, true, true>(s, mq, mk, mv, mo, p, st)
+           : lse   ? launch_persistent_as<D, false, true, false, true>(s, mq, mk, mv, mo, p, st)
+                   : launch_persistent_as<D, false, false, false, true>(s, mq, mk, mv, mo, p, st);
   if (dropout) return alibi ? launch_persistent_as<D, true, false, true>(s, mq, mk, mv, mo, p, st)
                             : launch_persistent_as<D, false, false, true>(s, mq, mk, mv, mo, p, st);
   if (alibi) return lse ? launch_persistent_as<D, true, true>(s, mq, mk, mv, mo, p, st)
@@ -337,7 +343,7 @@ struct NoAllocState {
   int num_sms = 0;
   int* scratch = nullptr;  // device address of g_noalloc_scratch on this device
   unsigned launches[kNoAllocSlots] = {};  // per slot: the next launch takes pair launches % kSlotPairs
-  bool attr_set[2] = {};
+  bool attr_set[4] = {};
 };
 NoAllocState g_noalloc[kMaxDevices];
 
@@ -366,24 +372,23 @@ int noalloc_state(NoAllocState** out) {
   return FA_OK;
 }
 
-template <int D>
+template <int D, bool kShort>
 int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                               const CUtensorMap& mo,
                               fa::FwdParams p, cudaStream_t st, bool early) {
   using Cfg = fa::PersistentCfg<D>;
+  constexpr auto kernel = fa::fwd_persistent_kernel<D, false, false, false, kShort>;
   {
     std::lock_guard<std::mutex> lk(s->mu);
-    bool& done = s->attr_set[D == 64 ? 0 : 1];
+    bool& done = s->attr_set[(D == 64 ? 0 : 1) + (kShort ? 2 : 0)];
     if (!done) {
-      cudaError_t e = cudaFuncSetAttribute(fa::fwd_persistent_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           Cfg::kSmemBytes);
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
       if (e != cudaSuccess) return fail_cuda("cudaFuncSetAttribute(MaxDynamicSharedMemorySize)", e);
       done = true;
     }
   }
   const int grid = p.num_items < s->num_sms ? p.num_items : s->num_sms;
-  cudaError_t e = launch_overlapped(fa::fwd_persistent_kernel<D, false>, grid, Cfg::kThreads, Cfg::kSmemBytes, st, mq, mk,
-                                    mv, mo, p, early);
+  cudaError_t e = launch_overlapped(kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, st, mq, mk, mv, mo, p, early);
   if (e != cudaSuccess) return fail_cuda("launch fwd_persistent_kernel", e);
   return FA_OK;
 }
@@ -799,8 +804,12 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   p.status_per_launch = 1;  // the launch writes its own verdict into the status word
   if (captured && (e = cudaMemsetAsync(p.sched, 0, 2 * sizeof(int), st)) != cudaSuccess)
     return fail_cuda("cudaMemsetAsync(scratch slot)", e);
-  rc = head_dim == 64 ? launch_persistent_noalloc<64>(s, mq, mk, mv, mo, p, st, !captured)
-                      : launch_persistent_noalloc<128>(s, mq, mk, mv, mo, p, st, !captured);
+  if (fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right))
+    rc = head_dim == 64 ? launch_persistent_noalloc<64, true>(s, mq, mk, mv, mo, p, st, !captured)
+                        : launch_persistent_noalloc<128, true>(s, mq, mk, mv, mo, p, st, !captured);
+  else
+    rc = head_dim == 64 ? launch_persistent_noalloc<64, false>(s, mq, mk, mv, mo, p, st, !captured)
+                        : launch_persistent_noalloc<128, false>(s, mq, mk, mv, mo, p, st, !captured);
   if (rc != FA_OK || !wait) return rc;
 
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda("cudaStreamSynchronize", e);
@@ -876,7 +885,7 @@ int flash_forward_shutdown(void) {
       std::lock_guard<std::mutex> lk2(na.mu);
       na.ready = false;
       na.scratch = nullptr;
-      na.attr_set[0] = na.attr_set[1] = false;
+      for (bool& b : na.attr_set) b = false;
     }
     HostPipe& hp = g_pipe[d];
     std::lock_guard<std::mutex> lkp(hp.mu);

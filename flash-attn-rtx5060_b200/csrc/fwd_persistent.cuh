@@ -9,7 +9,8 @@
 //               the warp's staging area in shared memory -> one TMA store)
 //   warp 12     tensor-core issuer: the warp walks the schedule, one elected lane issues tcgen05.mma
 //   warp 13     TMA producer: Q tiles and the K/V tile ring
-//   warps 14-15 idle (they only donate registers)
+//   warp 14     Q of the CTA's first item, beside the producer's first K/V tiles; else idle, as warp 15 (they only donate
+//               registers)
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D); the fp16 P tile of a
 // stage overwrites the first 64 columns of its own S and is handed to the tensor pipe in two
 // parts of 96 and 32 keys, so that most of P.V runs while the last keys are still being exponentiated and little of it
@@ -88,6 +89,9 @@ struct PersistentCfg {
   // Registers per thread after setmaxnreg: 8 softmax warps, 4 epilogue warps, 4 others; 256 * softmax + 128 * epilogue +
   // 128 * others <= 65536. At head_dim 64, where the exponentials are the limit, 200 let more of them be in flight (32
   // heads x 8192 rows 719 -> 680 us); at head_dim 128 it costs 2-4 %.
+  // Columns that the epilogue takes at a time: 8 fit the 40 registers of head_dim 64 (16 spill, 3 % of the smallest calls);
+  // at head_dim 128 16 are 3 % faster than 8.
+  static constexpr int kEpilogueCols = D == 64 ? 8 : 16;
   static constexpr int kRegSoftmax = D == 64 ? 200 : 184, kRegEpilogue = D == 64 ? 40 : 72, kRegOthers = 72;
 };
 
@@ -189,7 +193,14 @@ __device__ __forceinline__ void dropout_mask(uint32_t* pk, const FwdParams& p, c
   }
 }
 
-template <int D, bool kAlibi, bool kLse = false, bool kDropout = false>
+// kShort: the build for launches whose q tiles see few kv tiles (short_items() in work_items.h). There an item's code comes
+// from cold instruction caches as often as not and the time between items weighs as much as the rounds, so what counts is
+// how little code there is: cut tiles are blanked in tensor memory by a small loop and go through the same body as all
+// others, the row max comes before any exponential (no second copy of the first ones), the issuer has no rounds of its
+// own for the inside of an item, and at head_dim 128, where these launches are not bound by the exponentials, none are
+// taken on the FMA pipe. Without ALiBi, whose body differs for cut tiles. (With a body per kind of tile, one of them
+// blanked: nothing gained. In long sequences one body costs 3-6 %.)
+template <int D, bool kAlibi, bool kLse = false, bool kDropout = false, bool kShort = false>
 __global__ void __launch_bounds__(512, 1)
 fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO,
@@ -267,13 +278,13 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   };
   ItemGeom g_first;
   g_first.steps = 0;
-  if (warp == 13 && lane == 0) {
+  if ((warp == 13 || warp == 14) && lane == 0) {
     prefetch_tensormap(&mapK);
     prefetch_tensormap(&mapQ);
     prefetch_tensormap(&mapV);
     prefetch_tensormap(&mapO);
     g_first = decode_item(static_cast<int>(blockIdx.x), p);
-    if (g_first.steps > 0) write_item(0, g_first, static_cast<int>(blockIdx.x));
+    if (warp == 13 && g_first.steps > 0) write_item(0, g_first, static_cast<int>(blockIdx.x));
   }
   tc_fence_before();
   __syncthreads();
@@ -285,7 +296,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   // A short launch is one chain of latencies: with the first item decoded here, the next launch let in at once where each
   // CTA has one item, the first loads without waits, and the last CTA found by the producers instead of at the very end,
   // calls in a row take (us, B200): 1 head x 64 rows d64 6.8 -> 5.0, 4 x 512 d64 9.4 -> 7.2, 8 x 333 d128 causal
-  // 10.4 -> 8.1, 16 x 256 d128 8.3 -> 6.2, 8 x 1024 d128 causal 13.8 -> 11.9. (Running a tile's code once on nothing
+  // 10.4 -> 8.1, 16 x 256 d128 8.3 -> 6.2, 8 x 1024 d128 causal 13.8 -> 11.9. With a warp of its own for the first Q tiles
+  // and the next launch let in behind the first loads: 4.5, 6.8, 7.9, 5.9, 11.9. (Running a tile's code once on nothing
   // while the first loads are under way, so that it comes from the instruction caches, gained nothing in a row of calls
   // and cost a lone one up to 2 us.)
 
@@ -366,11 +378,44 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         tc_fence_after();
         // One body, instantiated twice: tiles cut by a mask boundary (or by the end of the sequence) take the
         // per-element predicate, all others carry none of that code. (Blanking a cut tile in tensor memory first
-        // and sharing one body saved 10 KB of instructions but made every tile 4 % slower: the body then
-        // starts behind a merge point instead of directly behind the wait.)
+        // and sharing one body, as the short build does, makes every tile 3-6 % slower: the body then starts behind a
+        // merge point instead of directly behind the wait.)
+        // Visible columns of this row: c_lo <= c <= c_hi, i.e. |c - mid| <= half. The predicate is applied on the
+        // FMA pipe, which the softmax leaves nearly idle, instead of as two integer compares and a select per
+        // element: t = saturate(|c - mid| - half) is 0 for a visible column and 1 for a hidden one (both
+        // operands are multiples of 1/2, so the difference is exact), and sc - 3e38 * t leaves a visible
+        // score bit for bit as it is and puts a hidden one near -3e38, where its exponential is 0 for any scale the
+        // host accepts.
+        auto visible_columns = [&](float& mid, float& half) {
+          const int c_lo = (wl >= 0) ? row - wl - kv0 : -(1 << 20);
+          int c_hi = N - 1 - kv0;
+          if (wr >= 0) c_hi = min(c_hi, row + wr - kv0);
+          mid = 0.5f * static_cast<float>(c_lo + c_hi);
+          half = 0.5f * static_cast<float>(c_hi - c_lo);  // negative: no visible column at all
+        };
+        auto hide = [](float score, float c, float mid, float half) {
+          return fmaf(__saturatef(fabsf(c - mid) - half), -3.0e38f, score);
+        };
+        auto blank_hidden = [&]() {
+          float mid, half;
+          visible_columns(mid, half);
+#pragma unroll 1
+          for (int c0 = 0; c0 < kBlockN; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld32(tS + c0, r);
+            tmem_wait_ld();
+            tmem_ld_fence(r);
+            const float m0 = mid - static_cast<float>(c0);
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+              r[c] = __float_as_uint(hide(__uint_as_float(r[c]), static_cast<float>(c), m0, half));
+            tmem_st32(tS + c0, r);
+          }
+          tmem_wait_st();
+        };
         auto tile_body = [&](auto masked_tag) {
           constexpr bool kMasked = decltype(masked_tag)::value;
-          constexpr bool kPoly = !kMasked && !kDropout;
+          constexpr bool kPoly = !kMasked && !kDropout && !(kShort && D == 128);
           if (kDropout) {
             if (lane < 8) drop_blocks[lane] = drop_block(p, g.bh, static_cast<uint32_t>(kv0 / 16 + lane));
             __syncwarp();
@@ -416,23 +461,10 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             }
           }
           if (kMasked) {
-            // Visible columns of this row: c_lo <= c <= c_hi, i.e. |c - mid| <= half. The predicate is applied on the
-            // FMA pipe, which the softmax leaves nearly idle, instead of as two integer compares and a select per
-            // element: t = saturate(|c - mid| - half) is 0 for a visible column and 1 for a hidden one (both
-            // operands are multiples of 1/2, so the difference is exact), and sc - kHidden * t leaves a visible
-            // score bit for bit as it is and puts a hidden one near -3e38, where its exponential is 0 for any scale the
-            // host accepts.
-            const int c_lo = (wl >= 0) ? row - wl - kv0 : -(1 << 20);
-            int c_hi = N - 1 - kv0;
-            if (wr >= 0) c_hi = min(c_hi, row + wr - kv0);
-            const float mid = 0.5f * static_cast<float>(c_lo + c_hi);
-            const float half = 0.5f * static_cast<float>(c_hi - c_lo);  // negative: no visible column at all
-            constexpr float kHidden = 3.0e38f;
+            float mid, half;
+            visible_columns(mid, half);
   #pragma unroll
-            for (int c = 0; c < kBlockN; ++c) {
-              const float t = __saturatef(fabsf(static_cast<float>(c) - mid) - half);
-              sc[c] = fmaf(t, -kHidden, sc[c]);
-            }
+            for (int c = 0; c < kBlockN; ++c) sc[c] = hide(sc[c], static_cast<float>(c), mid, half);
           }
           // The exponentials of the first 32 keys are taken against the reference the previous tile left while
           // the row max of this tile is still being reduced: nearly always the reference stays where it is (lazy
@@ -441,7 +473,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           // speculate: most of them are the first tile of their walk.
           uint64_t lsum_a = 0ull, lsum_b = 0ull;
           uint32_t pk0[32];
-          if (!kMasked) {
+          if (!kMasked && !kShort) {
             const float neg_ms0 = -m_used * sl2;
             exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms0, neg_ms0), pk0, lsum_a, lsum_b);
           }
@@ -454,7 +486,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             mx3 = max3(mx3, sc[c + 6], sc[c + 7]);
           }
           float m_new = max3(mx0, mx1, fmaxf(mx2, mx3));
-          if (kMasked && m_new < -1.0e37f) m_new = -INFINITY;  // nothing visible (hidden scores sit near -3e38)
+          if ((kMasked || kShort) && m_new < -1.0e37f) m_new = -INFINITY;  // nothing visible (hidden scores sit near -3e38)
           // The reference moves when the tile's max has grown past it (see kLazyLog2), and always on the first tile that
           // shows a finite score: the reference then IS the row max, so the largest term of the row is exactly 1 in
           // fp16 (a row with a single visible key returns that key's V bit for bit). A cut tile over the first keys is
@@ -483,14 +515,14 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 tmem_st16(tO + c * 16, r);
               }
             }
-            if (!kMasked) {
+            if (!kMasked && !kShort) {
               lsum_a = 0ull;
               lsum_b = 0ull;
               const float neg_ms1 = -m_used * sl2;
               exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
             }
           }
-          if (kMasked) {
+          if (kMasked || kShort) {
             const float neg_ms1 = -m_used * sl2;
             exp_tile<16, 0>(sc, scale2, f2_pack(neg_ms1, neg_ms1), pk0, lsum_a, lsum_b);
           }
@@ -518,10 +550,16 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           __syncwarp();
           mbar_arrive_lane0(&p_full2[s], lane);  // P of keys 96..127
         };
-        // (ALiBi: a tile that the diagonal crosses takes the cut tiles' body, whose bias has the absolute value)
-        if (kv0 < kv_a || kv0 > kv_b || (kAlibi && kv0 + kBlockN - 1 > q_r0 && kv0 < q_r1))
+        const bool cut = kv0 < kv_a || kv0 > kv_b;
+        if (kShort) {
+          if (cut) blank_hidden();
+          tile_body(std::false_type{});
+        } else if (cut || (kAlibi && kv0 + kBlockN - 1 > q_r0 && kv0 < q_r1)) {
+          // (ALiBi: a tile that the diagonal crosses takes the cut tiles' body, whose bias has the absolute value)
           tile_body(std::true_type{});
-        else tile_body(std::false_type{});
+        } else {
+          tile_body(std::false_type{});
+        }
         ok = __all_sync(0xffffffffu, ok);
       }
       if (!ok) break;
@@ -548,6 +586,9 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     uint8_t* out_stage = smem + Cfg::kOffOut + (warp & 3) * Cfg::kOutWarpBytes;
+    // Columns 8u .. 8u+7 of the lane's row are 16-byte unit u%8 of panel u/8; unit x of row r sits at x ^ (r%8).
+    auto out_row = [&](int u) { return out_stage + (u >> 3) * (32 * 128) + lane * 128 + ((u & 7) ^ (lane & 7)) * 16; };
+    constexpr int kCols = Cfg::kEpilogueCols;
     // Bit s: phase parity of stage s's barriers. The stages share one copy of this code (rolled loops, state in bit
     // masks): with copies for both and the epilogue in four places it was 38 KB, mostly run from cold instructions.
     uint32_t par_l = 0, par_o = 0;
@@ -572,29 +613,26 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         // clocks per tile, and the barrier traffic of every other warp of the SM queued behind them.
         if (lane == 0) tma_store_wait_read();  // the previous store of this warp has read the staging area
         __syncwarp();
-        // 16 columns at a time, the load of the next chunk in flight while this one is converted and stored.
+        // kCols columns at a time, the load of the next chunk in flight while this one is converted and stored.
         // (Rolled up: this path runs once per item and stage, and instructions that are rarely executed are
         // fetched slowly; unrolling it eightfold made the change-over between items slower, not faster.)
-        uint32_t ra[16], rb[16];
-        tmem_ld16(tO, ra);
+        uint32_t ra[kCols], rb[kCols];
+        tmem_ld_cols(tO, ra);
   #pragma unroll 2
-        for (int c = 0; c < D / 16; ++c) {
-          uint32_t (&cur)[16] = (c & 1) ? rb : ra;
-          uint32_t (&nxt)[16] = (c & 1) ? ra : rb;
+        for (int c = 0; c < D / kCols; ++c) {
+          uint32_t (&cur)[kCols] = (c & 1) ? rb : ra;
+          uint32_t (&nxt)[kCols] = (c & 1) ? ra : rb;
           tmem_wait_ld();
-          tmem_ld_fence16(cur);
-          if (c + 1 < D / 16) tmem_ld16(tO + (c + 1) * 16, nxt);
-          // columns 16c .. 16c+15 are 16-byte units 2(c%4), 2(c%4)+1 of panel c/4; unit u of row r sits at u ^ (r%8)
-          uint8_t* prow = out_stage + (c >> 2) * (32 * 128) + lane * 128;
-  #pragma unroll
-          for (int i = 0; i < 2; ++i) {
+          tmem_ld_fence_cols(cur);
+          if (c + 1 < D / kCols) tmem_ld_cols(tO + (c + 1) * kCols, nxt);
+#pragma unroll
+          for (int i = 0; i < kCols / 8; ++i) {
             uint4 v;
             v.x = pack_f16x2(__uint_as_float(cur[i * 8 + 0]) * inv_l, __uint_as_float(cur[i * 8 + 1]) * inv_l);
             v.y = pack_f16x2(__uint_as_float(cur[i * 8 + 2]) * inv_l, __uint_as_float(cur[i * 8 + 3]) * inv_l);
             v.z = pack_f16x2(__uint_as_float(cur[i * 8 + 4]) * inv_l, __uint_as_float(cur[i * 8 + 5]) * inv_l);
             v.w = pack_f16x2(__uint_as_float(cur[i * 8 + 6]) * inv_l, __uint_as_float(cur[i * 8 + 7]) * inv_l);
-            const int unit = ((c & 3) * 2 + i) ^ (lane & 7);
-            *reinterpret_cast<uint4*>(prow + unit * 16) = v;
+            *reinterpret_cast<uint4*>(out_row(c * (kCols / 8) + i)) = v;
           }
         }
         fence_proxy_async_smem();
@@ -639,16 +677,15 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (lane == 0) tma_store_wait_read();
         __syncwarp();
 #pragma unroll 1
-        for (int c = 0; c < D / 16; ++c) {
-          uint32_t ra[16], rb[16];
-          tmem_ld16(tO0 + c * 16, ra);
-          tmem_ld16(tO1 + c * 16, rb);
+        for (int c = 0; c < D / kCols; ++c) {
+          uint32_t ra[kCols], rb[kCols];
+          tmem_ld_cols(tO0 + c * kCols, ra);
+          tmem_ld_cols(tO1 + c * kCols, rb);
           tmem_wait_ld();
-          tmem_ld_fence16(ra);
-          tmem_ld_fence16(rb);
-          uint8_t* prow = out_stage + (c >> 2) * (32 * 128) + lane * 128;
+          tmem_ld_fence_cols(ra);
+          tmem_ld_fence_cols(rb);
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
+          for (int i = 0; i < kCols / 8; ++i) {
             uint32_t v[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -656,8 +693,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               v[k] = pack_f16x2(fmaf(__uint_as_float(ra[e]), f0, __uint_as_float(rb[e]) * f1),
                                 fmaf(__uint_as_float(ra[e + 1]), f0, __uint_as_float(rb[e + 1]) * f1));
             }
-            const int unit = ((c & 3) * 2 + i) ^ (lane & 7);
-            *reinterpret_cast<uint4*>(prow + unit * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<uint4*>(out_row(c * (kCols / 8) + i)) = make_uint4(v[0], v[1], v[2], v[3]);
           }
         }
         fence_proxy_async_smem();
@@ -865,8 +901,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           pos += 2u * static_cast<uint32_t>(g.hi[0] + g.hi[1]);
         } else {
           for (int j = j_first; j < j_end && ok; ++j) {
-            if (j == in_lo && in_lo < in_hi) ok &= mbar_wait(&kv_full[slot_v], par_v, abort_flag);
-            if (j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
+            if (!kShort && j == in_lo && in_lo < in_hi) ok &= mbar_wait(&kv_full[slot_v], par_v, abort_flag);
+            if (!kShort && j >= in_lo && j < in_hi) round_body(std::true_type{}, std::false_type{}, j);
             else round_body(std::false_type{}, std::false_type{}, j);
             // V_{j+1} sits right after K_{j+1}; K_{j+2} two positions after K_{j+1}
             slot_v = slot_k;
@@ -890,6 +926,17 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         // give-up path: let products that are still in flight end before the CTA retires
         for (int i = 0; i < 64; ++i) __nanosleep(2000);
       }
+    } else if (warp == 14 && lane == 0) {
+      // Q of the CTA's first item, beside the producer's first K/V tiles
+      griddep_wait();
+      if (g_first.steps > 0) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (g_first.r1[s] < g_first.r0[s]) continue;
+          mbar_arrive_expect_tx(&q_full[s], Cfg::kTileBytes);
+          tma_load_4d(sQ + s * Cfg::kTileBytes, &mapQ, &q_full[s], 0, g_first.r0[s], 0, g_first.bh);
+        }
+      }
     } else if (warp == 13 && lane == 0) {
       // ===================================================================================
       // TMA producer
@@ -898,6 +945,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       uint32_t n_q[2] = {0, 0};
       uint32_t n_pub = 0;
       bool ok = true;
+      bool first = g_first.steps > 0;
       // The first item was decoded in front of the CTA's first barrier. (It may be without rows: then it is none.)
       ItemGeom g = g_first;
       int item = -1, claimed = -1;
@@ -912,8 +960,6 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         p.sched[p.clear_at] = 0;
         p.sched[p.clear_at + 1] = 0;
       }
-      // One item per CTA: the next kernel of the stream may take up the free SMs at once.
-      if (p.num_items <= static_cast<int>(gridDim.x)) griddep_launch();
       while (ok) {
         if (item < 0) {
           const int next = static_cast<int>(gridDim.x) + (claimed >= 0 ? claimed : atomicAdd(p.sched, 1));
@@ -953,10 +999,17 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         // The Q tiles of the previous item are released one after the other, stage 0 first; the ring slots of the
         // first kv tiles usually before either.
         load_tile(&mapK, g.top);
-        load_q(0);
-        load_q(1);
+        if (it == 1 && first) {  // (warp 14 loads the first item's)
+          for (int s = 0; s < 2; ++s) n_q[s] += g.r1[s] >= g.r0[s] ? 1 : 0;
+        } else {
+          load_q(0);
+          load_q(1);
+        }
+        first = false;
         // Claim the following item; the answer is looked at behind this item's loads.
         claimed = atomicAdd(p.sched, 1);
+        // One item per CTA: the next kernel of the stream may take up the free SMs at once.
+        if (p.num_items <= static_cast<int>(gridDim.x)) griddep_launch();
         if (g.split) {  // in the order of use
           load_tile(&mapK, g.top - 1);
           for (int j = 0; j < g.steps && ok; ++j) {

@@ -73,6 +73,25 @@ inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, in
   return few || 2 * pairs <= num_sms ? pairs : 0;
 }
 
+// Whether a launch takes the kernel's short build: q tiles that see few kv tiles, most of all where some of them are cut,
+// since the other build has a body of code for either kind. It depends on the shape of a head alone, so chunks and slabs
+// of a problem take the build that the whole would. Time of the other build over the short one's, head_dim 64 / 128
+// (batch x heads x rows):
+//   no mask        16x16x128 1.08 / 1.16, 16x16x256 1.08 / 1.07, 8x16x640 1.05 / 1.08, 8x16x768 0.98 / 1.01,
+//                  8x16x1024 0.98 / 1.02
+//   ..., ragged    8x12x700 1.04 / 1.06, 8x12x1000 1.01 / 1.04, 8x12x1200, 1300 1.01 / 1.05, 8x12x1700 - / 1.00
+//   causal         16x16x512 1.11 / 1.09, 8x16x1024 1.09 / 1.08, 4x16x2048 1.03 / 1.05, 4x16x2560 1.01 / 1.02,
+//                  4x16x3072 1.00 / 1.02, 24x4001 - / 0.97
+//   window (left, right) over 4x16x4096   256,0 1.09 / 1.02, 512,0 1.01 / 1.01, 768,0 0.99 / 1.00, 1024,0 0.98 / 0.96,
+//                  128,128 1.10 / 1.03, 256,256 1.04 / 1.04, 512,512 1.02 / 1.00
+// With dropout 16x4x256 1.24, 16x4x1024 1.07 / 1.10, 16x4x2048 1.02 / 1.06.
+inline bool short_items(int seqlen, int causal, int window_left, int window_right) {
+  const int wr = eff_window_right(causal, window_right);
+  if (window_left < 0 && wr < 0) return seqlen <= (seqlen % kBlockN ? 10 : 5) * kBlockN;
+  if (seqlen <= 20 * kBlockN) return true;
+  return window_left >= 0 && wr >= 0 && wr <= 4 * kBlockN && window_left <= 4 * kBlockN - wr;
+}
+
 // The items of a launch on p->bh heads, the first of which is head `first_head` of a problem of `total_heads`: its order
 // (head_group), and how many pairs at the end of that order are taken apart. A split q tile is summed in another order
 // than a pair's, so which pairs are split is decided for the whole problem: the chunks of flash_forward_host and the slabs

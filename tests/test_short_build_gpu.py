@@ -1,0 +1,82 @@
+"""The kernel has a build for q tiles that see few kv tiles and one for all others; which of them a launch takes depends on
+the sequence length and the masks alone (short_items() in csrc/work_items.h). Both sides of every line, against the
+attention of the same inputs in 64 bits."""
+import math
+
+import numpy as np
+import pytest
+
+from conftest import make_inputs
+
+pytestmark = pytest.mark.gpu
+
+#          rows, causal, left, right
+EDGES = [(640, False, -1, -1), (768, False, -1, -1), (641, False, -1, -1), (1280, False, -1, -1), (1279, False, -1, -1),
+         (1281, False, -1, -1), (2560, True, -1, -1), (2561, True, -1, -1), (2688, True, -1, -1), (2900, True, 512, -1),
+         (2900, True, 513, -1), (2816, False, 200, 312), (2816, False, 200, 313), (2800, False, -1, 40), (2500, False, 90, -1),
+         (1, True, -1, -1), (128, False, -1, -1), (129, True, 0, -1)]
+
+
+def exact(q, k, v, causal, wl, wr):
+    import torch
+
+    n, d = q.shape[2:]
+    i = torch.arange(n, device="cuda")
+    gap = i[None, :] - i[:, None]
+    hidden = torch.zeros(n, n, dtype=torch.bool, device="cuda")
+    if wl >= 0:
+        hidden |= gap < -wl
+    if causal:
+        hidden |= gap > 0
+    elif wr >= 0:
+        hidden |= gap > wr
+    s = (q.double() @ k.double().transpose(-1, -2) / math.sqrt(d)).masked_fill_(hidden, -math.inf)
+    return torch.softmax(s, dim=-1) @ v.double(), torch.logsumexp(s, dim=-1)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n,causal,wl,wr", EDGES)
+def test_both_builds_at_the_lines_between_them(pkg, d, n, causal, wl, wr):
+    import torch
+
+    q, k, v = (torch.from_numpy(a).cuda() for a in make_inputs(n + d, 1, 3, n, d))
+    want, want_lse = exact(q, k, v, causal, wl, wr)
+    kw = dict(causal=causal, window_left=wl, window_right=wr)
+    out = pkg.attention_forward(q, k, v, **kw)
+    out2, lse = pkg.attention_forward(q, k, v, return_lse=True, **kw)
+    own = torch.empty_like(q)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert pkg.lib().flash_forward_noalloc(q.data_ptr(), k.data_ptr(), v.data_ptr(), own.data_ptr(), 1, 3, n, d, 0.0,
+                                           int(causal), wl, wr, stream, 0, 1) == pkg.FA_OK
+    pkg.check(stream)
+    for o in (out, out2, own):
+        # probabilities and output rounded to fp16: 2^-11 of |v| (rows that see one key: exact) and half an ulp of the
+        # output; the largest |v| is about 4.5
+        assert (o.double() - want).abs().max().item() < 4e-3
+        assert ((o.double() - want).norm() / want.norm()).item() < 4e-4
+    assert torch.equal(own, out)                            # the same kernel behind either entry point
+    assert (lse.double() - want_lse).abs().max().item() < 5e-5  # fp32 sums of up to 2900 terms
+    if causal or wl == 0:
+        assert torch.equal(out[:, :, 0], v[:, :, 0])        # one visible key: its value bit for bit
+
+
+@pytest.mark.parametrize("n,d,causal", [(2500, 64, True), (2700, 64, True), (1200, 128, False), (1400, 128, False)])
+def test_dropout_in_both_builds(pkg, ob, n, d, causal):
+    import torch
+
+    q, k, v = make_inputs(n, 1, 1, n, d)
+    out = pkg.attention_forward(*(torch.from_numpy(a).cuda() for a in (q, k, v)), causal=causal, dropout_p=0.2, seed=5)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    mx, mean, nans = ob.abs_error(out.cpu().numpy(), ob.attention_dropout(q, k, v, 0.2, 5, causal=causal))
+    assert nans == 0 and mx <= 2.5e-3 and mean <= 2.5e-4, (mx, mean, nans)
+
+
+def test_the_line_does_not_depend_on_the_number_of_heads(pkg):
+    import torch
+
+    q, k, v = (torch.from_numpy(a).cuda() for a in make_inputs(3, 1, 8, 2560, 64))
+    whole = pkg.attention_forward(q, k, v, causal=True)
+    parts = [pkg.attention_forward(*(t[:, h:h + 4].contiguous() for t in (q, k, v)), causal=True) for h in (0, 4)]
+    err = (torch.cat(parts, dim=1).float() - whole.float()).abs().max().item()
+    assert err <= 2.0 ** -9  # an ulp of outputs of up to 4: pairs of q tiles may be split in the one and not the other
+    assert np.isfinite(err)
