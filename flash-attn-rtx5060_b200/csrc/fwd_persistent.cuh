@@ -88,11 +88,12 @@ struct PersistentCfg {
   static constexpr int kPolyOf1 = D == 64 ? 2 : 4, kPolyOf2 = 4, kPolyOf3 = 4;
   // Registers per thread after setmaxnreg: 8 softmax warps, 4 epilogue warps, 4 others; 256 * softmax + 128 * epilogue +
   // 128 * others <= 65536. At head_dim 64, where the exponentials are the limit, 200 let more of them be in flight (32
-  // heads x 8192 rows 719 -> 680 us); at head_dim 128 it costs 2-4 %.
+  // heads x 8192 rows 719 -> 680 us); at head_dim 128 it costs 2-4 %. The short build has fewer values live.
   // Columns that the epilogue takes at a time: 8 fit the 40 registers of head_dim 64 (16 spill, 3 % of the smallest calls);
   // at head_dim 128 16 are 3 % faster than 8.
   static constexpr int kEpilogueCols = D == 64 ? 8 : 16;
   static constexpr int kRegSoftmax = D == 64 ? 200 : 184, kRegEpilogue = D == 64 ? 40 : 72, kRegOthers = 72;
+  static constexpr int kRegSoftmaxShort = 184, kRegEpilogueShort = 72;
 };
 
 // 2^x of two values on the FMA pipe: x = n + f with n the nearest integer (the usual addition of 1.5 * 2^23 rounds x to
@@ -326,7 +327,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // =====================================================================================
     // softmax: stage s = warp / 4, row = tid % 128
     // =====================================================================================
-    reg_inc<Cfg::kRegSoftmax>();
+    reg_inc<kShort ? Cfg::kRegSoftmaxShort : Cfg::kRegSoftmax>();
     const int s = warp >> 2;
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
@@ -581,14 +582,14 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // =====================================================================================
     // epilogue: row = tid % 128 of both stages
     // =====================================================================================
-    reg_dec<Cfg::kRegEpilogue>();
+    reg_dec<kShort ? Cfg::kRegEpilogueShort : Cfg::kRegEpilogue>();
     griddep_wait();
     const int row_l = tid & 127;
     const uint32_t lane_base = static_cast<uint32_t>(warp & 3) * 32u;
     uint8_t* out_stage = smem + Cfg::kOffOut + (warp & 3) * Cfg::kOutWarpBytes;
     // Columns 8u .. 8u+7 of the lane's row are 16-byte unit u%8 of panel u/8; unit x of row r sits at x ^ (r%8).
     auto out_row = [&](int u) { return out_stage + (u >> 3) * (32 * 128) + lane * 128 + ((u & 7) ^ (lane & 7)) * 16; };
-    constexpr int kCols = Cfg::kEpilogueCols;
+    constexpr int kCols = kShort ? 16 : Cfg::kEpilogueCols;
     // Bit s: phase parity of stage s's barriers. The stages share one copy of this code (rolled loops, state in bit
     // masks): with copies for both and the epilogue in four places it was 38 KB, mostly run from cold instructions.
     uint32_t par_l = 0, par_o = 0;

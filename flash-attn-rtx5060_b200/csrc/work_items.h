@@ -50,18 +50,29 @@ inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
 // (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
 // the epilogue merges two outputs), but there are twice as many items of half the length.
 // - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
-//   one wave. B2 H16 N4096 d128: 3.46 waves of 32 steps, 277 -> 255 us; 8 heads of 333 rows: 14.3 -> 12.6 us.
-// - Under a causal mask items are handed out longest first and a partial wave costs little; but with few of them the
-//   longest one sets the time. All are split while a CTA has at most half an item, or at most 7/4 items that are also
-//   at most a seventh of a head's pairs (where sequences are short, the fill and drain of an item weigh more). The same
-//   rule serves a window bounded on one side without a causal mask, whose items differ likewise. (d64 us, pairs against
-//   singles; heads x rows: 20x1024 20.5/18.4, 30x1024 21.1/23.4, 14x2048 33.2/29.8, 20x2048 36.7/34.8,
-//   26x2048 43.6/43.9, 8x4096 59.4/47.8, 16x4096 81.1/75.0, 8x8192 150/120, 4x16384 289/210; d128: 8x4096 63.5/57.1,
-//   16x4096 87.6/87.0, 8x8192 164/150; 32x2048 and 24x4001, with 1.7 and 2.6 items per CTA, lose 10-25 %). Singles over
-//   pairs with ALiBi, log-sum-exp and dropout, where the rule splits: 0.75-0.95, 0.79-1.01, 0.76-1.03 (20x1024 to
-//   4x16384, both head dims; the largest at d128 16x4096), and at d64 30x1024, where it does not, 1.11, 1.05, 1.10.
-inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, int window_left, int window_right,
-                                int num_sms) {
+//   one wave. 32x4096 d128: 3.46 waves of 32 steps, 246 -> 220 us; 40x1000 d64 31.3 -> 25.3 us.
+// - Under a causal mask items are handed out longest first, and what decides is how they fill the waves. Let r be the
+//   pairs per CTA (tiles / 2, so that an unfilled last pair counts half). Up to r = 1 pairs are one wave that lasts as
+//   long as the longest of them; singles are two waves of half the length, which pays off while they fill little of the
+//   second or a head has many pairs of different lengths. From r = 1 on pairs need a second wave and singles balance
+//   better, until there are so many items of either kind that balance matters less than the cost of a single. Below, the
+//   lines in percent of r by a head's tiles t. The same rule serves a window bounded on one side without a causal mask,
+//   whose items differ likewise. Time of pairs over singles, d64 / d128 (heads x rows; r):
+//   20x640 (0.3) 1.03 / 1.08, 32x640 (0.5) 0.85 / 0.92, 28x768 (0.6) 1.04 / 1.02, 36x768 (0.7) 0.96 / 1.03, 20x896 (0.5)
+//   1.12 / 1.14, 28x896 (0.7) 0.89 / 1.03, 24x1000 (0.6) 1.11 / 1.09, 32x1000 (0.9) 0.94 / 1.03, 40x1024 (1.1) 1.09 / 1.12,
+//   60x1024 (1.6) 0.95 / 1.01, 24x1280 (0.8) 1.05 / 1.08, 32x1280 (1.1) 1.14 / 1.19, 48x1280 (1.6) 1.01 / 1.03, 24x1536
+//   (1.0) 1.08 / 1.08, 32x1536 (1.3) 1.15 / 1.16, 48x1536 (1.9) 0.96 / 1.00, 22x2048 (1.2) 1.24 / 1.26, 36x2048 (1.9) 1.05
+//   / 1.05, 48x2048 (2.6) 0.92 / 0.95, 20x3000 (1.6) 1.10 / 1.11, 26x3000 (2.1) 0.98 / 0.99, 18x4096 (1.9) 1.07 / 1.05,
+//   24x4096 (2.6) 0.92 / 0.93, 10x8192 (2.2) 1.16 / 1.08, 14x8192 (3.0) 0.98 / 0.94, 6x16384 (2.6) 1.11 / 1.01, 8x16384
+//   (3.5) 1.00 / 0.98, 4x32768 (3.5) 1.03 / 1.05. With dropout 30x768 1.08 / 1.06, 40x1024 1.11 / 1.10, 36x1536 1.14 / 1.10,
+//   32x2048 1.14 / 1.12.
+// - With ALiBi, whose tiles cost more and whose cut tiles go through code of their own, all are split while a CTA has at
+//   most half an item, or at most 7/4 items that are also at most a seventh of a head's pairs: 8x1024 1.45 / 1.44, 18x1024
+//   1.13 / 1.14, 8x4096 1.17 / 1.18, 16x4096 1.05 / 1.09, 4x16384 1.34 / 1.36 are, 40x1024 0.90 / 0.93, 26x2048 0.97 / 1.02,
+//   36x1536 0.91 / 0.93 are not.
+inline long long pairs_to_split(long long heads, int num_q_pairs, int seqlen, int window_left, int window_right,
+                                int num_sms, bool alibi) {
+  const long long pairs = heads * num_q_pairs;
   if (seqlen <= kBlockM || pairs >= (1 << 30)) return 0;
   const bool even = (window_left < 0 && window_right < 0) || (window_left >= 0 && window_right >= 0 &&
                                                                window_left < seqlen / 4 && window_right < seqlen / 4);
@@ -69,8 +80,16 @@ inline long long pairs_to_split(long long pairs, int num_q_pairs, int seqlen, in
     const long long tail = pairs % num_sms;
     return 2 * tail <= num_sms ? tail : 0;
   }
-  const bool few = 4 * pairs <= 7LL * num_sms && 7 * pairs <= (long long)num_q_pairs * num_sms;
-  return few || 2 * pairs <= num_sms ? pairs : 0;
+  if (alibi) {
+    const bool few = 4 * pairs <= 7LL * num_sms && 7 * pairs <= (long long)num_q_pairs * num_sms;
+    return few || 2 * pairs <= num_sms ? pairs : 0;
+  }
+  const int t = (seqlen + kBlockM - 1) / kBlockM;
+  const long long r100 = 50 * heads * t / num_sms;
+  constexpr int kOneWave[] = {61, 50, 66, 64, 85, 80};  // t = 6 .. 11
+  const int one_wave = t <= 5 ? 50 : t >= 12 ? 100 : kOneWave[t - 6];
+  const int most = t < 8 ? 0 : t < 10 ? 135 : t < 12 ? 160 : t < 14 ? 175 : t < 48 ? 200 : t < 96 ? 240 : t < 192 ? 280 : 350;
+  return r100 <= one_wave || (r100 > 100 && r100 <= most) ? pairs : 0;
 }
 
 // Whether a launch takes the kernel's short build: q tiles that see few kv tiles, most of all where some of them are cut,
@@ -109,7 +128,7 @@ inline void set_work_items(FwdParams* p, int head_dim, int num_sms, long long fi
   const long long all = total_heads * nq, last = first_head + p->bh;
   const int pairs = p->bh * nq, group_all = group(total_heads);
   p->head_group = group(p->bh);
-  long long split = pairs_to_split(all, nq, p->seqlen, wl, wr, num_sms);
+  long long split = pairs_to_split(total_heads, nq, p->seqlen, wl, wr, num_sms, p->alibi_slopes != nullptr);
   if (split > 0 && split < all && group_all > 1) {
     if (group_all < total_heads) {
       split = 0;

@@ -175,3 +175,18 @@ def test_item_hand_over_ends_for_every_claim_order(wi, shape):
             assert ring_ends([g["steps"] > 0 for g in pub])
             assert all(g["steps"] > 0 for g in pub)
             assert [g["item"] for g in pub] == [i for i in [first] + [i for i in order if i != first] if i not in row_less]
+
+
+@pytest.mark.parametrize("heads,n,causal,wl,wr,split", [
+    (37, 512, True, -1, -1, True), (38, 512, True, -1, -1, False),          # half a pair per CTA
+    (28, 768, True, -1, -1, True), (36, 768, True, -1, -1, False),
+    (24, 1000, True, -1, -1, True), (32, 1024, True, -1, -1, False),        # one wave of pairs against two of singles
+    (40, 1024, True, -1, -1, True), (60, 1024, True, -1, -1, False),        # two waves of pairs
+    (36, 2048, True, -1, -1, True), (40, 2048, True, -1, -1, False), (36, 2048, False, -1, 0, True),
+    (10, 8192, True, -1, -1, True), (12, 8192, True, -1, -1, False), (1, 32768, True, -1, -1, True),
+    (8, 128, True, -1, -1, False),                                          # one tile
+])
+def test_which_launches_take_their_pairs_apart(wi, heads, n, causal, wl, wr, split):
+    launch = Launch(wi, heads, n, causal=causal, wl=wl, wr=wr)
+    pairs = heads * -(-n // 256)
+    assert launch.items == pairs * (2 if split else 1) and launch.pair_items == (0 if split else pairs)
