@@ -80,7 +80,7 @@ struct DeviceState {
   unsigned long long slot_stream[kSchedSlots] = {};  // the id of that launch's stream
   bool slot_used[kSchedSlots] = {};
   unsigned long long acquired_by = 0;  // the stream id of the launch between sched_acquire and sched_release
-  bool attr_set[22] = {};
+  bool attr_set[28] = {};
 };
 
 // Hands out the scheduler words for one launch on `st`. Call with s->mu held; `*slot_out` is passed to
@@ -249,10 +249,9 @@ int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMa
                          const CUtensorMap& mo,
                          const fa::FwdParams& p, cudaStream_t st) {
   using Cfg = fa::PersistentCfg<D>;
-  // attribute slots 2..5, 8..15 and 16..21: one per instantiation
-  constexpr int slot = (kShort ? (kDropout ? 20 : kLse ? 18 : 16) : kDropout ? 12 : kLse ? 8 : 2) + (kAlibi ? 2 : 0) +
+  // attribute slots 2..5, 8..15 and 16..27: one per instantiation
+  constexpr int slot = (kShort ? (kDropout ? 24 : kLse ? 20 : 16) : kDropout ? 12 : kLse ? 8 : 2) + (kAlibi ? 2 : 0) +
                        (D == 64 ? 0 : 1);
-  static_assert(!(kShort && kAlibi), "the short build has no ALiBi");
   constexpr auto kernel = fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout, kShort>;
   int rc = ensure_smem_attr(s, slot, kernel, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
@@ -273,10 +272,14 @@ int launch_persistent(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& 
                       const CUtensorMap& mo,
                       const fa::FwdParams& p, cudaStream_t st, bool dropout) {
   const bool alibi = p.alibi_slopes != nullptr, lse = p.lse != nullptr;
-  if (!alibi && fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right))
-    return dropout ? launch_persistent_as<D, false, false, true, true>(s, mq, mk, mv, mo, p, st)
-           : lse   ? launch_persistent_as<D, false, true, false, true>(s, mq, mk, mv, mo, p, st)
-                   : launch_persistent_as<D, false, false, false, true>(s, mq, mk, mv, mo, p, st);
+  if (fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right, alibi)) {
+    if (dropout) return alibi ? launch_persistent_as<D, true, false, true, true>(s, mq, mk, mv, mo, p, st)
+                              : launch_persistent_as<D, false, false, true, true>(s, mq, mk, mv, mo, p, st);
+    if (alibi) return lse ? launch_persistent_as<D, true, true, false, true>(s, mq, mk, mv, mo, p, st)
+                          : launch_persistent_as<D, true, false, false, true>(s, mq, mk, mv, mo, p, st);
+    return lse ? launch_persistent_as<D, false, true, false, true>(s, mq, mk, mv, mo, p, st)
+               : launch_persistent_as<D, false, false, false, true>(s, mq, mk, mv, mo, p, st);
+  }
   if (dropout) return alibi ? launch_persistent_as<D, true, false, true>(s, mq, mk, mv, mo, p, st)
                             : launch_persistent_as<D, false, false, true>(s, mq, mk, mv, mo, p, st);
   if (alibi) return lse ? launch_persistent_as<D, true, true>(s, mq, mk, mv, mo, p, st)
@@ -804,7 +807,7 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   p.status_per_launch = 1;  // the launch writes its own verdict into the status word
   if (captured && (e = cudaMemsetAsync(p.sched, 0, 2 * sizeof(int), st)) != cudaSuccess)
     return fail_cuda("cudaMemsetAsync(scratch slot)", e);
-  if (fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right))
+  if (fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right, false))
     rc = head_dim == 64 ? launch_persistent_noalloc<64, true>(s, mq, mk, mv, mo, p, st, !captured)
                         : launch_persistent_noalloc<128, true>(s, mq, mk, mv, mo, p, st, !captured);
   else

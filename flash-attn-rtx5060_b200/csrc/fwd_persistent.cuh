@@ -199,8 +199,9 @@ __device__ __forceinline__ void dropout_mask(uint32_t* pk, const FwdParams& p, c
 // how little code there is: cut tiles are blanked in tensor memory by a small loop and go through the same body as all
 // others, the row max comes before any exponential (no second copy of the first ones), the issuer has no rounds of its
 // own for the inside of an item, and at head_dim 128, where these launches are not bound by the exponentials, none are
-// taken on the FMA pipe. Without ALiBi, whose body differs for cut tiles. (With a body per kind of tile, one of them
-// blanked: nothing gained. In long sequences one body costs 3-6 %.)
+// taken on the FMA pipe. ALiBi comes here under a causal mask only: a key left of the diagonal has a bias that is linear in
+// the column, and what lies right of it is hidden. (With a body per kind of tile, one of them blanked: nothing gained. In
+// long sequences one body costs 3-6 %.)
 template <int D, bool kAlibi, bool kLse = false, bool kDropout = false, bool kShort = false>
 __global__ void __launch_bounds__(512, 1)
 fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,

@@ -65,13 +65,10 @@ inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
 //   / 1.05, 48x2048 (2.6) 0.92 / 0.95, 20x3000 (1.6) 1.10 / 1.11, 26x3000 (2.1) 0.98 / 0.99, 18x4096 (1.9) 1.07 / 1.05,
 //   24x4096 (2.6) 0.92 / 0.93, 10x8192 (2.2) 1.16 / 1.08, 14x8192 (3.0) 0.98 / 0.94, 6x16384 (2.6) 1.11 / 1.01, 8x16384
 //   (3.5) 1.00 / 0.98, 4x32768 (3.5) 1.03 / 1.05. With dropout 30x768 1.08 / 1.06, 40x1024 1.11 / 1.10, 36x1536 1.14 / 1.10,
-//   32x2048 1.14 / 1.12.
-// - With ALiBi, whose tiles cost more and whose cut tiles go through code of their own, all are split while a CTA has at
-//   most half an item, or at most 7/4 items that are also at most a seventh of a head's pairs: 8x1024 1.45 / 1.44, 18x1024
-//   1.13 / 1.14, 8x4096 1.17 / 1.18, 16x4096 1.05 / 1.09, 4x16384 1.34 / 1.36 are, 40x1024 0.90 / 0.93, 26x2048 0.97 / 1.02,
-//   36x1536 0.91 / 0.93 are not.
+//   32x2048 1.14 / 1.12; with ALiBi 28x768 1.04 / 1.06, 40x1024 1.07 / 1.11, 32x1536 1.15 / 1.15, 34x2048 1.04 / 1.07, 12x4096
+//   1.31 / 1.29, 10x8192 1.05 / 1.08.
 inline long long pairs_to_split(long long heads, int num_q_pairs, int seqlen, int window_left, int window_right,
-                                int num_sms, bool alibi) {
+                                int num_sms) {
   const long long pairs = heads * num_q_pairs;
   if (seqlen <= kBlockM || pairs >= (1 << 30)) return 0;
   const bool even = (window_left < 0 && window_right < 0) || (window_left >= 0 && window_right >= 0 &&
@@ -79,10 +76,6 @@ inline long long pairs_to_split(long long heads, int num_q_pairs, int seqlen, in
   if (even) {
     const long long tail = pairs % num_sms;
     return 2 * tail <= num_sms ? tail : 0;
-  }
-  if (alibi) {
-    const bool few = 4 * pairs <= 7LL * num_sms && 7 * pairs <= (long long)num_q_pairs * num_sms;
-    return few || 2 * pairs <= num_sms ? pairs : 0;
   }
   const int t = (seqlen + kBlockM - 1) / kBlockM;
   const long long r100 = 50 * heads * t / num_sms;
@@ -104,8 +97,12 @@ inline long long pairs_to_split(long long heads, int num_q_pairs, int seqlen, in
 //   window (left, right) over 4x16x4096   256,0 1.09 / 1.02, 512,0 1.01 / 1.01, 768,0 0.99 / 1.00, 1024,0 0.98 / 0.96,
 //                  128,128 1.10 / 1.03, 256,256 1.04 / 1.04, 512,512 1.02 / 1.00
 // With dropout 16x4x256 1.24, 16x4x1024 1.07 / 1.10, 16x4x2048 1.02 / 1.06.
-inline bool short_items(int seqlen, int causal, int window_left, int window_right) {
+// With ALiBi the one body takes the bias as linear in the column, which holds where all visible keys lie on one side: under
+// a causal mask. A cut tile of the other build then costs more, too: 8x16x512 1.25 / 1.23, 8x16x1024 1.13 / 1.17, 4x16x2048
+// 1.08 / 1.08, 8x4096 1.15 / 1.12, 2x16x4096 1.01 / 1.04, 4x16x4096 0.98 / 1.04, 2x16x6144 0.96 / 1.02.
+inline bool short_items(int seqlen, int causal, int window_left, int window_right, bool alibi) {
   const int wr = eff_window_right(causal, window_right);
+  if (alibi) return causal && window_left < 0 && seqlen <= 32 * kBlockN;
   if (window_left < 0 && wr < 0) return seqlen <= (seqlen % kBlockN ? 10 : 5) * kBlockN;
   if (seqlen <= 20 * kBlockN) return true;
   return window_left >= 0 && wr >= 0 && wr <= 4 * kBlockN && window_left <= 4 * kBlockN - wr;
@@ -128,7 +125,7 @@ inline void set_work_items(FwdParams* p, int head_dim, int num_sms, long long fi
   const long long all = total_heads * nq, last = first_head + p->bh;
   const int pairs = p->bh * nq, group_all = group(total_heads);
   p->head_group = group(p->bh);
-  long long split = pairs_to_split(total_heads, nq, p->seqlen, wl, wr, num_sms, p->alibi_slopes != nullptr);
+  long long split = pairs_to_split(total_heads, nq, p->seqlen, wl, wr, num_sms);
   if (split > 0 && split < all && group_all > 1) {
     if (group_all < total_heads) {
       split = 0;

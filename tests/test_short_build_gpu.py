@@ -60,6 +60,34 @@ def test_both_builds_at_the_lines_between_them(pkg, d, n, causal, wl, wr):
         assert torch.equal(out[:, :, 0], v[:, :, 0])        # one visible key: its value bit for bit
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n,causal,wl", [(1, True, -1), (127, True, -1), (129, True, -1), (1000, True, -1), (4096, True, -1),
+                                         (4100, True, -1), (1000, True, 300), (1000, False, -1)])
+def test_alibi_in_both_builds(pkg, d, n, causal, wl):
+    import torch
+
+    q, k, v = (torch.from_numpy(a).cuda() for a in make_inputs(n + d, 1, 4, n, d))
+    slopes = torch.tensor([0.5, 2.0 ** -6, 0.0, -0.01], device="cuda")  # no bias, and one that grows with the distance
+    i = torch.arange(n, device="cuda")
+    gap = i[None, :] - i[:, None]
+    s = q.double() @ k.double().transpose(-1, -2) / math.sqrt(d) - slopes.double()[:, None, None] * gap.abs()
+    hidden = (gap > 0) & causal
+    if wl >= 0:
+        hidden |= gap < -wl
+    s.masked_fill_(hidden, -math.inf)
+    want, want_lse = torch.softmax(s, dim=-1) @ v.double(), torch.logsumexp(s, dim=-1)
+    kw = dict(causal=causal, window_left=wl, alibi_slopes=slopes)
+    out = pkg.attention_forward(q, k, v, **kw)
+    out2, lse = pkg.attention_forward(q, k, v, return_lse=True, **kw)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    for o in (out, out2):
+        assert (o.double() - want).abs().max().item() < 4e-3
+        assert ((o.double() - want).norm() / want.norm()).item() < 4e-4
+    assert (lse.double() - want_lse).abs().max().item() < 1e-4  # biases of up to 60, in fp32
+    if causal:
+        assert torch.equal(out[:, :, 0], v[:, :, 0])
+
+
 @pytest.mark.parametrize("n,d,causal", [(2500, 64, True), (2700, 64, True), (1200, 128, False), (1400, 128, False)])
 def test_dropout_in_both_builds(pkg, ob, n, d, causal):
     import torch
@@ -69,6 +97,12 @@ def test_dropout_in_both_builds(pkg, ob, n, d, causal):
     pkg.check(torch.cuda.current_stream().cuda_stream)
     mx, mean, nans = ob.abs_error(out.cpu().numpy(), ob.attention_dropout(q, k, v, 0.2, 5, causal=causal))
     assert nans == 0 and mx <= 2.5e-3 and mean <= 2.5e-4, (mx, mean, nans)
+    slopes = np.array([0.03125], np.float32)
+    out = pkg.attention_forward(*(torch.from_numpy(a).cuda() for a in (q, k, v)), causal=causal, dropout_p=0.2, seed=5,
+                                alibi_slopes=torch.from_numpy(slopes).cuda())
+    want = ob.attention_dropout(q, k, v, 0.2, 5, causal=causal, alibi_slopes=slopes)
+    mx, mean, nans = ob.abs_error(out.cpu().numpy(), want)
+    assert nans == 0 and mx <= 4e-3 and mean <= 3e-4, (mx, mean, nans)
 
 
 def test_the_line_does_not_depend_on_the_number_of_heads(pkg):
