@@ -80,7 +80,7 @@ struct DeviceState {
   unsigned long long slot_stream[kSchedSlots] = {};  // the id of that launch's stream
   bool slot_used[kSchedSlots] = {};
   unsigned long long acquired_by = 0;  // the stream id of the launch between sched_acquire and sched_release
-  bool attr_set[28] = {};
+  bool attr_set[29] = {};
 };
 
 // Hands out the scheduler words for one launch on `st`. Call with s->mu held; `*slot_out` is passed to
@@ -244,15 +244,15 @@ cudaError_t launch_overlapped(K kernel, int grid, int threads, int smem, cudaStr
   return cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mo, p);
 }
 
-template <int D, bool kAlibi, bool kLse, bool kDropout = false, bool kShort = false>
+template <int D, bool kAlibi, bool kLse, bool kDropout = false, bool kShort = false, bool kOwnP = false>
 int launch_persistent_as(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                          const CUtensorMap& mo,
                          const fa::FwdParams& p, cudaStream_t st) {
   using Cfg = fa::PersistentCfg<D>;
-  // attribute slots 2..5, 8..15 and 16..27: one per instantiation
-  constexpr int slot = (kShort ? (kDropout ? 24 : kLse ? 20 : 16) : kDropout ? 12 : kLse ? 8 : 2) + (kAlibi ? 2 : 0) +
+  // attribute slots 2..5, 8..15, 16..27 and 28: one per instantiation
+  constexpr int slot = kOwnP ? 28 : (kShort ? (kDropout ? 24 : kLse ? 20 : 16) : kDropout ? 12 : kLse ? 8 : 2) + (kAlibi ? 2 : 0) +
                        (D == 64 ? 0 : 1);
-  constexpr auto kernel = fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout, kShort>;
+  constexpr auto kernel = fa::fwd_persistent_kernel<D, kAlibi, kLse, kDropout, kShort, kOwnP>;
   int rc = ensure_smem_attr(s, slot, kernel, Cfg::kSmemBytes);
   if (rc != FA_OK) return rc;
   fa::FwdParams pp = p;
@@ -277,6 +277,9 @@ int launch_persistent(DeviceState* s, const CUtensorMap& mq, const CUtensorMap& 
                               : launch_persistent_as<D, false, false, true, true>(s, mq, mk, mv, mo, p, st);
     if (alibi) return lse ? launch_persistent_as<D, true, true, false, true>(s, mq, mk, mv, mo, p, st)
                           : launch_persistent_as<D, true, false, false, true>(s, mq, mk, mv, mo, p, st);
+    if constexpr (D == 64)
+      if (!lse && fa::own_p_columns(p))
+        return launch_persistent_as<D, false, false, false, true, true>(s, mq, mk, mv, mo, p, st);
     return lse ? launch_persistent_as<D, false, true, false, true>(s, mq, mk, mv, mo, p, st)
                : launch_persistent_as<D, false, false, false, true>(s, mq, mk, mv, mo, p, st);
   }
@@ -326,7 +329,7 @@ int host_pipe(HostPipe** out) {
 // Scratch of flash_forward_noalloc: a fixed block in the library's own device image instead of
 // memory obtained from cudaMalloc. kNoAllocSlots slots of eight ints each:
 //   word 0 status (set non-zero when a bounded wait inside the kernel gave up),
-//   words 2-7 three pairs for the persistent kernel: work counter and finished-CTA counter.
+//   words 2-7 three pairs for the persistent kernel: work counter and the count of producers that have run out of items.
 // 512 bytes per GPU that loads the library, held until the process exits.
 // A launch finds its pair at zero and leaves it at zero. A caller that lets two launches on one slot overlap, which is
 // not allowed, may leave a pair off, and a launch that started from such a pair would skip work without knowing. So the
@@ -346,7 +349,7 @@ struct NoAllocState {
   int num_sms = 0;
   int* scratch = nullptr;  // device address of g_noalloc_scratch on this device
   unsigned launches[kNoAllocSlots] = {};  // per slot: the next launch takes pair launches % kSlotPairs
-  bool attr_set[4] = {};
+  bool attr_set[5] = {};
 };
 NoAllocState g_noalloc[kMaxDevices];
 
@@ -375,15 +378,15 @@ int noalloc_state(NoAllocState** out) {
   return FA_OK;
 }
 
-template <int D, bool kShort>
+template <int D, bool kShort, bool kOwnP = false>
 int launch_persistent_noalloc(NoAllocState* s, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                               const CUtensorMap& mo,
                               fa::FwdParams p, cudaStream_t st, bool early) {
   using Cfg = fa::PersistentCfg<D>;
-  constexpr auto kernel = fa::fwd_persistent_kernel<D, false, false, false, kShort>;
+  constexpr auto kernel = fa::fwd_persistent_kernel<D, false, false, false, kShort, kOwnP>;
   {
     std::lock_guard<std::mutex> lk(s->mu);
-    bool& done = s->attr_set[(D == 64 ? 0 : 1) + (kShort ? 2 : 0)];
+    bool& done = s->attr_set[kOwnP ? 4 : (D == 64 ? 0 : 1) + (kShort ? 2 : 0)];
     if (!done) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
       if (e != cudaSuccess) return fail_cuda("cudaFuncSetAttribute(MaxDynamicSharedMemorySize)", e);
@@ -808,8 +811,9 @@ int flash_forward_noalloc(const void* q, const void* k, const void* v, void* o, 
   if (captured && (e = cudaMemsetAsync(p.sched, 0, 2 * sizeof(int), st)) != cudaSuccess)
     return fail_cuda("cudaMemsetAsync(scratch slot)", e);
   if (fa::short_items(p.seqlen, p.causal, p.window_left, p.window_right, false))
-    rc = head_dim == 64 ? launch_persistent_noalloc<64, true>(s, mq, mk, mv, mo, p, st, !captured)
-                        : launch_persistent_noalloc<128, true>(s, mq, mk, mv, mo, p, st, !captured);
+    rc = head_dim == 128         ? launch_persistent_noalloc<128, true>(s, mq, mk, mv, mo, p, st, !captured)
+         : fa::own_p_columns(p) ? launch_persistent_noalloc<64, true, true>(s, mq, mk, mv, mo, p, st, !captured)
+                                : launch_persistent_noalloc<64, true>(s, mq, mk, mv, mo, p, st, !captured);
   else
     rc = head_dim == 64 ? launch_persistent_noalloc<64, false>(s, mq, mk, mv, mo, p, st, !captured)
                         : launch_persistent_noalloc<128, false>(s, mq, mk, mv, mo, p, st, !captured);

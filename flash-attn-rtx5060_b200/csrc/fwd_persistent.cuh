@@ -58,12 +58,13 @@ struct PersistentCfg {
   static constexpr int kOffAlpha = kOffOut + 4 * kOutWarpBytes;  // float[2][128]: references of a split item; drop_blocks
   static constexpr int kOffRowSum = kOffAlpha + 2 * kBlockM * 4;   // float[2][128]
   static constexpr int kOffBars = kOffRowSum + 2 * kBlockM * 4;
-  static constexpr int kNumBars = 20 + 2 * kStages;
+  static constexpr int kNumBars = 22 + 2 * kStages;
   static constexpr int kOffMisc = kOffBars + kNumBars * 8;
   static constexpr int kOffGeom = kOffMisc + 16;     // TMEM base, abort flag (+ 8 spare bytes)
   static constexpr int kSmemBytes = kOffGeom + 2 * 64;  // two work-item slots: the item's decoded geometry and its id
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 384;
+  static constexpr uint32_t kOwnPFromS = 320;  // kOwnP: P in columns 320 and 448, beside an O of 64 columns
   // Lazy rescale, in log2 units: a row's reference (the score that its exponentials are taken against) stays where it is
   // until a tile's row max passes it by more than kLazyLog2, so P stays below 2^8, well inside fp16, and l and O, held
   // in fp32, have the room. The key that sets the reference has P = 1 exactly; a key above it has a P rounded to 11 bits,
@@ -202,12 +203,15 @@ __device__ __forceinline__ void dropout_mask(uint32_t* pk, const FwdParams& p, c
 // taken on the FMA pipe. ALiBi comes here under a causal mask only: a key left of the diagonal has a bias that is linear in
 // the column, and what lies right of it is hidden. (With a body per kind of tile, one of them blanked: nothing gained. In
 // long sequences one body costs 3-6 %.)
-template <int D, bool kAlibi, bool kLse = false, bool kDropout = false, bool kShort = false>
+// kOwnP (own_p_columns() in work_items.h; head_dim 64, short build): P has columns of its own instead of S's, and the next
+// score tile is issued ahead of the rest of P.V, so a stage waits for one hand-over and 96 keys' products less per tile.
+template <int D, bool kAlibi, bool kLse = false, bool kDropout = false, bool kShort = false, bool kOwnP = false>
 __global__ void __launch_bounds__(512, 1)
 fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO,
                       const FwdParams p) {
   using Cfg = PersistentCfg<D>;
+  static_assert(!kOwnP || (D == 64 && kShort), "columns of P's own lie beside an O of 64 columns");
   extern __shared__ __align__(1024) uint8_t smem[];
 
   const int tid = threadIdx.x;
@@ -236,6 +240,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   uint64_t* item_empty = bars + 18;   // [2] all roles -> producer: id slot read
   uint64_t* kv_full = bars + 20;      // [kStages] TMA -> MMA
   uint64_t* kv_empty = bars + 20 + Cfg::kStages;  // [kStages] MMA -> TMA
+  uint64_t* p_empty = bars + 20 + 2 * Cfg::kStages;  // [2] MMA -> softmax: P.V of the tile complete (kOwnP)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   // [2][16]: ItemGeom of the published item in words 0..11, its id (-1: no more items) in word 12, `split` in word 13
@@ -257,6 +262,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       mbar_init(&o_empty[s], 4);
       mbar_init(&l_ready[s], 4);
       mbar_init(&o_full[s], 1);
+      if (kOwnP) mbar_init(&p_empty[s], 1);
       mbar_init(&item_full[s], 1);
       mbar_init(&item_empty[s], kItemReaders);
     }
@@ -338,6 +344,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const float sl2 = kAlibi ? 1.f : p.scale_log2;
     const uint64_t scale2 = f2_pack(sl2, sl2);
     const uint32_t tO = tmem_addr(tmem_base, lane_base, s == 0 ? Cfg::kColO0 : Cfg::kColO1);
+    const uint32_t tP = tS + (kOwnP ? Cfg::kOwnPFromS : 0);
     uint32_t par_s = 0;  // parity of the next s_full phase
     griddep_wait();
     const float lazy = Cfg::kLazyLog2 / sl2;
@@ -504,8 +511,13 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             }
             m_limit = l_run == 0.f && m_new == -INFINITY ? -INFINITY : m_used + lazy;
             l_run *= alpha;
-            // s_full for this tile was committed behind the previous tile's P.V, so O is at rest here.
+            // s_full for this tile was committed behind the previous tile's P.V (kOwnP: behind its first 96 keys), so O is
+            // at rest here.
             if (kv0 != kv_first && __any_sync(0xffffffffu, alpha != 1.f)) {
+              if (kOwnP) {
+                ok &= mbar_wait(&p_empty[s], par_s, abort_flag);
+                tc_fence_after();
+              }
 #pragma unroll 1
               for (int c = 0; c < D / 16; ++c) {
                 uint32_t r[16];
@@ -532,18 +544,22 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           const uint64_t negms2 = f2_pack(neg_ms, neg_ms);
           exp_tile<16, kPoly ? Cfg::kPolyOf1 : 0>(sc + 32, scale2, negms2, pk0 + 16, lsum_a, lsum_b);
           if (kDropout) dropout_mask<4>(pk0, p, drow, drop_blocks);  // the row sum keeps every exponential
-          tmem_st32(tS + 0, pk0);
+          tmem_st32(tP + 0, pk0);  // (kOwnP: s_full says that the previous tile's first 96 keys have been read)
           uint32_t pk1[16], pk2[16];
           exp_tile<16, kPoly ? Cfg::kPolyOf2 : 0>(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
           if (kDropout) dropout_mask<2>(pk1, p, drow, drop_blocks + 4);
-          tmem_st16(tS + 32, pk1);
+          tmem_st16(tP + 32, pk1);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
           mbar_arrive_lane0(&p_full[s], lane);  // P of keys 0..95 is in TMEM
           exp_tile<16, kPoly ? Cfg::kPolyOf3 : 0>(sc + 96, scale2, negms2, pk2, lsum_a, lsum_b);
           if (kDropout) dropout_mask<2>(pk2, p, drow, drop_blocks + 6);
-          tmem_st16(tS + 48, pk2);
+          if (kOwnP) {
+            ok &= mbar_wait(&p_empty[s], par_s, abort_flag);
+            tc_fence_after();
+          }
+          tmem_st16(tP + 48, pk2);
           float l0, l1;
           f2_unpack(f2_add(lsum_a, lsum_b), l0, l1);
           l_run += l0 + l1;
@@ -767,25 +783,32 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           const int alo = s ? a.lo[1] : a.lo[0], ahi = s ? a.hi[1] : a.hi[0];
           const int blo = s ? b.lo[1] : b.lo[0], bhi = s ? b.hi[1] : b.hi[0];
           const uint32_t tS = tmem_base + (s ? Cfg::kColS1 : Cfg::kColS0);
-          if (j >= alo && j < ahi) {  // O_s += P_s V
-            const uint32_t tO = tmem_base + (s ? Cfg::kColO1 : Cfg::kColO0);
+          const uint32_t tP = tS + (kOwnP ? Cfg::kOwnPFromS : 0);
+          auto rest_of_pv = [&](uint32_t tO, uint32_t slot, uint32_t vdesc) {
+            ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
+            par_p ^= 1u << s;
+            tc_fence_after();
+            umma_pv32(tO, tP + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
+            umma_commit_warp(&kv_empty[slot], a.split || s == 1 || j < a.lo[1] || j >= a.hi[1]);
+            if (kOwnP) umma_commit_warp(&p_empty[s]);
+            umma_commit_warp(&o_full[s]);
+          };
+          const bool has_pv = j >= alo && j < ahi;
+          uint32_t tO = 0, slot_pv = 0, vdesc_pv = 0;
+          if (has_pv) {  // O_s += P_s V
+            tO = tmem_base + (s ? Cfg::kColO1 : Cfg::kColO0);
             const uint32_t pv = end - ((a.split && s == 0 && j < a.hi[1]) ? 2 : 1);
-            const uint32_t slot = pv % Cfg::kStages;
-            const uint32_t vdesc = vdesc0 + ((kv_addr + slot * Cfg::kTileBytes) >> 4);
-            ok &= mbar_wait(&kv_full[slot], (pv / Cfg::kStages) & 1, abort_flag);
+            slot_pv = pv % Cfg::kStages;
+            vdesc_pv = vdesc0 + ((kv_addr + slot_pv * Cfg::kTileBytes) >> 4);
+            ok &= mbar_wait(&kv_full[slot_pv], (pv / Cfg::kStages) & 1, abort_flag);
             if (j == alo) {  // the previous item's O has been read
               ok &= mbar_wait(&o_empty[s], (par_e >> s) & 1, abort_flag);
               par_e ^= 1u << s;
             }
             ok &= mbar_wait(&p_full[s], (par_p >> s) & 1, abort_flag);
             tc_fence_after();
-            umma_pv96(tO, tS, vdesc, kDescHi, idesc_pv, j > alo ? 1u : 0u);
-            ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
-            par_p ^= 1u << s;
-            tc_fence_after();
-            umma_pv32(tO, tS + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
-            umma_commit_warp(&kv_empty[slot], a.split || s == 1 || j < a.lo[1] || j >= a.hi[1]);
-            umma_commit_warp(&o_full[s]);
+            umma_pv96(tO, tP, vdesc_pv, kDescHi, idesc_pv, j > alo ? 1u : 0u);
+            if (!kOwnP) rest_of_pv(tO, slot_pv, vdesc_pv);
           }
           if (blo == 0 && bhi > 0) {  // S_s = Q_s K^T
             const uint32_t pk = end + (b.split ? s : 0);
@@ -803,6 +826,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             umma_commit_warp(&kv_empty[slot], b.split || s == 1 || b.lo[1] > 0 || b.hi[1] == 0);
             umma_commit_warp(&q_empty[s], bhi == 1);
           }
+          if (kOwnP && has_pv) rest_of_pv(tO, slot_pv, vdesc_pv);
         }
       };
       ItemGeom g;
@@ -852,13 +876,25 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const bool k_seen = !kSplit && (s == 1) && (kInterior || (j + 1 >= g.lo[0] && j + 1 < g.hi[0]));
             const uint32_t colS = (s == 0) ? Cfg::kColS0 : Cfg::kColS1;
             const uint32_t colO = (s == 0) ? Cfg::kColO0 : Cfg::kColO1;
+            const uint32_t colP = colS + (kOwnP ? Cfg::kOwnPFromS : 0);
+            auto rest_of_pv = [&](uint32_t slot, uint32_t vdesc) {
+              ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
+              par_p ^= 1u << s;
+              tc_fence_after();
+              umma_pv32(tmem_base + colO, tmem_base + colP + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
+              if (!kInterior || !other_j) umma_commit_warp(&kv_empty[slot], !other_j);
+              if (kOwnP) umma_commit_warp(&p_empty[s]);
+              if (!kInterior) umma_commit_warp(&o_full[s], j + 1 == g.hi[s]);
+            };
+            uint32_t slot_pv = 0, vdesc_pv = 0;
             if (act_j) {  // O_s += P_s(j) V_j, 96 keys and 32 as P arrives
               if (kSplit) {
                 slot_v = slot_k;
                 par_v = par_k;
                 advance(slot_k, par_k, 1);
               }
-              const uint32_t vdesc = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
+              slot_pv = slot_v;
+              vdesc_pv = vdesc0 + ((kv_addr + slot_v * Cfg::kTileBytes) >> 4);
               if (!kInterior && !v_seen) ok &= mbar_wait(&kv_full[slot_v], par_v, abort_flag);
               if (!kInterior && j == g.lo[s]) {  // the previous item's O has been read
                 ok &= mbar_wait(&o_empty[s], (par_e >> s) & 1, abort_flag);
@@ -866,13 +902,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               }
               ok &= mbar_wait(&p_full[s], (par_p >> s) & 1, abort_flag);
               tc_fence_after();
-              umma_pv96(tmem_base + colO, tmem_base + colS, vdesc, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
-              ok &= mbar_wait(&p_full2[s], (par_p >> s) & 1, abort_flag);
-              par_p ^= 1u << s;
-              tc_fence_after();
-              umma_pv32(tmem_base + colO, tmem_base + colS + 48, vdesc + 6 * (2048 >> 4), kDescHi, idesc_pv);
-              if (!kInterior || !other_j) umma_commit_warp(&kv_empty[slot_v], !other_j);
-              if (!kInterior) umma_commit_warp(&o_full[s], j + 1 == g.hi[s]);
+              umma_pv96(tmem_base + colO, tmem_base + colP, vdesc_pv, kDescHi, idesc_pv, (kInterior || j > g.lo[s]) ? 1u : 0u);
+              if (!kOwnP) rest_of_pv(slot_pv, vdesc_pv);
             }
             if (act_n) {  // S_s = Q_s K_{j+1}^T
               if (!kInterior && j + 1 == g.lo[s]) {
@@ -893,6 +924,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
               if (!kInterior) umma_commit_warp(&q_empty[s], j + 2 == g.hi[s]);
               if (kSplit) advance(slot_k, par_k, 1);
             }
+            if (kOwnP && act_j) rest_of_pv(slot_pv, vdesc_pv);
           }
         };
         if (g.split) {

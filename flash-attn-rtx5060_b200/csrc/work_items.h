@@ -142,6 +142,22 @@ inline void set_work_items(FwdParams* p, int head_dim, int num_sms, long long fi
   p->num_items = pairs + static_cast<int>(split);
 }
 
+// Whether a plain launch of the short build at head_dim 64 gives P tensor-memory columns of its own (kOwnP in
+// fwd_persistent.cuh; the same bits either way). The turnaround that it saves is worth more than its two further waits and
+// their cold code from about six rounds an item on, and nothing in single q tiles, whose stages have half the rounds. Time
+// of the build without over the one with them (batch x heads x rows):
+//   no mask     16x12x200 0.96, 1x4x512 0.97, 8x16x512 1.00, 16x16x640 1.00 (five tiles), 8x12x700 1.02, 8x12x1000 1.05,
+//               16x12x1200 1.05, 8x16x1250 1.05, 1x8x900 1.00
+//   causal      1x16x1000 0.91, 16x16x256 0.96, 8x16x1024 0.99, 16x16x1280 1.00, 8x16x1500 1.00, 8x16x2048 1.01,
+//               4x16x2048 1.02, 4x16x2560 1.02; with single q tiles 2x16x1800 0.95, 1x32x2048 0.94, 2x12x2300 0.95
+//   window      4x16x4096 left 256 0.97, 4x12x2000 left 128 0.96
+// (In the build for long sequences it gains 0-1 % without a mask, loses 0-2 % under a causal one and 4-6 % with ALiBi.)
+inline bool own_p_columns(const FwdParams& p) {
+  if (p.window_left >= 0 || (!p.causal && p.window_right >= 0)) return false;
+  const int t = (p.seqlen + kBlockN - 1) / kBlockN;
+  return p.causal ? t >= 14 && p.num_items == p.num_pair_items : t >= 6;
+}
+
 // Work item -> geometry. Every role decodes the same item the same way.
 // The kv tiles of an item are walked from the last visible one to the first. Under a causal mask (and for a ragged
 // end) the tiles that carry the per-element predicate then come first, where the pipeline fills anyway, instead of

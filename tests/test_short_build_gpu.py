@@ -114,3 +114,33 @@ def test_the_line_does_not_depend_on_the_number_of_heads(pkg):
     err = (torch.cat(parts, dim=1).float() - whole.float()).abs().max().item()
     assert err <= 2.0 ** -9  # an ulp of outputs of up to 4: pairs of q tiles may be split in the one and not the other
     assert np.isfinite(err)
+
+
+# Plain launches at head_dim 64 give P columns of its own in part of the short build's range (own_p_columns() in
+# csrc/work_items.h); with the log-sum-exp they do not. One arithmetic: the same bits.
+@pytest.mark.parametrize("rising", [False, True])
+@pytest.mark.parametrize("b,h,n,causal", [(1, 1, 641, False), (2, 20, 700, False), (8, 24, 897, False), (1, 3, 1279, False),
+                                          (1, 2, 640, False), (4, 16, 1665, True), (2, 48, 1664, True), (5, 30, 1793, True),
+                                          (3, 32, 2560, True), (1, 16, 2048, True)])
+def test_columns_of_its_own_for_p_change_no_bit(pkg, b, h, n, causal, rising):
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    q, k, v = (torch.randn(b, h, n, 64, device="cuda", generator=g) for _ in range(3))
+    if rising:  # kv runs from the last tile to the first: scores that grow that way move every row's reference in every tile
+        q = q.abs()
+        k = k * 0.1 + torch.linspace(6.0, -1.0, n, device="cuda")[:, None]
+    q, k, v = q.half(), k.half(), v.half()
+    out = pkg.attention_forward(q, k, v, causal=causal)
+    again = pkg.attention_forward(q, k, v, causal=causal)
+    want, _ = pkg.attention_forward(q, k, v, causal=causal, return_lse=True)
+    own = torch.empty_like(q)
+    stream = torch.cuda.current_stream().cuda_stream
+    assert pkg.lib().flash_forward_noalloc(q.data_ptr(), k.data_ptr(), v.data_ptr(), own.data_ptr(), b, h, n, 64, 0.0,
+                                           int(causal), -1, -1, stream, 0, 1) == pkg.FA_OK
+    pkg.check(stream)
+    for o in (out, again, own):
+        assert torch.equal(o, want)
+    exact_out, _ = exact(q[:1, :2], k[:1, :2], v[:1, :2], causal, -1, -1)
+    assert (out[:1, :2].double() - exact_out).abs().max().item() < 4e-3  # as above
