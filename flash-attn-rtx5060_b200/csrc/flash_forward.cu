@@ -671,6 +671,21 @@ size_t flash_forward_host_workspace_bytes(int seqlen, int head_dim, int chunk_he
   return (size_t)2 * 4 * (size_t)chunk_heads * seqlen * head_dim * 2;
 }
 
+// Heads of the next piece of a host call's last chunk, of which `left` remain. The chunks before it overlap each other's
+// uploads, but behind the last upload a whole chunk's kernel and download would still have to run: the chunk is taken in
+// halves, then halves of the rest, down to pieces of 2 MiB a tensor (40 us of upload). us, whole -> in pieces
+// (heads x rows, head_dim, heads per chunk): 32x8192 d128 by 8 causal 4388 -> 4232, not causal 4455 -> 4252; in one
+// chunk 8x8192 1365 -> 1203, 8x32768 6510 -> 4586, 5x8192 d64 496 -> 447, 16x2048 670 -> 637, 8x2048 359 -> 351; pieces
+// of at least 1 MiB 8x2048 370, 64x2048 d64 by 8 1237 against 1231, of 256 KiB 16x1024 d64 207 -> 235; of 3 MiB 16x2048 643.
+// Where the products and not the uploads set the pace a small piece leaves SMs idle: 6x65536 d128 by 2, not causal,
+// 13270 -> 13470 (8x32768 by 4 6035 -> 5468, 4x65536 causal by 2 5966 -> 5978), so many keys a row leave the last of
+// several chunks whole.
+static int last_chunk_piece(int left, size_t head_bytes, bool only_chunk, long long keys_per_row) {
+  if (!only_chunk && keys_per_row > 48 * 1024) return left;
+  const int half = (left + 1) / 2;
+  return (size_t)half * head_bytes < (2u << 20) ? left : half;
+}
+
 int flash_forward_host(const void* q_host, const void* k_host, const void* v_host, void* o_host, int batch,
                        int heads, int seqlen, int head_dim, float softmax_scale, int is_causal, int window_left,
                        int window_right, void* workspace, size_t workspace_bytes, int chunk_heads) {
@@ -697,27 +712,35 @@ int flash_forward_host(const void* q_host, const void* k_host, const void* v_hos
   const char* what = nullptr;  // the CUDA call that failed, if any
 #define FA_TRY(call)                                  \
   if (!what && (e = (call)) != cudaSuccess) what = #call
+  long long keys = is_causal ? (seqlen + 1ll) / 2 : seqlen;  // that a row sees, about
+  if (window_left >= 0 && (is_causal || window_right >= 0)) {
+    const long long span = 1ll + window_left + (is_causal ? 0 : window_right);
+    if (span < keys) keys = span;
+  }
   int n = 0;
   for (long long h0 = 0; h0 < bh && !what && rc == FA_OK; h0 += chunk_heads, ++n) {
     const int slot = n & 1;
     const int nh = (int)((bh - h0 < chunk_heads) ? (bh - h0) : chunk_heads);
-    const size_t bytes = (size_t)nh * head_bytes;
     // the slot is free once the download that used it two chunks ago has finished
     if (n >= 2) FA_TRY(cudaStreamWaitEvent(hp->up, hp->out_done[slot], 0));
-    for (int t = 0; t < 3; ++t)
-      FA_TRY(cudaMemcpyAsync(dev_ptr(slot, t), src[t] + (size_t)h0 * head_bytes, bytes, cudaMemcpyHostToDevice, hp->up));
-    FA_TRY(cudaEventRecord(hp->in_ready[slot], hp->up));
-    FA_TRY(cudaStreamWaitEvent(hp->run, hp->in_ready[slot], 0));
     if (n >= 2) FA_TRY(cudaStreamWaitEvent(hp->run, hp->out_done[slot], 0));
-    if (what) break;
-    rc = forward_impl(dev_ptr(slot, 0), dev_ptr(slot, 1), dev_ptr(slot, 2), dev_ptr(slot, 3), 1, nh, seqlen, head_dim,
-                      softmax_scale, is_causal, window_left, window_right, nullptr, hp->run, 0, 0, nullptr, nullptr, 0.f,
-                      0, h0, bh);
-    if (rc != FA_OK) break;
-    FA_TRY(cudaEventRecord(hp->done[slot], hp->run));
-    FA_TRY(cudaStreamWaitEvent(hp->down, hp->done[slot], 0));
-    FA_TRY(cudaMemcpyAsync(static_cast<char*>(o_host) + (size_t)h0 * head_bytes, dev_ptr(slot, 3), bytes,
-                           cudaMemcpyDeviceToHost, hp->down));
+    for (int i = 0, np; i < nh && !what && rc == FA_OK; i += np) {
+      np = h0 + nh < bh ? nh : last_chunk_piece(nh - i, head_bytes, h0 == 0, keys);
+      const size_t at = (size_t)i * head_bytes, host_at = (size_t)h0 * head_bytes + at, bytes = (size_t)np * head_bytes;
+      for (int t = 0; t < 3; ++t)
+        FA_TRY(cudaMemcpyAsync(dev_ptr(slot, t) + at, src[t] + host_at, bytes, cudaMemcpyHostToDevice, hp->up));
+      FA_TRY(cudaEventRecord(hp->in_ready[slot], hp->up));
+      FA_TRY(cudaStreamWaitEvent(hp->run, hp->in_ready[slot], 0));
+      if (what) break;
+      rc = forward_impl(dev_ptr(slot, 0) + at, dev_ptr(slot, 1) + at, dev_ptr(slot, 2) + at, dev_ptr(slot, 3) + at, 1, np,
+                        seqlen, head_dim, softmax_scale, is_causal, window_left, window_right, nullptr, hp->run, 0, 0,
+                        nullptr, nullptr, 0.f, 0, h0 + i, bh);
+      if (rc != FA_OK) break;
+      FA_TRY(cudaEventRecord(hp->done[slot], hp->run));
+      FA_TRY(cudaStreamWaitEvent(hp->down, hp->done[slot], 0));
+      FA_TRY(cudaMemcpyAsync(static_cast<char*>(o_host) + host_at, dev_ptr(slot, 3) + at, bytes, cudaMemcpyDeviceToHost,
+                             hp->down));
+    }
     FA_TRY(cudaEventRecord(hp->out_done[slot], hp->down));
   }
 #undef FA_TRY

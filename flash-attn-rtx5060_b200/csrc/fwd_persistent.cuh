@@ -211,6 +211,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO,
                       const FwdParams p) {
   using Cfg = PersistentCfg<D>;
+  constexpr bool kLateO = kShort && !kDropout && !kAlibi;
   static_assert(!kOwnP || (D == 64 && kShort), "columns of P's own lie beside an O of 64 columns");
   extern __shared__ __align__(1024) uint8_t smem[];
 
@@ -422,6 +423,36 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           }
           tmem_wait_st();
         };
+        // O of this warp's rows times the rows' factors. s_full for this tile was committed behind the previous tile's P.V
+        // (kOwnP: behind its first 96 keys), so O is at rest.
+        // It has to be done before P is handed over, and the short build does it last, with 96 keys' scores gone from the
+        // registers: 64 columns a turn instead of 16, one or two waits instead of four or eight. A warp moves a row in
+        // every few tiles where scores spread widely. us before -> after, scores of spread 1 / 4: B4 H16 N2048 d64 causal
+        // 62.9 -> 62.2 / 68.1 -> 63.5, B8 H12 N1000 d64 45.2 -> 44.6 / 50.2 -> 45.6, d128 61.7 -> 61.6 / 69.1 -> 63.2, with
+        // log-sum-exp 46.9 -> 45.4 / 49.7 -> 45.7, window 512 B4 H16 N8192 d64 154.9 -> 154.3 / 164.9 -> 155.2. In the
+        // long build the factor is a register too many through the exponentials: B2 H16 N4096 d128 241 -> 248 / 277 -> 269,
+        // and 32 columns a turn at the old place spill (252 / 284); dropout 84.8 -> 86.3 / 87.8 -> 87.8.
+        auto rescale_o = [&](float alpha) {
+          constexpr int kW = kLateO ? 64 : 16;  // columns at a time
+          if (kOwnP) {
+            ok &= mbar_wait(&p_empty[s], par_s, abort_flag);
+            tc_fence_after();
+          }
+#pragma unroll 1
+          for (int c = 0; c < D; c += kW) {
+            uint32_t r[kW / 16][16];
+#pragma unroll
+            for (int x = 0; x < kW / 16; ++x) tmem_ld16(tO + c + x * 16, r[x]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int x = 0; x < kW / 16; ++x) {
+              tmem_ld_fence16(r[x]);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) r[x][i] = __float_as_uint(__uint_as_float(r[x][i]) * alpha);
+              tmem_st16(tO + c + x * 16, r[x]);
+            }
+          }
+        };
         auto tile_body = [&](auto masked_tag) {
           constexpr bool kMasked = decltype(masked_tag)::value;
           constexpr bool kPoly = !kMasked && !kDropout && !(kShort && D == 128);
@@ -501,6 +532,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           // fp16 (a row with a single visible key returns that key's V bit for bit). A cut tile over the first keys is
           // the only tile of its walk (with ALiBi it may be the last), or the far edge of a left window lies in it.
           const bool first_keys = (!kMasked || kAlibi) && kv0 == 0;
+          float alpha_o = 1.f;  // kLateO: the factor for this row's O
           if (__any_sync(0xffffffffu, m_new > (first_keys ? fminf(m_used, m_limit) : m_limit))) {
             const bool fresh = l_run == 0.f;
             float alpha = 1.f;
@@ -511,24 +543,8 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             }
             m_limit = l_run == 0.f && m_new == -INFINITY ? -INFINITY : m_used + lazy;
             l_run *= alpha;
-            // s_full for this tile was committed behind the previous tile's P.V (kOwnP: behind its first 96 keys), so O is
-            // at rest here.
-            if (kv0 != kv_first && __any_sync(0xffffffffu, alpha != 1.f)) {
-              if (kOwnP) {
-                ok &= mbar_wait(&p_empty[s], par_s, abort_flag);
-                tc_fence_after();
-              }
-#pragma unroll 1
-              for (int c = 0; c < D / 16; ++c) {
-                uint32_t r[16];
-                tmem_ld16(tO + c * 16, r);
-                tmem_wait_ld();
-                tmem_ld_fence16(r);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                tmem_st16(tO + c * 16, r);
-              }
-            }
+            if (kLateO) alpha_o = kv0 == kv_first ? 1.f : alpha;
+            else if (kv0 != kv_first && __any_sync(0xffffffffu, alpha != 1.f)) rescale_o(alpha);
             if (!kMasked && !kShort) {
               lsum_a = 0ull;
               lsum_b = 0ull;
@@ -549,6 +565,7 @@ fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           exp_tile<16, kPoly ? Cfg::kPolyOf2 : 0>(sc + 64, scale2, negms2, pk1, lsum_a, lsum_b);
           if (kDropout) dropout_mask<2>(pk1, p, drow, drop_blocks + 4);
           tmem_st16(tP + 32, pk1);
+          if (kLateO && __any_sync(0xffffffffu, alpha_o != 1.f)) rescale_o(alpha_o);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();

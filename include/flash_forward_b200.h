@@ -142,7 +142,7 @@ int flash_forward_ex(const void* q, const void* k, const void* v, void* o, int b
 /* The same forward for callers that hold Q, K, V and want O in HOST memory: the flow of the
  * reference's driver (src/main.cu:83-85 upload, :99 run, :101 download) as one blocking call.
  * The (batch, head) axis is cut into chunks of `chunk_heads` heads; upload, kernel and download
- * of successive chunks overlap on three internal streams through a two-slot device workspace
+ * of successive chunks (the last one in pieces) overlap on three internal streams through a two-slot device workspace
  * of flash_forward_host_workspace_bytes() bytes that the caller provides (256-byte aligned).
  * Pinned host buffers give full overlap; pageable ones work but serialise. Returns after O is
  * complete in o_host, with FA_DEVICE_TIMEOUT if a device-side wait gave up. */

@@ -144,3 +144,34 @@ def test_columns_of_its_own_for_p_change_no_bit(pkg, b, h, n, causal, rising):
         assert torch.equal(o, want)
     exact_out, _ = exact(q[:1, :2], k[:1, :2], v[:1, :2], causal, -1, -1)
     assert (out[:1, :2].double() - exact_out).abs().max().item() < 4e-3  # as above
+
+
+# Where a row's reference moves, O is rescaled; the short build does that behind the exponentials of the first 96 keys. Scores
+# that grow from the last tile to the first move rows in every tile, in a spread of 4 in some.
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n,causal,wl", [(300, False, -1), (640, False, -1), (1000, False, -1), (1024, True, -1),
+                                         (2500, True, -1), (2700, True, -1), (2900, True, 500)])
+@pytest.mark.parametrize("rising", [False, True])
+def test_rows_whose_reference_moves(pkg, d, n, causal, wl, rising):
+    import torch
+
+    heads = 3 if n < 2000 else 40  # (whole pairs of q tiles and single ones)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + d)
+    q, k, v = (torch.randn(1, heads, n, d, device="cuda", generator=g) for _ in range(3))
+    if rising:
+        q, k = q.abs(), k * 0.1 + torch.linspace(6.0, -1.0, n, device="cuda")[:, None]
+    else:
+        q = q * 4
+    q, k, v = q.half(), k.half(), v.half()
+    kw = dict(causal=causal, window_left=wl)
+    out = pkg.attention_forward(q, k, v, **kw)
+    out2, lse = pkg.attention_forward(q, k, v, return_lse=True, **kw)
+    pkg.check(torch.cuda.current_stream().cuda_stream)
+    want, want_lse = exact(q[:, -2:], k[:, -2:], v[:, -2:], causal, wl, -1)
+    for o in (out, out2):
+        # P and the output rounded to fp16, 2^-11 each, where one key has all the weight
+        assert ((o[:, -2:].double() - want).norm() / want.norm()).item() < 2.0 ** -10
+        assert (o[:, -2:].double() - want).abs().max().item() < 6e-3  # the same of |v| < 6
+    # scores of up to about 6 * d / sqrt(d) in fp32, 2^-24 of them per product and add
+    assert ((lse[:, -2:].double() - want_lse).abs() / (1 + want_lse.abs())).max().item() < 2e-5
