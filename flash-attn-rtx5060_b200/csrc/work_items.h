@@ -47,7 +47,8 @@ inline int pick_head_group(int bh, int seqlen, int head_dim, int causal, int win
 }
 
 // Takes some of the pairs of q tiles apart into single q tiles whose kv tiles the two stages of a CTA share out
-// (ItemGeom::split). Per unit of work a single costs 1.2 times a pair (every product fetches a kv tile of its own, and
+// (ItemGeom::split). Per unit of work a single costs more than a pair (where balance
+// no longer matters about 1.05 times, 48x1536 and 60x1024 below: every product fetches a kv tile of its own, and
 // the epilogue merges two outputs), but there are twice as many items of half the length.
 // - Items of about equal cost (no mask, a short window): the last, partial wave is split when its halves still make
 //   one wave. 32x4096 d128: 3.46 waves of 32 steps, 246 -> 220 us; 40x1000 d64 31.3 -> 25.3 us.
