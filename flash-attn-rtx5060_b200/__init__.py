@@ -14,6 +14,7 @@ reference) and its call site (src/main.cu:99).
 import ctypes
 import os
 import sys
+import threading
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflashfwd_b200.so")
@@ -43,6 +44,7 @@ EXPORTS = (
     "flash_forward_shutdown",
 )
 
+_lock = threading.RLock()  # around the first load of either
 _lib = None
 _native = None  # forward() of _torch_binding once looked for; answers NotImplemented where there is none
 
@@ -56,8 +58,16 @@ class FlashForwardError(RuntimeError):
 def lib():
     """Loads the shared library once. Raises OSError when it has not been built."""
     global _lib
-    if _lib is not None:
-        return _lib
+    if _lib is None:
+        with _lock:
+            if _lib is None:
+                _lib = _open()
+        if "torch" in sys.modules:
+            _load_native()
+    return _lib
+
+
+def _open():
     if not os.path.exists(LIB_PATH):
         raise OSError(f"{LIB_PATH} not found: build it with `make -C {os.path.join(_HERE, 'csrc')}`")
     L = ctypes.CDLL(LIB_PATH)
@@ -100,9 +110,6 @@ def lib():
     L.flash_forward_head_group.restype = i
     L.flash_forward_shutdown.argtypes = []
     L.flash_forward_shutdown.restype = i
-    _lib = L
-    if "torch" in sys.modules:
-        _load_native()
     return L
 
 
@@ -112,19 +119,20 @@ def _load_native():
     called without ctypes as well, where the arguments are plain numbers."""
     global _native
     L = lib()
-    if _native is not None:
-        return _native
-    try:
-        import torch  # noqa: F401  (its libraries have to be loaded first)
+    with _lock:
+        if _native is not None:
+            return _native
+        try:
+            import torch  # noqa: F401  (its libraries have to be loaded first)
 
-        from . import _torch_binding
-    except ImportError:
-        _native = lambda *args: NotImplemented  # noqa: E731
+            from . import _torch_binding
+        except ImportError:
+            _native = lambda *args: NotImplemented  # noqa: E731
+            return _native
+        _torch_binding.set_noalloc(L.flash_forward_noalloc)
+        L.flash_forward_noalloc = _torch_binding.noalloc
+        _native = _torch_binding.forward
         return _native
-    _torch_binding.set_noalloc(L.flash_forward_noalloc)
-    L.flash_forward_noalloc = _torch_binding.noalloc
-    _native = _torch_binding.forward
-    return _native
 
 
 def _raise(code):

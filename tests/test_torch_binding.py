@@ -1,8 +1,15 @@
 """The native form of the Python entry points (host/torch_binding.cpp) against the Python code that it stands in for: the
 same results bit for bit, the same errors, and whatever it does not know is left to the Python code."""
+import builtins
 import ctypes
+import importlib.util
+import os
+import sys
+import threading
 
 import pytest
+
+from conftest import ROOT
 
 torch = pytest.importorskip("torch")
 
@@ -13,6 +20,54 @@ def native(pkg):
     fn = pkg._load_native()
     assert type(fn).__name__ == "builtin_function_or_method", "the binding was not built"
     return fn
+
+
+PKG_DIR = os.path.join(ROOT, "flash-attn-rtx5060_b200")
+
+
+@pytest.fixture
+def load_as(monkeypatch):
+    """Imports the package a second time, under a name of its own."""
+    def load(name, directory=PKG_DIR):
+        spec = importlib.util.spec_from_file_location(name, os.path.join(directory, "__init__.py"),
+                                                      submodule_search_locations=[directory])
+        module = importlib.util.module_from_spec(spec)
+        monkeypatch.setitem(sys.modules, name, module)
+        spec.loader.exec_module(module)
+        return module
+    return load
+
+
+def test_first_calls_of_two_threads(load_as, monkeypatch):
+    """Two threads that load the native part at once, the second of them as late as it can be."""
+    pkg = load_as("flash_attn_of_two_threads")
+    both_here, first_done, arrivals = threading.Barrier(2), threading.Event(), []
+    plain_import = builtins.__import__
+
+    def slow_import(name, globals=None, locals=None, fromlist=(), level=0):
+        module = plain_import(name, globals, locals, fromlist, level)
+        if fromlist and "_torch_binding" in fromlist:
+            arrivals.append(None)
+            second = len(arrivals) == 2
+            try:
+                both_here.wait(timeout=1.0)
+            except threading.BrokenBarrierError:
+                pass  # the other thread is kept out meanwhile
+            if second:
+                first_done.wait(timeout=10.0)
+        return module
+
+    def load():
+        pkg._load_native()
+        first_done.set()
+    monkeypatch.setattr(builtins, "__import__", slow_import)
+    threads = [threading.Thread(target=load) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    with pytest.raises(ctypes.ArgumentError):  # (once loaded twice, it passed such arguments on to itself)
+        pkg.lib().flash_forward_noalloc(object(), 16, 16, 16, 1, 1, 1, 63, 0.0, 0, -1, -1, None, 0, 0)
 
 
 def test_arguments_that_are_not_plain_go_to_ctypes(pkg, native):
