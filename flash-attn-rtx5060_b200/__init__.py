@@ -129,9 +129,10 @@ def _load_native():
         except ImportError:
             _native = lambda *args: NotImplemented  # noqa: E731
             return _native
-        _torch_binding.set_noalloc(L.flash_forward_noalloc)
-        L.flash_forward_noalloc = _torch_binding.noalloc
-        _native = _torch_binding.forward
+        entry_points = (L.flash_forward, L.flash_forward_alibi, L.flash_forward_lse, L.flash_forward_dropout,
+                        L.flash_forward_noalloc)
+        _native, L.flash_forward_noalloc = _torch_binding.bind(
+            *(ctypes.cast(fn, ctypes.c_void_p).value for fn in entry_points), L.flash_forward_noalloc)
         return _native
 
 

@@ -1,5 +1,7 @@
 // Native part of the Python entry points: argument checks, output allocation and the call of the C ABI for torch tensors,
-// as one function of the CPython API, and a caller of flash_forward_noalloc for plain numbers. A small call is bound by
+// as one function of the CPython API, and a caller of flash_forward_noalloc for plain numbers. Nothing is linked or kept
+// here: bind() makes both for the library whose entry points it is given, the one that the package has loaded, whatever
+// other copies of it the process holds. A small call is bound by
 // the host: with ctypes and the checks in Python attention_forward took 9.2 us a call (2.1 of them in the library and
 // the driver, 1.5 ctypes, 1.3 the output tensor) where the kernel takes 7.2 (B1 H4 N512 d64).
 //
@@ -30,9 +32,20 @@ bool plain_int(PyObject* o) { return PyLong_Check(o); }
 int low_int(PyObject* o) { return static_cast<int>(PyLong_AsUnsignedLongMask(o)); }
 bool plain_number(PyObject* o) { return PyFloat_Check(o) || PyLong_Check(o); }
 
+// What bind() was given; the `self` of the functions that it returns, as a capsule.
+struct Library {
+  decltype(&flash_forward) plain;
+  decltype(&flash_forward_alibi) alibi;
+  decltype(&flash_forward_lse) lse;
+  decltype(&flash_forward_dropout) dropout;
+  decltype(&flash_forward_noalloc) noalloc;
+  PyObject* ctypes_noalloc;  // takes the calls of noalloc() with anything but plain numbers
+};
+const Library& library(PyObject* self) { return *static_cast<Library*>(PyCapsule_GetPointer(self, nullptr)); }
+
 // forward(q, k, v, causal, window_left, window_right, softmax_scale, out, alibi_slopes, return_lse, dropout_p, seed):
 // the result of attention_forward, an int (status code of a call that failed) or NotImplemented.
-PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+PyObject* forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 12) return not_here();
   PyObject *py_out = a[7], *py_slopes = a[8];
@@ -75,12 +88,13 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int b = static_cast<int>(B), h = static_cast<int>(H), s = static_cast<int>(N), d = static_cast<int>(D);
   const int wl = low_int(a[4]), wr = low_int(a[5]);
   const unsigned long long seed = PyLong_AsUnsignedLongLongMask(a[11]);
+  const Library& lib = library(self);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  if (dropout > 0.f) rc = flash_forward_dropout(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, dropout, seed, stream);
-  else if (want_lse) rc = flash_forward_lse(pq, pk, pv, po, pl, b, h, s, d, scale, causal, wl, wr, slopes, stream);
-  else if (slopes) rc = flash_forward_alibi(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, stream);
-  else rc = flash_forward(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, stream);
+  if (dropout > 0.f) rc = lib.dropout(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, dropout, seed, stream);
+  else if (want_lse) rc = lib.lse(pq, pk, pv, po, pl, b, h, s, d, scale, causal, wl, wr, slopes, stream);
+  else if (slopes) rc = lib.alibi(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, stream);
+  else rc = lib.plain(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, stream);
   Py_END_ALLOW_THREADS
   if (rc != FA_OK) return PyLong_FromLong(rc);
   PyObject* py_result = py_out;
@@ -95,15 +109,6 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// The ctypes function that noalloc() passes anything but plain numbers on to.
-PyObject* g_ctypes_noalloc = nullptr;
-
-PyObject* set_noalloc(PyObject*, PyObject* fn) {
-  Py_INCREF(fn);
-  Py_XSETREF(g_ctypes_noalloc, fn);
-  Py_RETURN_NONE;
-}
-
 bool address(PyObject* o, void** p) {
   if (o == Py_None) {
     *p = nullptr;
@@ -115,7 +120,7 @@ bool address(PyObject* o, void** p) {
 }
 
 // flash_forward_noalloc for pointers given as ints or None and numbers
-PyObject* noalloc(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names) {
+PyObject* noalloc(PyObject* self, PyObject* const* a, Py_ssize_t n, PyObject* names) {
   void *q, *k, *v, *o, *stream;
   bool known = n == 15 && (names == nullptr || PyTuple_GET_SIZE(names) == 0) && address(a[0], &q) && address(a[1], &k) &&
                address(a[2], &v) && address(a[3], &o) && address(a[12], &stream) && plain_number(a[8]);
@@ -129,21 +134,48 @@ PyObject* noalloc(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names) 
       known = false;
     }
   }
-  if (!known) return PyObject_Vectorcall(g_ctypes_noalloc, a, n, names);
+  const Library& lib = library(self);
+  if (!known) return PyObject_Vectorcall(lib.ctypes_noalloc, a, n, names);
   const int x[] = {low_int(a[4]), low_int(a[5]), low_int(a[6]), low_int(a[7]), low_int(a[9]), low_int(a[10]), low_int(a[11]),
                    low_int(a[13]), low_int(a[14])};
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = flash_forward_noalloc(q, k, v, o, x[0], x[1], x[2], x[3], scale, x[4], x[5], x[6], stream, x[7], x[8]);
+  rc = lib.noalloc(q, k, v, o, x[0], x[1], x[2], x[3], scale, x[4], x[5], x[6], stream, x[7], x[8]);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
 }
 
-PyMethodDef methods[] = {
-    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward)), METH_FASTCALL, nullptr},
-    {"set_noalloc", set_noalloc, METH_O, nullptr},
-    {"noalloc", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(noalloc)), METH_FASTCALL | METH_KEYWORDS, nullptr},
-    {nullptr, nullptr, 0, nullptr}};
+PyMethodDef forward_def = {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward)), METH_FASTCALL, nullptr};
+PyMethodDef noalloc_def = {"flash_forward_noalloc", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(noalloc)),
+                           METH_FASTCALL | METH_KEYWORDS, nullptr};
+
+void drop_library(PyObject* capsule) {
+  Library* lib = static_cast<Library*>(PyCapsule_GetPointer(capsule, nullptr));
+  Py_DECREF(lib->ctypes_noalloc);
+  delete lib;
+}
+
+// bind(addresses of flash_forward, flash_forward_alibi, flash_forward_lse, flash_forward_dropout, flash_forward_noalloc as
+// ints, the ctypes function of the last): (forward, noalloc)
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long plain, alibi, lse, dropout, noalloc_address;
+  PyObject* fn;
+  if (!PyArg_ParseTuple(args, "KKKKKO", &plain, &alibi, &lse, &dropout, &noalloc_address, &fn)) return nullptr;
+  Library* lib = new Library{reinterpret_cast<decltype(Library::plain)>(plain), reinterpret_cast<decltype(Library::alibi)>(alibi),
+                             reinterpret_cast<decltype(Library::lse)>(lse), reinterpret_cast<decltype(Library::dropout)>(dropout),
+                             reinterpret_cast<decltype(Library::noalloc)>(noalloc_address), fn};
+  PyObject* capsule = PyCapsule_New(lib, nullptr, drop_library);
+  if (!capsule) {
+    delete lib;
+    return nullptr;
+  }
+  Py_INCREF(fn);
+  PyObject* pair = Py_BuildValue("(NN)", PyCFunction_New(&forward_def, capsule), PyCFunction_New(&noalloc_def, capsule));
+  Py_DECREF(capsule);
+  return pair;
+}
+
+PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -3,7 +3,9 @@ same results bit for bit, the same errors, and whatever it does not know is left
 import builtins
 import ctypes
 import importlib.util
+import math
 import os
+import shutil
 import sys
 import threading
 
@@ -68,6 +70,42 @@ def test_first_calls_of_two_threads(load_as, monkeypatch):
         t.join()
     with pytest.raises(ctypes.ArgumentError):  # (once loaded twice, it passed such arguments on to itself)
         pkg.lib().flash_forward_noalloc(object(), 16, 16, 16, 1, 1, 1, 63, 0.0, 0, -1, -1, None, 0, 0)
+
+
+@pytest.fixture
+def copies(load_as, native, tmp_path):
+    """The package, a copy of it, and the package with another build of the library, in one process."""
+    second = str(tmp_path / "second")
+    shutil.copytree(PKG_DIR, second)
+    other_build = str(tmp_path / "another_build.so")
+    shutil.copy(os.path.join(PKG_DIR, "libflashfwd_b200.so"), other_build)
+    packages = [load_as("flash_attn_first"), load_as("flash_attn_second", second), load_as("flash_attn_other_build")]
+    packages[2].LIB_PATH = other_build
+    for p in packages:
+        p.lib()
+    return packages
+
+
+def test_noalloc_calls_the_library_that_its_package_loaded(copies):
+    """(A failing call leaves its text in the library that ran.)"""
+    faults = [(dict(q=None), b"null tensor"), (dict(head_dim=63), b"head_dim"), (dict(scale=math.nan), b"NaN")]
+    for p, (fault, _) in zip(copies, faults):
+        a = dict(q=16, k=16, v=16, o=16, batch=1, heads=1, seqlen=1, head_dim=64, scale=0.0) | fault
+        assert p.lib().flash_forward_noalloc(*a.values(), 0, -1, -1, None, 0, 0) != p.FA_OK
+    for p, (_, text) in zip(copies, faults):
+        assert text in p.lib().flash_forward_last_error()
+
+
+@pytest.mark.gpu
+def test_attention_forward_calls_the_library_that_its_package_loaded(copies):
+    x = torch.zeros(1, 1, 8, 64, device="cuda", dtype=torch.float16)
+    y = torch.zeros(1, 1, 8, 32, device="cuda", dtype=torch.float16)
+    faults = [(y, 0.0, "head_dim"), (x, math.nan, "NaN"), (x, 1e-35, "finite")]
+    for p, (t, scale, text) in zip(copies, faults):
+        with pytest.raises(p.FlashForwardError, match=text):
+            p.attention_forward(t, t, t, softmax_scale=scale)
+    for p, (_, _, text) in zip(copies, faults):
+        assert text.encode() in p.lib().flash_forward_last_error()
 
 
 def test_arguments_that_are_not_plain_go_to_ctypes(pkg, native):
