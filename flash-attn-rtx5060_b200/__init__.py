@@ -220,8 +220,10 @@ def run_flash_attention(B, N, S, d, Q, K, V, O, L=None, M=None, Is_dropout=False
 
 def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, softmax_scale=0.0, out=None, kernel=0,
                       variant=0, alibi_slopes=None, return_lse=False, dropout_p=0.0, seed=0):
-    """Convenience wrapper for torch CUDA tensors of shape [B, H, N, d], fp16, contiguous.
+    """Convenience wrapper for torch CUDA tensors of shape [B, H, N, d], fp16, contiguous, on one device.
 
+    `out`, if given, is written as [B, H, N, d] from its beginning, so its own shape does not matter as long as it is
+    contiguous and large enough. alibi_slopes: float32, one per head. Other operands raise an AssertionError.
     torch is used for device memory and the current stream only; the computation is the library's.
     With return_lse the result is (out, lse), lse a float32 [B, H, N] tensor (flash_forward_lse).
     With dropout_p > 0 the call is flash_forward_dropout(dropout_p, seed).
@@ -235,8 +237,7 @@ def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, so
             return r
     import torch
 
-    assert q.is_cuda and q.dtype == torch.float16 and q.is_contiguous() and q.dim() == 4
-    assert k.shape == q.shape and v.shape == q.shape and k.is_contiguous() and v.is_contiguous()
+    _check_operands(torch, q, k, v, out, alibi_slopes)
     if out is None:
         out = torch.empty_like(q)
     args = (torch, q, k, v, out, causal, window_left, window_right, softmax_scale, kernel, variant, alibi_slopes,
@@ -246,6 +247,22 @@ def attention_forward(q, k, v, causal=False, window_left=-1, window_right=-1, so
         return _enqueue_forward(device, *args)
     with torch.cuda.device(device):
         return _enqueue_forward(device, *args)
+
+
+def _check_operands(torch, q, k, v, out, alibi_slopes):
+    """The kernels get bare addresses: a tensor elsewhere, smaller or laid out otherwise would be read or written out of
+    bounds. Raised here and not asserted, so that it holds under `python -O` too."""
+    def fits(t, dtype):
+        return t.is_cuda and t.get_device() == q.get_device() and t.dtype == dtype and t.is_contiguous()
+    half = torch.float16
+    if not (q.is_cuda and q.dim() == 4 and fits(q, half)):
+        raise AssertionError("q: a contiguous fp16 CUDA tensor [B, H, N, d] is needed")
+    if not (k.shape == q.shape and v.shape == q.shape and fits(k, half) and fits(v, half)):
+        raise AssertionError("k and v have to be like q, on its device")
+    if out is not None and not (fits(out, half) and out.numel() >= q.numel()):
+        raise AssertionError("out: a contiguous fp16 tensor on q's device with room for the result is needed")
+    if alibi_slopes is not None and not (fits(alibi_slopes, torch.float32) and alibi_slopes.numel() == q.shape[1]):
+        raise AssertionError("alibi_slopes: a contiguous float32 tensor on q's device, one slope per head, is needed")
 
 
 def _current_raw_stream(torch, device):
@@ -262,8 +279,6 @@ def _enqueue_forward(device, torch, q, k, v, out, causal, window_left, window_ri
     B, H, N, d = q.shape
     L = lib()
     lse = None
-    if alibi_slopes is not None:  # float32 CUDA tensor with one slope per head
-        assert alibi_slopes.is_cuda and alibi_slopes.dtype == torch.float32 and alibi_slopes.numel() == H
     if dropout_p > 0.0:
         assert kernel == 0 and variant == 0 and not return_lse
         rc = L.flash_forward_dropout(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, H, N, d, softmax_scale,

@@ -59,8 +59,16 @@ PyObject* forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   if (at::impl::torch_function_mode_enabled() || c10::impl::dispatch_mode_enabled()) return not_here();
 
   const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
-  if (!q.is_cuda() || q.scalar_type() != at::kHalf || q.dim() != 4 || !q.is_contiguous()) return not_here();
-  if (k.sizes() != q.sizes() || v.sizes() != q.sizes() || !k.is_contiguous() || !v.is_contiguous()) return not_here();
+  if (!q.is_cuda() || q.dim() != 4) return not_here();
+  const auto device = q.get_device();
+  // what the kernel may be given the address of
+  auto fits = [&](const at::Tensor& t, at::ScalarType type) {
+    return t.is_cuda() && t.get_device() == device && t.scalar_type() == type && t.is_contiguous();
+  };
+  if (!fits(q, at::kHalf) || !fits(k, at::kHalf) || !fits(v, at::kHalf)) return not_here();
+  if (k.sizes() != q.sizes() || v.sizes() != q.sizes()) return not_here();
+  if (py_out != Py_None && (!fits(THPVariable_Unpack(py_out), at::kHalf) || THPVariable_Unpack(py_out).numel() < q.numel()))
+    return not_here();
   const bool causal = a[3] == Py_True, want_lse = a[9] == Py_True;
   const float scale = static_cast<float>(PyFloat_AsDouble(a[6])), dropout = static_cast<float>(PyFloat_AsDouble(a[10]));
   if (PyErr_Occurred()) {  // an int beyond the range of a double
@@ -72,10 +80,9 @@ PyObject* forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   const float* slopes = nullptr;
   if (py_slopes != Py_None) {
     const at::Tensor& t = THPVariable_Unpack(py_slopes);
-    if (!t.is_cuda() || t.scalar_type() != at::kFloat || t.numel() != H) return not_here();
+    if (!fits(t, at::kFloat) || t.numel() != H) return not_here();
     slopes = static_cast<const float*>(t.data_ptr());
   }
-  const auto device = q.get_device();
   if (device != c10::cuda::current_device()) return not_here();
 
   const at::Tensor out = py_out == Py_None ? at::empty_like(q) : THPVariable_Unpack(py_out);

@@ -132,6 +132,78 @@ def test_tensors_that_are_refused_stay_refused(pkg, native):
         pkg.attention_forward(None, q, q)
 
 
+class Tensor:
+    """What the Python code asks of a tensor."""
+    def __init__(self, shape=(1, 2, 64, 64), dtype=torch.float16, device=0, contiguous=True):
+        self.shape, self.dtype, self.device, self.contiguous = shape, dtype, device, contiguous
+        self.is_cuda = device >= 0
+    dim = lambda self: len(self.shape)  # noqa: E731
+    numel = lambda self: math.prod(self.shape)  # noqa: E731
+    get_device = lambda self: self.device  # noqa: E731
+    is_contiguous = lambda self: self.contiguous  # noqa: E731
+
+
+ROOMY = (1, 2, 65, 64)
+REFUSED = [dict(k=dict(device=-1)), dict(v=dict(device=-1)), dict(k=dict(device=1)), dict(v=dict(device=1)),
+           dict(k=dict(dtype=torch.float32)), dict(v=dict(dtype=torch.bfloat16)), dict(v=dict(contiguous=False)),
+           dict(out=dict(device=-1)), dict(out=dict(device=1)), dict(out=dict(shape=(1, 2, 63, 64))),
+           dict(out=dict(contiguous=False)), dict(out=dict(dtype=torch.float32)), dict(out=dict(dtype=torch.bfloat16)),
+           dict(alibi_slopes=dict(shape=(2,), dtype=torch.float32, contiguous=False)),
+           dict(alibi_slopes=dict(shape=(2,), dtype=torch.float32, device=1)),
+           dict(alibi_slopes=dict(shape=(2,), dtype=torch.float32, device=-1)),
+           dict(alibi_slopes=dict(shape=(3,), dtype=torch.float32)), dict(alibi_slopes=dict(shape=(2,)))]
+ACCEPTED = [dict(), dict(out=dict()), dict(out=dict(shape=(2, 64, 64))), dict(out=dict(shape=ROOMY)),
+            dict(alibi_slopes=dict(shape=(2,), dtype=torch.float32)), dict(alibi_slopes=dict(shape=(2, 1), dtype=torch.float32))]
+
+
+@pytest.mark.parametrize("operands,accepted", [(o, False) for o in REFUSED] + [(o, True) for o in ACCEPTED], ids=str)
+def test_operands_that_the_kernel_could_not_take_are_refused(pkg, monkeypatch, operands, accepted):
+    enqueued = []
+    monkeypatch.setattr(pkg, "_native", lambda *a: NotImplemented)
+    monkeypatch.setattr(pkg, "_enqueue_forward", lambda *a: enqueued.append(a))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch, "empty_like", lambda t: t)
+    a = {n: Tensor(**operands.get(n, {})) for n in "qkv"}
+    a |= {n: Tensor(**operands[n]) for n in ("out", "alibi_slopes") if n in operands}
+    if accepted:
+        pkg.attention_forward(**a)
+    else:
+        with pytest.raises(AssertionError):
+            pkg.attention_forward(**a)
+    assert len(enqueued) == accepted
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("operands,accepted", [(o, False) for o in REFUSED] + [(o, True) for o in ACCEPTED], ids=str)
+def test_the_native_part_leaves_such_operands_to_the_python_code(pkg, native, monkeypatch, operands, accepted):
+    """Bound to entry points that only count their calls, so that nothing is launched whatever the answer."""
+    def tensor(shape=(1, 2, 64, 64), dtype=torch.float16, device=0, contiguous=True):
+        if device >= torch.cuda.device_count():
+            pytest.skip("one GPU")
+        t = torch.zeros(*shape, 1 if contiguous else 2, dtype=dtype, device="cpu" if device < 0 else f"cuda:{device}")
+        return t[..., 0]
+    calls = []
+    vp, i, f, u = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_ulonglong
+    head = [vp, vp, vp, vp], [i, i, i, i, f, i, i, i]
+    signatures = [head[0] + head[1] + [vp], head[0] + head[1] + [vp, vp], head[0] + [vp] + head[1] + [vp, vp],
+                  head[0] + head[1] + [vp, f, u, vp], head[0] + head[1] + [vp, i, i]]
+    stand_ins = [ctypes.CFUNCTYPE(i, *s)(lambda *a: calls.append(a) or 0) for s in signatures]
+    from flash_attn_rtx5060_b200 import _torch_binding
+
+    forward, _ = _torch_binding.bind(*(ctypes.cast(s, vp).value for s in stand_ins), stand_ins[-1])
+    a = {n: tensor(**operands.get(n, {})) for n in "qkv"}
+    a |= {n: tensor(**operands[n]) for n in ("out", "alibi_slopes") if n in operands}
+    r = forward(a["q"], a["k"], a["v"], False, -1, -1, 0.0, a.get("out"), a.get("alibi_slopes"), False, 0.0, 0)
+    assert (r is not NotImplemented) == accepted and len(calls) == accepted
+    if accepted:
+        assert calls[0][:4] == (a["q"].data_ptr(), a["k"].data_ptr(), a["v"].data_ptr(), r.data_ptr())
+    else:
+        monkeypatch.setattr(pkg, "_native", forward)
+        monkeypatch.setattr(pkg, "_enqueue_forward", None)
+        with pytest.raises(AssertionError):
+            pkg.attention_forward(**a)
+
+
 FORMS = [dict(), dict(causal=True), dict(causal=1), dict(causal=True, window_left=40), dict(window_left=64, window_right=10),
          dict(softmax_scale=0.25), dict(softmax_scale=1), dict(alibi=True, causal=True), dict(return_lse=True),
          dict(return_lse=True, alibi=True), dict(dropout_p=0.3, seed=7), dict(dropout_p=0.3, seed=-1),
