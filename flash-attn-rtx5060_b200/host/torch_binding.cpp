@@ -70,12 +70,13 @@ PyObject* forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   if (py_out != Py_None && (!fits(THPVariable_Unpack(py_out), at::kHalf) || THPVariable_Unpack(py_out).numel() < q.numel()))
     return not_here();
   const bool causal = a[3] == Py_True, want_lse = a[9] == Py_True;
-  const float scale = static_cast<float>(PyFloat_AsDouble(a[6])), dropout = static_cast<float>(PyFloat_AsDouble(a[10]));
+  const float scale = static_cast<float>(PyFloat_AsDouble(a[6]));
+  const double dropout = PyFloat_AsDouble(a[10]);  // (positive, though 0 as a float, it still asks for the dropout call)
   if (PyErr_Occurred()) {  // an int beyond the range of a double
     PyErr_Clear();
     return not_here();
   }
-  if (dropout > 0.f && want_lse) return not_here();
+  if (dropout > 0.0 && want_lse) return not_here();
   const auto B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
   const float* slopes = nullptr;
   if (py_slopes != Py_None) {
@@ -98,7 +99,8 @@ PyObject* forward(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   const Library& lib = library(self);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  if (dropout > 0.f) rc = lib.dropout(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, dropout, seed, stream);
+  if (dropout > 0.0)
+    rc = lib.dropout(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, static_cast<float>(dropout), seed, stream);
   else if (want_lse) rc = lib.lse(pq, pk, pv, po, pl, b, h, s, d, scale, causal, wl, wr, slopes, stream);
   else if (slopes) rc = lib.alibi(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, slopes, stream);
   else rc = lib.plain(pq, pk, pv, po, b, h, s, d, scale, causal, wl, wr, stream);

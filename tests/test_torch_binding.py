@@ -173,35 +173,52 @@ def test_operands_that_the_kernel_could_not_take_are_refused(pkg, monkeypatch, o
     assert len(enqueued) == accepted
 
 
+def bind_to_counters():
+    """The native part bound to entry points that only note their calls, so that nothing is launched: (forward, calls)."""
+    from flash_attn_rtx5060_b200 import _torch_binding
+
+    vp, i, f, u = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_ulonglong
+    tensors, shape = [vp, vp, vp, vp], [i, i, i, i, f, i, i, i]
+    signatures = dict(plain=tensors + shape + [vp], alibi=tensors + shape + [vp, vp], lse=tensors + [vp] + shape + [vp, vp],
+                      dropout=tensors + shape + [vp, f, u, vp], noalloc=tensors + shape + [vp, i, i])
+    calls = []
+    note = [ctypes.CFUNCTYPE(i, *s)(lambda *a, n=n: calls.append((n, *a)) or 0) for n, s in signatures.items()]
+    native, _ = _torch_binding.bind(*(ctypes.cast(f, vp).value for f in note), note[-1])
+    return lambda *a, keep=note: native(*a), calls
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("operands,accepted", [(o, False) for o in REFUSED] + [(o, True) for o in ACCEPTED], ids=str)
 def test_the_native_part_leaves_such_operands_to_the_python_code(pkg, native, monkeypatch, operands, accepted):
-    """Bound to entry points that only count their calls, so that nothing is launched whatever the answer."""
     def tensor(shape=(1, 2, 64, 64), dtype=torch.float16, device=0, contiguous=True):
         if device >= torch.cuda.device_count():
             pytest.skip("one GPU")
         t = torch.zeros(*shape, 1 if contiguous else 2, dtype=dtype, device="cpu" if device < 0 else f"cuda:{device}")
         return t[..., 0]
-    calls = []
-    vp, i, f, u = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_ulonglong
-    head = [vp, vp, vp, vp], [i, i, i, i, f, i, i, i]
-    signatures = [head[0] + head[1] + [vp], head[0] + head[1] + [vp, vp], head[0] + [vp] + head[1] + [vp, vp],
-                  head[0] + head[1] + [vp, f, u, vp], head[0] + head[1] + [vp, i, i]]
-    stand_ins = [ctypes.CFUNCTYPE(i, *s)(lambda *a: calls.append(a) or 0) for s in signatures]
-    from flash_attn_rtx5060_b200 import _torch_binding
-
-    forward, _ = _torch_binding.bind(*(ctypes.cast(s, vp).value for s in stand_ins), stand_ins[-1])
+    forward, calls = bind_to_counters()
     a = {n: tensor(**operands.get(n, {})) for n in "qkv"}
     a |= {n: tensor(**operands[n]) for n in ("out", "alibi_slopes") if n in operands}
     r = forward(a["q"], a["k"], a["v"], False, -1, -1, 0.0, a.get("out"), a.get("alibi_slopes"), False, 0.0, 0)
     assert (r is not NotImplemented) == accepted and len(calls) == accepted
     if accepted:
-        assert calls[0][:4] == (a["q"].data_ptr(), a["k"].data_ptr(), a["v"].data_ptr(), r.data_ptr())
+        assert calls[0][1:5] == (a["q"].data_ptr(), a["k"].data_ptr(), a["v"].data_ptr(), r.data_ptr())
     else:
         monkeypatch.setattr(pkg, "_native", forward)
         monkeypatch.setattr(pkg, "_enqueue_forward", None)
         with pytest.raises(AssertionError):
             pkg.attention_forward(**a)
+
+
+@pytest.mark.gpu
+def test_a_dropout_probability_below_the_range_of_a_float(pkg, native):
+    """1e-50 is 0 as a float and still a probability: with the log-sum-exp refused, else the dropout entry point's."""
+    forward, calls = bind_to_counters()
+    q = torch.zeros(1, 2, 64, 64, device="cuda", dtype=torch.float16)
+    assert forward(q, q, q, False, -1, -1, 0.0, None, None, True, 1e-50, 0) is NotImplemented
+    assert forward(q, q, q, False, -1, -1, 0.0, None, None, False, 1e-50, 7) is not NotImplemented
+    assert [c[0] for c in calls] == ["dropout"] and calls[0][14:16] == (0.0, 7)
+    with pytest.raises(AssertionError):
+        pkg.attention_forward(q, q, q, return_lse=True, dropout_p=1e-50)
 
 
 FORMS = [dict(), dict(causal=True), dict(causal=1), dict(causal=True, window_left=40), dict(window_left=64, window_right=10),
