@@ -122,6 +122,23 @@ def test_arguments_that_are_not_plain_go_to_ctypes(pkg, native):
         fn(16, 16, 16, 16, 1, 1, 1, 63.0, 0.0, 0, -1, -1, None, 0, 0)
 
 
+def test_noalloc_is_still_a_ctypes_function(load_as, native):
+    p = load_as("flash_attn_ctypes_function")
+    p.lib()
+    p._load_native()
+    fn, plain = p.lib().flash_forward_noalloc, p.lib().flash_forward
+    bad = (None, 16, 16, 16, 1, 1, 1, 64, 0.0, 0, -1, -1, None, 0, 0)
+    assert fn.argtypes == [*plain.argtypes, ctypes.c_int, ctypes.c_int] and fn.restype is ctypes.c_int
+    assert fn.errcheck is None and fn.__name__ == "flash_forward_noalloc"
+    assert ctypes.cast(fn, ctypes.c_void_p).value and isinstance(fn, ctypes._CFuncPtr)
+    assert fn(*bad) == p.FA_INVALID_ARG
+    fn.errcheck = lambda result, func, args: ("checked", result, func is fn, args[0])
+    assert fn(*bad) == ("checked", p.FA_INVALID_ARG, True, None)
+    del fn.errcheck
+    fn.restype = lambda rc: -rc
+    assert fn(*bad) == -p.FA_INVALID_ARG
+
+
 def test_tensors_that_are_refused_stay_refused(pkg, native):
     q = torch.zeros(1, 2, 64, 64, dtype=torch.float16)
     with pytest.raises(AssertionError):
