@@ -15,6 +15,7 @@ import ctypes
 import os
 import sys
 import threading
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflashfwd_b200.so")
@@ -114,7 +115,7 @@ def _open():
 
 
 def _load_native():
-    """The native form of attention_forward (host/torch_binding.cpp), which is built against the torch it is used with.
+    """The native form of attention_forward (host/torch_binding.cpp), if it was built against the torch it is used with.
     Without it everything runs through ctypes, with the same results. With it the loaded library's flash_forward_noalloc is
     called without ctypes as well, where the arguments are plain numbers."""
     global _native
@@ -126,7 +127,14 @@ def _load_native():
             import torch  # noqa: F401  (its libraries have to be loaded first)
 
             from . import _torch_binding
+            built_against = getattr(_torch_binding, "torch_version", None)
+            usable = built_against == str(torch.__version__)
+            if not usable:
+                warnings.warn(f"{_torch_binding.__file__} was built against torch {built_against}, not {torch.__version__}: "
+                              "calls go through ctypes, 5 us slower, until `make` has built it again")
         except ImportError:
+            usable = False
+        if not usable:
             _native = lambda *args: NotImplemented  # noqa: E731
             return _native
         entry_points = (L.flash_forward, L.flash_forward_alibi, L.flash_forward_lse, L.flash_forward_dropout,

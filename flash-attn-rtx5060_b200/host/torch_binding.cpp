@@ -189,4 +189,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_binding", nullptr, -1, meth
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_binding(void) { return PyModule_Create(&module); }
+#define FA_STRING_OF(x) #x
+#define FA_STRING(x) FA_STRING_OF(x)
+
+PyMODINIT_FUNC PyInit__torch_binding(void) {
+  PyObject* m = PyModule_Create(&module);
+  // the torch whose object layouts are compiled in
+  if (m && PyModule_AddStringConstant(m, "torch_version", FA_STRING(FA_TORCH_VERSION)) < 0) Py_CLEAR(m);
+  return m;
+}

@@ -122,6 +122,15 @@ def test_arguments_that_are_not_plain_go_to_ctypes(pkg, native):
         fn(16, 16, 16, 16, 1, 1, 1, 63.0, 0.0, 0, -1, -1, None, 0, 0)
 
 
+def test_a_binding_built_against_another_torch_is_not_used(load_as, native, monkeypatch):
+    p = load_as("flash_attn_another_torch")
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.warns(UserWarning, match="0.0.1"):
+        p.lib()
+    assert p._load_native()(None) is NotImplemented
+    assert type(p.lib().flash_forward_noalloc) is type(p.lib().flash_forward)
+
+
 def test_noalloc_is_still_a_ctypes_function(load_as, native):
     p = load_as("flash_attn_ctypes_function")
     p.lib()
