@@ -21,16 +21,54 @@ pytestmark = pytest.mark.gpu
 WAITTEST = os.path.join(ROOT, "tests", "_build", "libflashfwd_waittest.so")
 
 
-def test_wait_gives_up_and_the_device_stays_usable(pkg, ob):
-    import torch
+EARLY = os.path.join(ROOT, "tests", "_build", "libearly_release.so")
 
+
+def load_waittest():
     if not os.path.isfile(WAITTEST):
         pytest.skip("tests/_build/libflashfwd_waittest.so was not built")
     L = ctypes.CDLL(WAITTEST)
     vp, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
     L.flash_forward_ex.argtypes = [vp, vp, vp, vp, i, i, i, i, f, i, i, i, vp, i, i, vp]
+    L.flash_forward_noalloc.argtypes = [vp, vp, vp, vp, i, i, i, i, f, i, i, i, vp, i, i]
+    L.flash_forward_noalloc_check.argtypes = [vp, i]
     L.flash_forward_check.argtypes = [vp]
     L.flash_forward_last_error.restype = ctypes.c_char_p
+    return L
+
+
+@pytest.mark.parametrize("h,n,d,causal", [(1, 100, 64, True), (4, 512, 64, False), (8, 333, 128, True), (40, 1500, 128, True),
+                                          (40, 1500, 64, False)])
+def test_the_kernel_in_front_may_take_longer_than_the_limit(pkg, h, n, d, causal):
+    """The kernel in front in the stream lets this one in at once and goes on for 20 ms, ten times the limit of the test
+    build's waits: they count from its end."""
+    import torch
+
+    L = load_waittest()
+    early = ctypes.CDLL(EARLY)
+    early.launch_early_release.argtypes = [ctypes.c_ulonglong, ctypes.c_void_p]
+    q, k, v = (torch.from_numpy(a).cuda() for a in make_inputs(n, 1, h, n, d))
+    want = pkg.attention_forward(q, k, v, causal=causal)
+    stream = torch.cuda.current_stream().cuda_stream
+    pkg.check(stream)
+    shape = (1, h, n, d, 0.0, int(causal), -1, -1, stream, 0, 0)
+    out, own = torch.zeros_like(q), torch.zeros_like(q)
+    for _ in range(2):
+        assert early.launch_early_release(20_000_000, stream) == 0
+        assert L.flash_forward_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *shape, None) == pkg.FA_OK
+        assert L.flash_forward_check(stream) == pkg.FA_OK
+        assert early.launch_early_release(20_000_000, stream) == 0
+        assert L.flash_forward_noalloc(q.data_ptr(), k.data_ptr(), v.data_ptr(), own.data_ptr(), *shape) == pkg.FA_OK
+        assert L.flash_forward_noalloc_check(stream, 0) == pkg.FA_OK
+        assert torch.equal(out, want) and torch.equal(own, want)
+        out.zero_()
+        own.zero_()
+
+
+def test_wait_gives_up_and_the_device_stays_usable(pkg, ob):
+    import torch
+
+    L = load_waittest()
 
     B, H, N, d = 1, 1, 512, 128   # two work items; CTA 0's first item has four kv tiles
     q, k, v = make_inputs(61, B, H, N, d)
