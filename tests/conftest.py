@@ -1,4 +1,6 @@
+import ctypes
 import os
+import subprocess
 import sys
 
 import numpy as np
@@ -49,6 +51,22 @@ def ob():
         entry._run(["make", "-C", os.path.join(ROOT, "oracle"), "liboracle_attn.so"], ROOT)
     b.port()
     return b
+
+
+@pytest.fixture(scope="session")
+def wi(tmp_path_factory):
+    """The rules of csrc/work_items.h, compiled for the host (tests/work_items_host.cpp)."""
+    so = str(tmp_path_factory.mktemp("work_items") / "work_items.so")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    csrc = os.path.join(ROOT, "flash-attn-rtx5060_b200", "csrc")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", csrc, "-I", cuda, "-o", so,
+                           os.path.join(ROOT, "tests", "work_items_host.cpp")])
+    return ctypes.CDLL(so)
+
+
+def rules_args(heads, n, d, causal=False, wl=-1, wr=-1, sms=148):
+    """A launch on all heads of a problem, as the functions of `wi` take it."""
+    return (ctypes.c_int * 9)(heads, n, d, int(causal), wl, wr, sms, 0, heads)
 
 
 def make_inputs(seed, B, H, N, d, dist="normal"):

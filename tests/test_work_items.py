@@ -3,25 +3,11 @@ out exactly once with exactly its visible kv tiles, and the hand-over of items t
 order in which a CTA may claim them."""
 import ctypes
 import itertools
-import os
 import random
-import subprocess
 
 import pytest
 
-from conftest import ROOT
-
-CSRC = os.path.join(ROOT, "flash-attn-rtx5060_b200", "csrc")
 SMS = 148
-
-
-@pytest.fixture(scope="module")
-def wi(tmp_path_factory):
-    so = str(tmp_path_factory.mktemp("work_items") / "work_items.so")
-    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
-    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-I", cuda, "-o", so,
-                           os.path.join(ROOT, "tests", "work_items_host.cpp")])
-    return ctypes.CDLL(so)
 
 
 class Launch:

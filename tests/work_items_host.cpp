@@ -28,6 +28,12 @@ void plan(const int* args, int* out) {
   out[2] = p.head_group;
 }
 
+// short_items() of a launch, with ALiBi or without
+int short_build(const int* args, int alibi) { return fa::short_items(args[1], args[3], args[4], args[5], alibi != 0); }
+
+// own_p_columns(), which plain launches of the short build at head_dim 64 ask
+int own_p(const int* args) { return fa::own_p_columns(params(args)); }
+
 // next_item() from `item` on, claims taken from the list; out[0..12] = item, head, rows and steps of both stages, top,
 // steps, split. Returns the number of claims used.
 int walk(const int* args, int item, const int* claims, int* out) {
