@@ -22,7 +22,8 @@
 // stages' tiles overlap more. Done together (B200, us): the issuer's products in branch-free groups (umma_pv64 and the
 // like) without a vote behind each wait; O rescaled by the softmax warps themselves, which took a hand-over per tile to
 // the warps 8-11 off the path; a fifth of the exponentials on the FMA pipe (exp2_poly); what is fixed for an item
-// computed once per item. B2 H32 N8192 d128 causal 1085 -> 971, B2 H16 N4096 d128 268 -> 237, B4 H16 N16384 d128 window
+// computed once per item. (Short runs at the full clock and scores of spread 1; in rows of calls at the power cap the first and
+// third of these gain 3-5 %, and less the wider the scores spread.) B2 H32 N8192 d128 causal 1085 -> 971, B2 H16 N4096 d128 268 -> 237, B4 H16 N16384 d128 window
 // 1024 690 -> 613, 24 heads x 4001 rows d128 with log-sum-exp 120 -> 109, 32 heads x 8192 rows d64 761 -> 675, B8 H12
 // N1000 d64 50.0 -> 47.4, B4 H16 N2048 d64 causal 66.5 -> 62.8, with dropout 97.2 -> 94.5, ALiBi B2 H16 N4096 d64 128.9
 // -> 121.0. Of a round of two tiles at head_dim 128, 2725 clocks of 3050 before, 2370 remain without any products.

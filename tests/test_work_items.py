@@ -107,7 +107,7 @@ def test_slabs_take_the_same_pairs_apart(wi, shape):
 def ring_ends(rows):
     """The hand-over of items between the roles of a CTA, as the kernel does it at head_dim 64. `rows[i]`: published item i
     has rows. Two slots; the producer fills one again when every reader has taken it. The issuing warp takes the next item
-    with rows (or the end) before it commits the last product of the current one; the correction warps take an item and
+    with rows (or the end) before it commits the last product of the current one; the epilogue warps take an item and
     wait for that commit before they take another. Returns whether everybody reaches the end."""
     end = len(rows)  # the end marker is published like an item
     published = issuer = corr = 0  # items published / taken
